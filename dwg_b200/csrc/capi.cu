@@ -650,7 +650,7 @@ int dwg_zero_repair(dwg_knn_index* index, float* normals_dev, const unsigned cha
             DWG_CHECK_CUDA(cudaStreamSynchronize(S(stream)));
             index->zpos_ready = true;
         }
-        DWG_TRY(zero_repair(index->ix, pos.ptr, index->ix.n, normals_dev, is_zero_dev, k, min_zero, index->zws,
+        DWG_TRY(zero_repair(index->ix, pos.ptr, index->ix.n, normals_dev, is_zero_dev, k, min_zero, index->zws, false,
                             S(stream)));
         DWG_CHECK_CUDA(cudaStreamSynchronize(S(stream)));
         return DWG_OK;

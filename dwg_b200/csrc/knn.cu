@@ -3,13 +3,14 @@
 // The reference builds a left-balanced kd-tree with log2(N) thrust sorts and
 // walks it per query with a 30-entry stack (src/KNN_GWN.cu:42-66,490-715,
 // include/cudaKDTree/cukd/traverse-cct.h:25-101).  Point clouds here are
-// surfaces, so a uniform grid sized for ~3 points per occupied cell is built
-// with one counting sort (histogram, scan, scatter), and each query visits
-// Chebyshev shells of cells around its own cell until the k-th candidate is
-// closer than anything outside the visited block.  Candidates are ranked by
-// the cukd key (float bits of dist^2) << 32 | index
-// (include/cudaKDTree/cukd/knn.h:279-282), with dist^2 = (dx*dx + dy*dy) + dz*dz
-// in round-to-nearest single precision, and kept sorted in registers.
+// surfaces, so a uniform grid sized for 3 to 4 points per occupied cell is
+// built with one counting sort (histogram, scan, scatter).  Up to k = 16 a
+// query reads the points within a trial radius of it (k_knn_near) and the
+// queries far from the points walk an occupancy pyramid in groups
+// (k_knn_far); above, a thread per query visits shells of cells and then the
+// pyramid (k_knn_thread).  Candidates are ranked by the cukd key (float bits
+// of dist^2) << 32 | index (include/cudaKDTree/cukd/knn.h:279-282), with
+// dist^2 = (dx*dx + dy*dy) + dz*dz in round-to-nearest single precision.
 #include <cub/cub.cuh>
 
 #include <climits>
@@ -19,6 +20,13 @@
 #include "octree.cuh"
 
 namespace dwg {
+
+// work that runs only when a device count exceeds a minimum
+struct Gate {
+    const int* count = nullptr;
+    int min = 0;
+    __device__ __forceinline__ bool closed() const { return count && *count <= min; }
+};
 
 struct KnnGrid {
     int G0, G1, G2;
@@ -74,7 +82,8 @@ __device__ __forceinline__ unsigned atomic_or_byte(unsigned char* p, unsigned v)
 }
 
 __global__ void k_pyr_fill(const int* __restrict__ cell_start, int G0, int G1, int G2, PyrDims pd,
-                           unsigned char* __restrict__ occ) {
+                           unsigned char* __restrict__ occ, Gate gate) {
+    if (gate.closed()) return;
     const int D0 = pd.ldim[1][0], D1 = pd.ldim[1][1], D2 = pd.ldim[1][2];
     const long long m = (long long)D0 * D1 * D2;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < m;
@@ -126,7 +135,7 @@ static int pyramid_dims(KnnIndex& ix) {
 }
 
 // the occupancy masks of every level from ix.cell_start (stream-ordered)
-static int pyramid_fill(KnnIndex& ix, cudaStream_t s) {
+static int pyramid_fill(KnnIndex& ix, Gate gate, cudaStream_t s) {
     if (ix.levels < 1) return DWG_OK;
     PyrDims pd;
     pd.levels = ix.levels;
@@ -139,14 +148,15 @@ static int pyramid_fill(KnnIndex& ix, cudaStream_t s) {
     long long blocks = div_up(m, 256);
     const long long cap = (long long)num_sms() * 8;
     if (blocks > cap) blocks = cap;
-    k_pyr_fill<<<(unsigned)blocks, 256, 0, s>>>(ix.cell_start.ptr, ix.G[0], ix.G[1], ix.G[2], pd, ix.occ.ptr);
+    k_pyr_fill<<<(unsigned)blocks, 256, 0, s>>>(ix.cell_start.ptr, ix.G[0], ix.G[1], ix.G[2], pd, ix.occ.ptr,
+                                                  gate);
     DWG_CHECK_LAUNCH();
     return DWG_OK;
 }
 
 static int build_pyramid(KnnIndex& ix, cudaStream_t s) {
     DWG_TRY(pyramid_dims(ix));
-    return pyramid_fill(ix, s);
+    return pyramid_fill(ix, Gate{}, s);
 }
 
 int knn_build(KnnIndex& ix, const float* P, int n, cudaStream_t s) {
@@ -182,12 +192,6 @@ int knn_build(KnnIndex& ix, const float* P, int n, cudaStream_t s) {
     }
     ix.h = h;
     ix.inv_h = 1.0f / h;
-    {
-        int gm = max(ix.G[0], max(ix.G[1], ix.G[2]));
-        int sh = 0;
-        while ((gm >> sh) > 32) ++sh;
-        ix.morton_shift = sh;
-    }
     for (int d = 0; d < 3; ++d) ix.lo[d] = bb[d];
     long long ncell = (long long)ix.G[0] * ix.G[1] * ix.G[2];
     KnnGrid g{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h};
@@ -226,7 +230,6 @@ struct KnnArgs {
     long long nq;
     const unsigned long long* nq_dev;
     const int* nq_dev_i32;
-    const unsigned char* __restrict__ exclude;
     const int* gate_count;
     int gate_min;
     int k;
@@ -235,14 +238,13 @@ struct KnnArgs {
     int* __restrict__ q_key;
     int* __restrict__ q_hist;
     int morton_shift;
-    // per-cell bound of the 16th-neighbour distance (null: none), seeds the
-    // per-thread search of queries with k <= 16
-    const float* __restrict__ kb;
-    // queries whose pyramid walk ran past kDeepBudget visits go on this list
-    // (null: no budget) and are finished by k_knn_deep
-    int* __restrict__ deep;
-    float* __restrict__ deep_bound;  // per entry: a bound on the k-th squared distance (its walk's k-th key)
-    int* __restrict__ deep_count;
+    // the queries that k_knn_far finishes, a bound on the k-th squared
+    // distance of each, the groups (first entry, entries), and the counts of
+    // entries and groups
+    int* __restrict__ far_list;
+    float* __restrict__ far_bound;
+    int2* __restrict__ far_group;
+    unsigned int* __restrict__ far_count;
     // per query (null: none): a key above its k-th nearest key, ~0 for none
     const unsigned long long* __restrict__ seed;
     // occupancy pyramid
@@ -251,12 +253,6 @@ struct KnnArgs {
     int ldim[KnnIndex::kMaxLevels][3];
     long long loff[KnnIndex::kMaxLevels];
 };
-
-// a seed key as a distance from the query that holds its k nearest: +inf
-// for none
-__device__ __forceinline__ float seed_radius(unsigned long long sd) {
-    return sd == ~0ull ? INFINITY : sqrtf(__uint_as_float((unsigned)(sd >> 32))) * 1.00002f + 1e-7f;
-}
 
 __device__ __forceinline__ long long knn_count(const KnnArgs& a) {
     long long nq = a.nq;
@@ -284,15 +280,17 @@ __device__ __forceinline__ void knn_load_query(const KnnArgs& a, long long qi, f
     }
 }
 
-__device__ __forceinline__ unsigned spread5(unsigned v) {
-    v &= 31u;
-    v = (v | (v << 8)) & 0x0300Fu;
-    v = (v | (v << 4)) & 0x030C3u;
-    v = (v | (v << 2)) & 0x09249u;
+// the low 10 bits of v, two zero bits between them
+__device__ __forceinline__ unsigned spread10(unsigned v) {
+    v &= 0x3ffu;
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    v = (v | (v << 2)) & 0x09249249u;
     return v;
 }
 
-// bucket the queries by the Morton code of their coarse cell (32^3 buckets)
+// bucket the queries by the Morton code of their coarse cell
 __global__ void k_knn_qkey(KnnArgs a) {
     if (a.gate_count && *a.gate_count <= a.gate_min) return;
     const long long nq = knn_count(a);
@@ -303,7 +301,7 @@ __global__ void k_knn_qkey(KnnArgs a) {
         unsigned cx = cell_coord(qx, a.g.lo0, a.g.inv_h, a.g.G0) >> a.morton_shift;
         unsigned cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1) >> a.morton_shift;
         unsigned cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2) >> a.morton_shift;
-        int key = (int)(spread5(cx) | (spread5(cy) << 1) | (spread5(cz) << 2));
+        int key = (int)(spread10(cx) | (spread10(cy) << 1) | (spread10(cz) << 2));
         a.q_key[qi] = key;
         atomicAdd(&a.q_hist[key], 1);
     }
@@ -316,7 +314,6 @@ __global__ void k_knn_qscatter(KnnArgs a, int* __restrict__ fill, int* __restric
          qi += (long long)gridDim.x * blockDim.x)
         order[atomicAdd(&fill[a.q_key[qi]], 1)] = (int)qi;
 }
-
 
 // top-k state of one lane: an unsorted set of KMAX keys and its maximum
 // (value, slot) of the largest of v[LO, LO + N), the lowest slot among equal
@@ -341,10 +338,7 @@ __device__ __forceinline__ void tour_max(const T (&v)[M], T& m, int& p) {
 // Batcher's odd-even merge sort on 16 inputs, 63 comparators in 10 layers
 // (the iterative form: for p = 1, 2, 4, 8, for d = p, p/2, ..., 1, for j =
 // d mod p, step 2d, for i < d, join i + j and i + j + d when both lie in the
-// same block of 2p); comparator t orders slots kSortLo[t] < kSortHi[t].  On
-// fewer slots the missing ones count as +infinity: a comparator that touches
-// one never swaps and is left out (59 remain for 15 slots, 32 for 10; the
-// odd-even transposition network took 105 and 45).
+// same block of 2p); comparator t orders slots kSortLo[t] < kSortHi[t]
 constexpr int kSortNet = 63;
 constexpr unsigned char kSortLo[kSortNet] = {0, 2, 4, 6, 8, 10, 12, 14, 0, 1, 4, 5, 8, 9, 12, 13, 1, 5, 9, 13, 0, 1, 2, 3, 8, 9, 10, 11, 2, 3, 10, 11, 1, 3, 5, 9, 11, 13, 0, 1, 2, 3, 4, 5, 6, 7, 4, 5, 6, 7, 2, 3, 6, 7, 10, 11, 1, 3, 5, 7, 9, 11, 13};
 constexpr unsigned char kSortHi[kSortNet] = {1, 3, 5, 7, 9, 11, 13, 15, 2, 3, 6, 7, 10, 11, 14, 15, 2, 6, 10, 14, 4, 5, 6, 7, 12, 13, 14, 15, 4, 5, 12, 13, 2, 4, 6, 10, 12, 14, 8, 9, 10, 11, 12, 13, 14, 15, 8, 9, 10, 11, 4, 5, 8, 9, 12, 13, 2, 4, 6, 8, 10, 12, 14};
@@ -359,15 +353,6 @@ struct TopK {
 #pragma unroll
         for (int q = 0; q < KMAX; ++q) e[q] = q < k ? ~0ull : 0ull;  // unused slots never become the max
         mx = ~0ull;
-        mpos = 0;
-        fill = 0;
-    }
-    // k slots holding the key T: only keys below T enter, and T must bound
-    // the k-th key from above so that every slot is replaced
-    __device__ __forceinline__ void init_bound(int k, unsigned long long T) {
-#pragma unroll
-        for (int q = 0; q < KMAX; ++q) e[q] = q < k ? T : 0ull;
-        mx = T;
         mpos = 0;
         fill = 0;
     }
@@ -386,21 +371,48 @@ struct TopK {
             replace_max(v);
         }
     }
-    template <int T>
+    __device__ __forceinline__ void order(int lo, int hi) {
+        const unsigned long long a = e[lo], b = e[hi];
+        e[lo] = a < b ? a : b;
+        e[hi] = a < b ? b : a;
+    }
+    // the 16 slots from LO
+    template <int LO, int T = 0>
     __device__ __forceinline__ void sort_net() {
         if constexpr (T < kSortNet) {
-            constexpr int lo = kSortLo[T], hi = kSortHi[T];
-            if constexpr (hi < KMAX) {
-                const unsigned long long a = e[lo], b = e[hi];
-                e[lo] = a < b ? a : b;
-                e[hi] = a < b ? b : a;
+            constexpr int lo = LO + kSortLo[T], hi = LO + kSortHi[T];
+            order(lo, hi);
+            sort_net<LO, T + 1>();
+        }
+    }
+    // sorted runs of RUN slots from LO on, merged in pairs: the first layer
+    // joins each slot with its mirror image, the others are half-cleaners
+    template <int RUN>
+    __device__ __forceinline__ void merge_runs() {
+        if constexpr (RUN < KMAX) {
+#pragma unroll
+            for (int lo = 0; lo < KMAX; lo += 2 * RUN) {
+#pragma unroll
+                for (int q = 0; q < RUN; ++q) order(lo + q, lo + 2 * RUN - 1 - q);
+#pragma unroll
+                for (int d = RUN / 2; d > 0; d >>= 1)
+#pragma unroll
+                    for (int q = 0; q < 2 * RUN; ++q)
+                        if (!(q & d)) order(lo + q, lo + q + d);
             }
-            sort_net<T + 1>();
+            merge_runs<2 * RUN>();
+        }
+    }
+    template <int LO = 0>
+    __device__ __forceinline__ void sort_blocks() {
+        if constexpr (LO < KMAX) {
+            sort_net<LO>();
+            sort_blocks<LO + 16>();
         }
     }
     // mx and mpos: the largest key and its lowest slot
     __device__ __forceinline__ void max_slot() {
-        if constexpr (KMAX <= 16) {
+        if constexpr (KMAX <= 32) {
             tour_max<0, KMAX>(e, mx, mpos);
         } else {
             mx = e[0];
@@ -413,12 +425,6 @@ struct TopK {
                 }
         }
     }
-    // drop e[0] of a sorted set: the keys move down one slot, NONE enters on top
-    __device__ __forceinline__ void shift_down() {
-#pragma unroll
-        for (int q = 0; q + 1 < KMAX; ++q) e[q] = e[q + 1];
-        e[KMAX - 1] = ~0ull;
-    }
     // replace the maximum by v (v < mx) and find the new maximum (a warp's
     // lanes take the same steps whether or not their slots are all filled)
     __device__ __forceinline__ void replace_max(unsigned long long v) {
@@ -427,11 +433,13 @@ struct TopK {
             if (q == mpos) e[q] = v;
         max_slot();
     }
-    // ascending order (once per query): up to 16 slots the sorting network
-    // of sort_net, more slots an insertion sort in local memory
+    // ascending order (once per query): up to 32 slots the networks, more
+    // slots an insertion sort in local memory
     __device__ __forceinline__ void sort() {
-        if constexpr (KMAX <= 16) {
-            sort_net<0>();
+        if constexpr (KMAX <= 32) {
+            static_assert(KMAX > 32 || KMAX % 16 == 0, "blocks of 16 slots, merged in pairs");
+            sort_blocks();
+            merge_runs<16>();
         } else {
             unsigned long long t[KMAX];
 #pragma unroll
@@ -461,13 +469,9 @@ struct TopK {
 // load) or its (eps-widened) box is farther than the current k-th candidate.
 // The walk is stackless: a 4-bit child counter per level in one 64-bit word,
 // the child masks of the nodes on the path (a byte per level in two 64-bit
-// words) and the current node's coordinates.  With a deep list the walk
-// gives up after kDeepBudget child visits (returns false): a query that far
-// from its neighbours is finished by a warp of k_knn_deep instead of holding
-// a thread (and its warp) for the length of a long walk.
-constexpr int kDeepBudget = 128;
+// words) and the current node's coordinates.
 template <int KMAX>
-__device__ __forceinline__ bool knn_pyramid(const KnnArgs& a, float qx, float qy, float qz, int cx, int cy, int cz,
+__device__ __forceinline__ void knn_pyramid(const KnnArgs& a, float qx, float qy, float qz, int cx, int cy, int cz,
                                             TopK<KMAX>& top) {
     const unsigned long long NONE = ~0ull;
     const float h = a.g.h;
@@ -475,7 +479,6 @@ __device__ __forceinline__ bool knn_pyramid(const KnnArgs& a, float qx, float qy
     const int top_l = a.levels;
     int lvl = top_l, ci = 0, cj = 0, ck = 0;
     unsigned long long ctr = 0;
-    int visits = 0;
     // byte l of (mk1:mk0): the child mask of the path's node at level l
     unsigned long long mk0 = 0ull, mk1 = 0ull;
     {
@@ -496,7 +499,6 @@ __device__ __forceinline__ bool knn_pyramid(const KnnArgs& a, float qx, float qy
             continue;
         }
         ctr += 1ull << sh;
-        if (a.deep && ++visits > kDeepBudget) return false;
         // octant of the query about the node's midpoint
         const int half = 1 << (lvl - 1);
         const float mx = a.g.lo0 + (float)((ci << lvl) + half) * h;
@@ -523,7 +525,6 @@ __device__ __forceinline__ bool knn_pyramid(const KnnArgs& a, float qx, float qy
             for (int t = a.cell_start[cell]; t < e; ++t) {
                 const float4 pp = a.pts[t];
                 const int id = __float_as_int(pp.w);
-                if (a.exclude && a.exclude[id]) continue;
                 const float d2 = sq3_rn(__fsub_rn(pp.x, qx), __fsub_rn(pp.y, qy), __fsub_rn(pp.z, qz));
                 const unsigned long long v = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)id;
                 if (v < top.mx) top.push(v, a.k);
@@ -540,10 +541,9 @@ __device__ __forceinline__ bool knn_pyramid(const KnnArgs& a, float qx, float qy
         cj = nj;
         ck = nk;
     }
-    return true;
 }
 
-// One thread per query; queries are processed in the order of their coarse
+// k > 16: one thread per query; queries are processed in the order of their coarse
 // Morton bucket so that neighbouring threads search neighbouring cells.  A
 // query visits Chebyshev shells of cells around its own cell; a cell is
 // skipped when its box is farther than the current k-th candidate; the k best
@@ -551,7 +551,7 @@ __device__ __forceinline__ bool knn_pyramid(const KnnArgs& a, float qx, float qy
 // (replace-the-maximum on insertion, one sort at the end).  The search stops
 // when the k-th key is closer than the boundary of the visited block.
 template <int KMAX>
-__global__ void __launch_bounds__(128, KMAX <= 10 ? 4 : 1) k_knn_thread(KnnArgs a) {
+__global__ void __launch_bounds__(128) k_knn_thread(KnnArgs a) {
     if (a.gate_count && *a.gate_count <= a.gate_min) return;
     const long long nq = knn_count(a);
     const unsigned long long NONE = ~0ull;
@@ -567,22 +567,7 @@ __global__ void __launch_bounds__(128, KMAX <= 10 ? 4 : 1) k_knn_thread(KnnArgs 
         const int cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1);
         const int cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2);
         TopK<KMAX> top;
-        bool deferred = false;
-        if (a.kb && k <= kKnnBoundK) {
-            // start from k copies of the key of the bound kb[c] + |q - x_c|
-            // on the 16th distance: everything beyond it is pruned at once
-            const float ex = qx - (a.g.lo0 + ((float)cx + 0.5f) * h), ey = qy - (a.g.lo1 + ((float)cy + 0.5f) * h),
-                        ez = qz - (a.g.lo2 + ((float)cz + 0.5f) * h);
-            const float rq = (a.kb[cx + a.g.G0 * (cy + a.g.G1 * cz)] + sqrtf(ex * ex + ey * ey + ez * ez) * 1.00002f) *
-                                 1.00002f + 1e-7f;
-            top.init_bound(k, ((unsigned long long)__float_as_uint(rq * rq * 1.00002f) << 32) | 0xffffffffull);
-        } else {
-            top.init(k);
-        }
-        if (a.seed) {
-            const unsigned long long sd = a.seed[qi];
-            if (sd < top.mx) top.init_bound(k, sd);
-        }
+        top.init(k);
         for (int r = 0;; ++r) {
             const float kd2 = top.mx == NONE ? INFINITY : __uint_as_float((unsigned)(top.mx >> 32)) * 1.00001f;
             for (int dz = -r; dz <= r; ++dz) {
@@ -610,7 +595,6 @@ __global__ void __launch_bounds__(128, KMAX <= 10 ? 4 : 1) k_knn_thread(KnnArgs 
                         for (int t = a.cell_start[c]; t < e; ++t) {
                             const float4 pp = a.pts[t];
                             const int id = __float_as_int(pp.w);
-                            if (a.exclude && a.exclude[id]) continue;
                             const float d2 =
                                 sq3_rn(__fsub_rn(pp.x, qx), __fsub_rn(pp.y, qy), __fsub_rn(pp.z, qz));
                             const unsigned long long v = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)id;
@@ -634,19 +618,10 @@ __global__ void __launch_bounds__(128, KMAX <= 10 ? 4 : 1) k_knn_thread(KnnArgs 
                 if (bd > 0.f && __uint_as_float((unsigned)(top.mx >> 32)) < bd * bd * 0.9999f) break;
             }
             if (r == 1 && a.levels > 0) {
-                if (!knn_pyramid<KMAX>(a, qx, qy, qz, cx, cy, cz, top)) {
-                    // at most once per query: the list holds nq.  The walk's
-                    // current maximum (its k-th key, or the initial bound)
-                    // bounds the k-th squared distance
-                    const int pos = atomicAdd(a.deep_count, 1);
-                    a.deep[pos] = (int)qi;
-                    a.deep_bound[pos] = top.mx == NONE ? INFINITY : __uint_as_float((unsigned)(top.mx >> 32));
-                    deferred = true;
-                }
+                knn_pyramid<KMAX>(a, qx, qy, qz, cx, cy, cz, top);
                 break;
             }
         }
-        if (deferred) continue;
         top.sort();
         // slots >= k hold 0 (below every key) and sort first; results start at KMAX - k
 #pragma unroll
@@ -657,739 +632,521 @@ __global__ void __launch_bounds__(128, KMAX <= 10 ? 4 : 1) k_knn_thread(KnnArgs 
     }
 }
 
-// ------------------------------------------------------ cell-grouped path --
-// Queries with k <= 16 and no exclusion are grouped by the grid cell they fall
-// in (clamped to the grid).  For cell c with centre x_c, kb[c] bounds the
-// distance from x_c to its 16th nearest point from above, and m_c is the
-// largest |q - x_c| over the cell's queries.  By the triangle inequality the
-// k nearest points of every such query lie within R_c = kb[c] + 2 m_c of x_c,
-// so one warp gathers that candidate set once (occupancy pyramid, then
-// cells, then points, all 32 lanes in step) into shared memory and every lane
-// then ranks the same candidates for its own query: no divergence, one search
-// per cell instead of one per query.  A cell whose candidate set does not fit
-// (or has no finite bound) sends its queries to the per-thread search.
-constexpr int kCqWarps = 4;
-constexpr int kCqNodes = 1024;  // frontier capacity per warp (ping-pong pair, shared memory), at level >= 1
-constexpr int kCqChunk = 256;   // candidates staged in shared memory at a time
+// -------------------------------------------------------- near queries --
+// k <= 16: kNearLanes lanes per query.  A query reads the points within a
+// trial radius of it: cells are x-fastest, so the cells of one row (y, z)
+// within the radius hold one contiguous run of points.  The lanes list the
+// rows' runs, join them into one list and walk it a point each; the keys
+// within the radius go to shared memory, and when there are k the rank of a
+// key among them (the number below it) is its place in the answer, so
+// nothing is kept sorted.  The first radius follows the density around the
+// query's cell, ~1.35 k points; a round that finds fewer than k is followed
+// by one that reads the shell up to 1.5 times the radius, and past the widest
+// the query goes to k_knn_far, as does one with more keys than are kept (from
+// its radius).  A query with a seed within reach starts from the seed's
+// radius.  The walk's instructions bound it: ~1,780 per warp and 4 queries on
+// 100,000 points of a sphere (k = 15), 80 % of issue slots, 250,000 queries
+// in 150 us (430 us before, one warp per cell streaming the cell's ball);
+// a thread per query keeping a sorted set took 220 us, waiting on its loads.
+constexpr int kNearThreads = 128;
+constexpr int kNearLanes = 8;  // lanes per query
+constexpr int kNearRuns = 4;   // rows a lane lists before it reads their points
+constexpr int kNearKeys = 64;  // keys kept per query
+constexpr int kNearUnit = 64;  // queries a warp takes at a time, at most
+constexpr float kNearFirst = 1.35f * 11.f / 3.14159265f;  // first radius^2 in cells^2: this k / points near
+constexpr float kNearMost = 4.f;                          // at most this
+// the widest radius, in cells
+constexpr float kNearWidest = 3.3f;
 
-__device__ __forceinline__ float cell_mid(float lo, int i, float h) { return lo + ((float)i + 0.5f) * h; }
-
-// kb from the 3x3x3 block around each cell: the 16th smallest distance, or
-// +inf when the block holds fewer than 16 points
-__global__ void k_kb_local(KnnGrid g, const int* __restrict__ cell_start, const float4* __restrict__ pts,
-                           const unsigned char* __restrict__ occ1, int D0, int D1, float* __restrict__ kb) {
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= (long long)g.G0 * g.G1 * g.G2) return;
-    const int i = (int)(c % g.G0), j = (int)((c / g.G0) % g.G1), k = (int)(c / ((long long)g.G0 * g.G1));
-    if (occ1) {
-        // the 3x3x3 block lies in at most 2x2x2 nodes of pyramid level 1:
-        // when they are all empty the bound stays +inf (cheap for empty space)
-        bool any = false;
-        for (int z = max(k - 1, 0) >> 1; z <= min(k + 1, g.G2 - 1) >> 1 && !any; ++z)
-            for (int y = max(j - 1, 0) >> 1; y <= min(j + 1, g.G1 - 1) >> 1 && !any; ++y)
-                for (int x = max(i - 1, 0) >> 1; x <= min(i + 1, g.G0 - 1) >> 1; ++x)
-                    if (occ1[x + (long long)D0 * (y + (long long)D1 * z)]) {
-                        any = true;
-                        break;
-                    }
-        if (!any) {
-            kb[c] = INFINITY;
-            return;
-        }
-    }
-    const float x = cell_mid(g.lo0, i, g.h), y = cell_mid(g.lo1, j, g.h), z = cell_mid(g.lo2, k, g.h);
-    float d[kKnnBoundK];
-#pragma unroll
-    for (int t = 0; t < kKnnBoundK; ++t) d[t] = INFINITY;
-    float mx = INFINITY;
-    int mpos = 0, cnt = 0;
-    for (int dz = -1; dz <= 1; ++dz) {
-        const int zz = k + dz;
-        if (zz < 0 || zz >= g.G2) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int yy = j + dy;
-            if (yy < 0 || yy >= g.G1) continue;
-            for (int dx = -1; dx <= 1; ++dx) {
-                const int xx = i + dx;
-                if (xx < 0 || xx >= g.G0) continue;
-                const int cc = xx + g.G0 * (yy + g.G1 * zz);
-                const int e = cell_start[cc + 1];
-                for (int t = cell_start[cc]; t < e; ++t) {
-                    const float4 p = pts[t];
-                    const float ex = p.x - x, ey = p.y - y, ez = p.z - z;
-                    const float d2 = ex * ex + ey * ey + ez * ez;
-                    if (cnt < kKnnBoundK) {  // the first keys fill the slots; the maximum once they are full
-#pragma unroll
-                        for (int q = 0; q < kKnnBoundK; ++q)
-                            if (q == cnt) d[q] = d2;
-                        if (cnt == kKnnBoundK - 1) {
-                            tour_max<0, kKnnBoundK>(d, mx, mpos);
-                        }
-                    } else if (d2 < mx) {
-#pragma unroll
-                        for (int q = 0; q < kKnnBoundK; ++q)
-                            if (q == mpos) d[q] = d2;
-                        tour_max<0, kKnnBoundK>(d, mx, mpos);
-                    }
-                    ++cnt;
-                }
-            }
-        }
-    }
-    kb[c] = cnt >= kKnnBoundK ? sqrtf(mx) * 1.00002f + 1e-7f : INFINITY;
-}
-
-// kb for the cells that hold queries: the 16th smallest distance from the
-// cell centre over the cells within Chebyshev radius r, r = 1, 2, 3 until 16
-// points are found (any 16 points bound the 16th nearest from above), +inf
-// when the radius-3 block holds fewer (those queries take the per-thread
-// search, which needs no bound) or when every query of the cell has a seed
-constexpr int kKbActiveRadius = 3;
-__global__ void k_kb_active(KnnGrid g, const int* __restrict__ cell_start, const float4* __restrict__ pts,
-                            const unsigned char* __restrict__ occ1, int D0, int D1, const int* __restrict__ active,
-                            const int* __restrict__ misc, const unsigned int* __restrict__ sbits,
-                            float* __restrict__ kb) {
-    const int na = misc[0];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < na; t += gridDim.x * blockDim.x) {
-        const int c = active[t];
-        // a cell whose queries all have seeds takes its radius from them
-        if (sbits && isfinite(__uint_as_float(sbits[c]))) {
-            kb[c] = INFINITY;
-            continue;
-        }
-        const int i = c % g.G0, j = (c / g.G0) % g.G1, k = c / (g.G0 * g.G1);
-        const float x = cell_mid(g.lo0, i, g.h), y = cell_mid(g.lo1, j, g.h), z = cell_mid(g.lo2, k, g.h);
-        float d[kKnnBoundK];
-#pragma unroll
-        for (int q = 0; q < kKnnBoundK; ++q) d[q] = INFINITY;
-        float mx = INFINITY;
-        int mpos = 0, cnt = 0;
-        for (int r = 0; r <= kKbActiveRadius; ++r) {
-            for (int dz = -r; dz <= r; ++dz) {
-                const int zz = k + dz;
-                if (zz < 0 || zz >= g.G2) continue;
-                for (int dy = -r; dy <= r; ++dy) {
-                    const int yy = j + dy;
-                    if (yy < 0 || yy >= g.G1) continue;
-                    for (int dx = -r; dx <= r; ++dx) {
-                        // the shell of radius r only
-                        if (max(abs(dx), max(abs(dy), abs(dz))) != r) continue;
-                        const int xx = i + dx;
-                        if (xx < 0 || xx >= g.G0) continue;
-                        // an empty cell by its bit in the level-1 child mask
-                        // (8 cells share a byte): no range loads
-                        if (occ1 && !((occ1[(xx >> 1) + (long long)D0 * ((yy >> 1) + (long long)D1 * (zz >> 1))] >>
-                                       ((xx & 1) | ((yy & 1) << 1) | ((zz & 1) << 2))) &
-                                      1))
-                            continue;
-                        const int cc = xx + g.G0 * (yy + g.G1 * zz);
-                        const int e = cell_start[cc + 1];
-                        for (int s = cell_start[cc]; s < e; ++s) {
-                            const float4 p = pts[s];
-                            const float ex = p.x - x, ey = p.y - y, ez = p.z - z;
-                            const float d2 = ex * ex + ey * ey + ez * ez;
-                            if (cnt < kKnnBoundK) {  // fill, then the maximum once
-#pragma unroll
-                                for (int q = 0; q < kKnnBoundK; ++q)
-                                    if (q == cnt) d[q] = d2;
-                                if (cnt == kKnnBoundK - 1) {
-                                    tour_max<0, kKnnBoundK>(d, mx, mpos);
-                                }
-                            } else if (d2 < mx) {
-#pragma unroll
-                                for (int q = 0; q < kKnnBoundK; ++q)
-                                    if (q == mpos) d[q] = d2;
-                                tour_max<0, kKnnBoundK>(d, mx, mpos);
-                            }
-                            ++cnt;
-                        }
-                    }
-                }
-            }
-            if (r >= 1 && cnt >= kKnnBoundK) break;
-        }
-        kb[c] = cnt >= kKnnBoundK ? sqrtf(mx) * 1.00002f + 1e-7f : INFINITY;
-    }
-}
-
-// one min-plus pass with the 26 neighbours at distance `step` cells:
-// kb[c] <= kb[c'] + |x_c - x_c'| (triangle inequality); len1..3 are the
-// neighbour distances rounded up
-__global__ void k_kb_jfa(KnnGrid g, const float* __restrict__ in, float* __restrict__ out, int step, float len1,
-                         float len2, float len3) {
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= (long long)g.G0 * g.G1 * g.G2) return;
-    const int i = (int)(c % g.G0), j = (int)((c / g.G0) % g.G1), k = (int)(c / ((long long)g.G0 * g.G1));
-    float v = in[c];
-    for (int dz = -1; dz <= 1; ++dz) {
-        const int zz = k + dz * step;
-        if (zz < 0 || zz >= g.G2) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int yy = j + dy * step;
-            if (yy < 0 || yy >= g.G1) continue;
-            for (int dx = -1; dx <= 1; ++dx) {
-                const int xx = i + dx * step;
-                if (xx < 0 || xx >= g.G0) continue;
-                const int nz = (dx != 0) + (dy != 0) + (dz != 0);
-                if (nz == 0) continue;
-                const float len = nz == 1 ? len1 : (nz == 2 ? len2 : len3);
-                v = fminf(v, __fadd_ru(in[xx + (long long)g.G0 * (yy + (long long)g.G1 * zz)], len));
-            }
-        }
-    }
-    out[c] = v;
-}
-
-static int build_kbound(const KnnIndex& ix, cudaStream_t s) {
-    const long long ncell = (long long)ix.G[0] * ix.G[1] * ix.G[2];
-    KnnGrid g{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h};
-    DWG_TRY(ix.kb.reserve(ncell));
-    DWG_TRY(ix.kb_tmp.reserve(ncell));
-    const unsigned char* occ1 = ix.levels >= 1 ? ix.occ.ptr + ix.loff[1] : nullptr;
-    k_kb_local<<<div_up(ncell, 128), 128, 0, s>>>(g, ix.cell_start.ptr, ix.pts.ptr, occ1, ix.ldim[1][0], ix.ldim[1][1],
-                                                   ix.kb.ptr);
-    DWG_CHECK_LAUNCH();
-    const int gmax = max(ix.G[0], max(ix.G[1], ix.G[2]));
-    int step = 1;
-    while (step * 2 < gmax) step *= 2;
-    std::vector<int> steps;
-    for (int st = step; st >= 1; st /= 2) steps.push_back(st);
-    steps.push_back(1);
-    steps.push_back(1);
-    float* a = ix.kb.ptr;
-    float* b = ix.kb_tmp.ptr;
-    for (int st : steps) {
-        const double hs = (double)st * (double)ix.h;
-        const float l1 = nextafterf((float)hs, INFINITY);
-        const float l2 = nextafterf((float)(hs * 1.4142135623730951), INFINITY);
-        const float l3 = nextafterf((float)(hs * 1.7320508075688772), INFINITY);
-        k_kb_jfa<<<div_up(ncell, 256), 256, 0, s>>>(g, a, b, st, l1, l2, l3);
-        DWG_CHECK_LAUNCH();
-        std::swap(a, b);
-    }
-    if (a != ix.kb.ptr)
-        DWG_CHECK_CUDA(cudaMemcpyAsync(ix.kb.ptr, a, sizeof(float) * ncell, cudaMemcpyDeviceToDevice, s));
-    ix.kb_ready = true;
-    return DWG_OK;
-}
-
-// cell of every query, queries per cell, largest |q - x_c| per cell
-// with seeds, sbits[c] gets the largest |q - x_c| + seed radius over the
-// cell's queries (+inf when one has no seed): the k nearest of every query of
-// the cell lie within it of the centre
-__global__ void k_cq_key(KnnArgs a, int* __restrict__ key, int* __restrict__ count, unsigned int* __restrict__ mbits,
-                         unsigned int* __restrict__ sbits) {
-    if (a.gate_count && *a.gate_count <= a.gate_min) return;
-    const long long nq = knn_count(a);
-    for (long long qi = blockIdx.x * (long long)blockDim.x + threadIdx.x; qi < nq;
-         qi += (long long)gridDim.x * blockDim.x) {
-        float qx, qy, qz;
-        knn_load_query(a, qi, qx, qy, qz);
-        const int cx = cell_coord(qx, a.g.lo0, a.g.inv_h, a.g.G0);
-        const int cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1);
-        const int cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2);
-        const int c = cx + a.g.G0 * (cy + a.g.G1 * cz);
-        const float ex = qx - cell_mid(a.g.lo0, cx, a.g.h), ey = qy - cell_mid(a.g.lo1, cy, a.g.h),
-                    ez = qz - cell_mid(a.g.lo2, cz, a.g.h);
-        const float m = sqrtf(ex * ex + ey * ey + ez * ez) * 1.00002f + 1e-7f;
-        key[qi] = c;
-        atomicAdd(&count[c], 1);
-        atomicMax(&mbits[c], __float_as_uint(m));  // non-negative floats order as their bits
-        if (sbits) atomicMax(&sbits[c], __float_as_uint((m + seed_radius(a.seed[qi])) * 1.00002f));
-    }
-}
-
-__global__ void k_cq_active(const int* __restrict__ count, long long ncell, int* __restrict__ active,
-                            int* __restrict__ nactive) {
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= ncell || count[c] == 0) return;
-    active[atomicAdd(nactive, 1)] = (int)c;
-}
-
-__global__ void k_cq_scatter(KnnArgs a, const int* __restrict__ key, int* __restrict__ fill, int* __restrict__ order) {
-    if (a.gate_count && *a.gate_count <= a.gate_min) return;
-    const long long nq = knn_count(a);
-    for (long long qi = blockIdx.x * (long long)blockDim.x + threadIdx.x; qi < nq;
-         qi += (long long)gridDim.x * blockDim.x)
-        order[atomicAdd(&fill[key[qi]], 1)] = (int)qi;
-}
-
-// is the node (ni, nj, nk) of level l non-empty and within R of (x, y, z)?
-__device__ __forceinline__ bool cq_node_hit(const KnnArgs& a, int l, int ni, int nj, int nk, float x, float y,
-                                            float z, float R2, float eps) {
-    const int* D = a.ldim[l];
-    if (ni < 0 || nj < 0 || nk < 0 || ni >= D[0] || nj >= D[1] || nk >= D[2]) return false;
-    const float h = a.g.h;
-    const float x0 = a.g.lo0 + (float)(ni << l) * h - eps, x1 = a.g.lo0 + (float)((ni + 1) << l) * h + eps;
-    const float y0 = a.g.lo1 + (float)(nj << l) * h - eps, y1 = a.g.lo1 + (float)((nj + 1) << l) * h + eps;
-    const float z0 = a.g.lo2 + (float)(nk << l) * h - eps, z1 = a.g.lo2 + (float)((nk + 1) << l) * h + eps;
-    const float ddx = fmaxf(0.f, fmaxf(x0 - x, x - x1));
-    const float ddy = fmaxf(0.f, fmaxf(y0 - y, y - y1));
-    const float ddz = fmaxf(0.f, fmaxf(z0 - z, z - z1));
-    if (ddx * ddx + ddy * ddy + ddz * ddz > R2) return false;
-    if (l == 0) {
-        const int c = ni + a.g.G0 * (nj + a.g.G1 * nk);
-        return a.cell_start[c + 1] > a.cell_start[c];
-    }
-    return a.occ[a.loff[l] + ni + (long long)D[0] * (nj + (long long)D[1] * nk)] != 0;
-}
-
+// the KMAX smallest keys, ascending (k < KMAX: the first KMAX - k slots hold
+// 0); an insertion is 2 compares and 2 selects of 64 bits per slot, without
+// branches, and leaves the set sorted for the output
 template <int KMAX>
-__global__ void __launch_bounds__(kCqWarps * 32) k_knn_cells(KnnArgs a, const int* __restrict__ active,
-                                                             const int* __restrict__ misc,
-                                                             const int* __restrict__ cstart,
-                                                             const int* __restrict__ ccount,
-                                                             const unsigned int* __restrict__ mbits,
-                                                             const unsigned int* __restrict__ sbits,
-                                                             const float* __restrict__ kb,
-                                                             const int* __restrict__ order,
-                                                             int* __restrict__ work, int* __restrict__ fb) {
-    __shared__ int nodes[kCqWarps][2][kCqNodes];
-    __shared__ float4 stage[kCqWarps][kCqChunk];
-    if (a.gate_count && *a.gate_count <= a.gate_min) return;
+struct SortedK {
+    unsigned long long e[KMAX];
+    __device__ __forceinline__ void init(int k, unsigned long long T) {
+#pragma unroll
+        for (int q = 0; q < KMAX; ++q) e[q] = q < KMAX - k ? 0ull : T;
+    }
+    __device__ __forceinline__ unsigned long long last() const { return e[KMAX - 1]; }
+    // the largest squared distance kept (NaN while a slot is empty)
+    __device__ __forceinline__ float last_d2() const { return __uint_as_float((unsigned)(e[KMAX - 1] >> 32)); }
+    __device__ __forceinline__ void insert(unsigned long long v) {
+#pragma unroll
+        for (int q = KMAX - 1; q > 0; --q) e[q] = v < e[q] ? (v < e[q - 1] ? e[q - 1] : v) : e[q];
+        e[0] = v < e[0] ? v : e[0];
+    }
+    // the k keys' indices (-1 in empty slots)
+    __device__ __forceinline__ void store(int* __restrict__ out, int k) const {
+#pragma unroll
+        for (int t = 0; t < KMAX; ++t) {
+            const int o = t - (KMAX - k);
+            if (o >= 0) out[o] = e[t] == ~0ull ? -1 : (int)(unsigned)(e[t] & 0xffffffffu);
+        }
+    }
+};
+
+// Far queries waiting in a warp: position and query, bound
+struct FarWait {
+    float4 q[64];
+    float bound[64];
+};
+
+// a square root rounded up (1e-4 over: the approximation's error is below 1e-6)
+__device__ __forceinline__ float sqrt_up(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y * 1.0001f;
+}
+
+// n (1 to 32) of them go to the far list, split into groups of queries near
+// each other: within 4 cells, or an eighth of the bound, of the group's first
+__device__ __forceinline__ void far_groups(const KnnArgs& a, const FarWait& f, int n, int lane) {
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned below = (1u << lane) - 1u;
-    const int nactive = misc[0];
+    unsigned pos = 0;
+    if (lane == 0) pos = atomicAdd(a.far_count, (unsigned)n);
+    pos = __shfl_sync(FULL, pos, 0);
+    const float4 q = f.q[lane];
+    const float b = f.bound[lane];
+    unsigned left = n == 32 ? FULL : (1u << n) - 1u;
+    while (left) {
+        const int first = __ffs(left) - 1;
+        const float dx = q.x - __shfl_sync(FULL, q.x, first), dy = q.y - __shfl_sync(FULL, q.y, first),
+                    dz = q.z - __shfl_sync(FULL, q.z, first);
+        const float b0 = __shfl_sync(FULL, b, first);
+        const float reach = fmaxf(16.f * a.g.h * a.g.h, b0 < INFINITY ? b0 * (1.f / 64.f) : 0.f);
+        const bool in = lane == first || (((left >> lane) & 1u) && dx * dx + dy * dy + dz * dz <= reach);
+        const unsigned m = __ballot_sync(FULL, in);
+        if (in) {
+            const unsigned o = pos + __popc(m & ((1u << lane) - 1u));
+            a.far_list[o] = __float_as_int(q.w);
+            a.far_bound[o] = b;
+        }
+        if (lane == 0) a.far_group[atomicAdd(a.far_count + 1, 1u)] = make_int2((int)pos, __popc(m));
+        pos += __popc(m);
+        left &= ~m;
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned int* __restrict__ work) {
+    constexpr int G = kNearLanes, QW = 32 / G;  // lanes per query, queries per warp
+    // a key's bits read as a double order like the key (d2 <= +inf: the
+    // exponent stays below the NaNs'), and compare in one instruction
+    __shared__ double keys[kNearThreads / G][kNearKeys];
+    __shared__ int2 runs[kNearThreads / G][G * kNearRuns];
+    __shared__ FarWait far[kNearThreads / 32];
+    if (a.gate_count && *a.gate_count <= a.gate_min) return;
+    const long long nq = knn_count(a);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int sub = lane & (G - 1);
+    const unsigned FULL = 0xffffffffu;
+    const unsigned mine = ((1u << G) - 1u) << (lane & ~(G - 1));  // the query's lanes
+    const unsigned before = mine & ((1u << lane) - 1u);
+    double* const key = keys[tid / G];
+    int2* const run = runs[tid / G];
     const unsigned long long NONE = ~0ull;
+    const int k = a.k;
     const float h = a.g.h;
     const float eps = 1e-4f * h + 1e-6f;
-    const int k = a.k;
+    const float widest = kNearWidest * h;
+    // a warp takes a run of consecutive queries at a time, short when the
+    // launch would leave warps idle; the far ones among them form the groups
+    // of the far search
+    const long long warps = (long long)gridDim.x * (kNearThreads / 32);
+    const unsigned unit = (unsigned)(max((long long)QW, min((long long)kNearUnit, nq / (2 * warps))) / QW * QW);
+    unsigned base = 0, end = 0;
+    int nfar = 0;  // queries waiting (warp-uniform)
     for (;;) {
-        int wi = 0;
-        if (lane == 0) wi = atomicAdd(&work[0], 1);
-        wi = __shfl_sync(FULL, wi, 0);
-        if (wi >= nactive) break;
-        const int c = active[wi];
-        const int ci = c % a.g.G0, cj = (c / a.g.G0) % a.g.G1, ck = c / (a.g.G0 * a.g.G1);
-        const float x = cell_mid(a.g.lo0, ci, h), y = cell_mid(a.g.lo1, cj, h), z = cell_mid(a.g.lo2, ck, h);
-        const int qs = cstart[c], qn = ccount[c];
-        float R = (kb[c] + 2.0f * __uint_as_float(mbits[c])) * 1.00002f + 1e-6f * h;
-        if (sbits) R = fminf(R, __uint_as_float(sbits[c]) * 1.00002f + 1e-6f * h);
-        bool ok = isfinite(R);
-        int* cur = nodes[w][0];
-        int nf = 0;
-        int l = 0;   // the level the frontier starts at
-        int fl = 0;  // the level it ends at (cells are streamed from there)
-        if (ok) {
-            const float R2 = R * R;
-            // the ball's box in cells
-            const int x0 = cell_coord(x - R, a.g.lo0, a.g.inv_h, a.g.G0), x1 = cell_coord(x + R, a.g.lo0, a.g.inv_h, a.g.G0);
-            const int y0 = cell_coord(y - R, a.g.lo1, a.g.inv_h, a.g.G1), y1 = cell_coord(y + R, a.g.lo1, a.g.inv_h, a.g.G1);
-            const int z0 = cell_coord(z - R, a.g.lo2, a.g.inv_h, a.g.G2), z1 = cell_coord(z + R, a.g.lo2, a.g.inv_h, a.g.G2);
-            // coarsest-enough level: the nodes covering the box fit the frontier
-            for (;;) {
-                const long long nn = (long long)((x1 >> l) - (x0 >> l) + 1) * ((y1 >> l) - (y0 >> l) + 1) *
-                                     ((z1 >> l) - (z0 >> l) + 1);
-                if (nn <= kCqNodes || l >= a.levels) break;
-                ++l;
+        if (base == end || (long long)base >= nq) {
+            if (nfar > 0) {
+                far_groups(a, far[w], nfar, lane);
+                nfar = 0;
             }
-            const int bx = (x1 >> l) - (x0 >> l) + 1, by = (y1 >> l) - (y0 >> l) + 1, bz = (z1 >> l) - (z0 >> l) + 1;
-            const int tot = bx * by * bz;
-            int* nxt = nodes[w][1];
-            // stage A: the nodes of level l covering the box
-            for (int b = 0; b < tot; b += 32) {
-                const int t = b + lane;
-                bool keep = false;
-                int id = 0;
-                if (t < tot) {
-                    const int ni = (x0 >> l) + t % bx, nj = (y0 >> l) + (t / bx) % by, nk = (z0 >> l) + t / (bx * by);
-                    keep = cq_node_hit(a, l, ni, nj, nk, x, y, z, R2, eps);
-                    id = ni + a.ldim[l][0] * (nj + a.ldim[l][1] * nk);
-                }
-                const unsigned bal = __ballot_sync(FULL, keep);
-                const int pos = nf + __popc(bal & below);
-                if (keep && pos < kCqNodes) cur[pos] = id;
-                nf += __popc(bal);
-            }
-            ok = nf <= kCqNodes;
-            // stage B: down to level 1 (the cells are expanded while
-            // streaming); when the next level would not fit, the frontier
-            // stays at the coarser level and its nodes' cells are streamed
-            fl = l;
-            for (int lv = l; lv >= 2 && ok; --lv) {
-                __syncwarp();
-                const int* D = a.ldim[lv];
-                int nn = 0;
-                for (int b = 0; b < nf * 8; b += 32) {
-                    const int t = b + lane;
-                    bool keep = false;
-                    int id = 0;
-                    if (t < nf * 8) {
-                        const int node = cur[t >> 3], oc = t & 7;
-                        const int ni = node % D[0], nj = (node / D[0]) % D[1], nk = node / (D[0] * D[1]);
-                        const int ui = 2 * ni + (oc & 1), uj = 2 * nj + ((oc >> 1) & 1), uk = 2 * nk + (oc >> 2);
-                        keep = cq_node_hit(a, lv - 1, ui, uj, uk, x, y, z, R2, eps);
-                        id = ui + a.ldim[lv - 1][0] * (uj + a.ldim[lv - 1][1] * uk);
-                    }
-                    const unsigned bal = __ballot_sync(FULL, keep);
-                    const int pos = nn + __popc(bal & below);
-                    if (keep && pos < kCqNodes) nxt[pos] = id;
-                    nn += __popc(bal);
-                }
-                if (nn > kCqNodes) break;  // keep the level-lv frontier
-                int* tmp = cur;
-                cur = nxt;
-                nxt = tmp;
-                nf = nn;
-                fl = lv - 1;
-            }
-            __syncwarp();
+            if (lane == 0) base = atomicAdd(work, unit);
+            base = __shfl_sync(FULL, base, 0);
+            end = base + unit;
         }
-        // a ball so large that the frontier stayed coarse, for a handful of
-        // queries: the per-thread search, seeded with each query's own bound,
-        // prunes it faster than the warp streams it
-        if (ok && fl >= 2 && qn < 8) ok = false;
-        if (!ok) {  // the per-thread search takes this cell's queries
-            for (int t = lane; t < qn; t += 32) fb[atomicAdd(&work[1], 1)] = order[qs + t];
-            continue;
+        if ((long long)base >= nq) break;
+        const long long j = (long long)base + lane / G;
+        const bool has = j < nq;
+        const long long qi = !has ? 0 : a.order ? a.order[j] : j;
+        base += QW;
+        float qx = 0.f, qy = 0.f, qz = 0.f, seed2 = INFINITY;
+        bool search = has, wait = false;
+        if (has) {
+            knn_load_query(a, qi, qx, qy, qz);
+            if (a.seed) {
+                const unsigned long long T = a.seed[qi];
+                if (T != NONE) seed2 = __uint_as_float((unsigned)(T >> 32));
+            }
+            // a NaN has no neighbours
+            search = !(isnan(qx) || isnan(qy) || isnan(qz));
         }
-        // stages C + D, per chunk of up to 32 queries: the points of the
-        // frontier cells within R of the centre are streamed through shared
-        // memory and ranked for every query, starting from the bound
-        // kb[c] + |q - x_c| on its 16th distance.  A chunk of nb queries gives
-        // each query G lanes (the largest power of two with nb * G <= 32): a
-        // lane ranks every G-th staged point for its query, and the G lanes'
-        // sets are merged at the end.  Cells hold a few queries, so this
-        // keeps the lanes busy instead of ranking for absent queries.
-        const float kbc = kb[c];
-        const float R2 = R * R;
-        for (int base = 0; base < qn; base += 32) {
-            const int nb = qn - base < 32 ? qn - base : 32;
-            const int lg = nb > 16 ? 0 : nb > 8 ? 1 : nb > 4 ? 2 : nb > 2 ? 3 : nb > 1 ? 4 : 5;
-            const int G = 1 << lg;
-            const int u = lane >> lg, sl = lane & (G - 1);
-            const bool has = u < nb;
-            long long qi = 0;
-            float qx = x, qy = y, qz = z;
-            if (has) {
-                qi = order[qs + base + u];
-                knn_load_query(a, qi, qx, qy, qz);
+        int found = 0;  // keys of the query
+        // The first radius: a surface through the 3x3x3 block around the
+        // query's cell covers ~11 faces of cells, so 1.35 k points lie within
+        // r^2 = 1.35 k 11 / (pi N) cells^2 for N points in the block
+        const int cx = cell_coord(qx, a.g.lo0, a.g.inv_h, a.g.G0), cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1),
+                  cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2);
+        int near = 0;
+        if (search) {
+            const int x0 = max(cx - 1, 0), x1 = min(cx + 1, a.g.G0 - 1) + 1;
+#pragma unroll
+            for (int u = 0; u < (9 + G - 1) / G; ++u) {
+                const int i = u * G + sub, y = cy + i % 3 - 1, z = cz + i / 3 - 1;
+                if (i < 9 && y >= 0 && y < a.g.G1 && z >= 0 && z < a.g.G2) {
+                    const int* row = a.cell_start + a.g.G0 * (y + a.g.G1 * z);
+                    near += row[x1] - row[x0];
+                }
             }
-            const float ex = qx - x, ey = qy - y, ez = qz - z;
-            const float rq = (kbc + sqrtf(ex * ex + ey * ey + ez * ez) * 1.00002f) * 1.00002f + 1e-7f;
-            unsigned long long T = ((unsigned long long)__float_as_uint(rq * rq * 1.00002f) << 32) | 0xffffffffull;
-            if (a.seed && has) {
-                const unsigned long long sd = a.seed[qi];
-                T = sd < T ? sd : T;
-            }
-            TopK<KMAX> top;
-            top.init_bound(k, T);
-            int staged = 0;
-            auto rank = [&]() {
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) near += __shfl_xor_sync(FULL, near, o);
+        // (a one-cell grid is read whole)
+        float hi2 = a.levels > 0 ? fminf(__fdividef(kNearFirst * (float)k, (float)near), kNearMost) * (h * h) : INFINITY;
+        if (seed2 <= widest * widest) hi2 = seed2;
+        float lo2 = -1.f;  // the round reads the points with lo2 < d2 <= hi2
+        while (__any_sync(FULL, search)) {
+            // the rows (y, z) of cells within the radius
+            const float out2 = hi2 * 1.00001f, reach = sqrt_up(hi2) + eps;
+            const int y0 = cell_coord(qy - reach, a.g.lo1, a.g.inv_h, a.g.G1);
+            const int ny = cell_coord(qy + reach, a.g.lo1, a.g.inv_h, a.g.G1) - y0 + 1;
+            const int z0 = cell_coord(qz - reach, a.g.lo2, a.g.inv_h, a.g.G2);
+            const int nrow = search ? ny * (cell_coord(qz + reach, a.g.lo2, a.g.inv_h, a.g.G2) - z0 + 1) : 0;
+            // row i is (i % ny, i / ny), i / ny = i * inv >> 16 (i < 2^8)
+            const unsigned inv = (unsigned)__fdividef(65536.f, (float)ny) + 1u;
+            const float by = a.g.lo1 + (float)y0 * h - eps - qy, bz = a.g.lo2 + (float)z0 * h - eps - qz;
+            const float wide = h + 2.f * eps;
+            for (int rb = 0; __any_sync(FULL, rb < nrow); rb += G * kNearRuns) {
+                // the lane's runs of this batch of rows
+                int s[kNearRuns], e[kNearRuns];
+#pragma unroll
+                for (int u = 0; u < kNearRuns; ++u) {
+                    const int i = rb + u * G + sub;
+                    s[u] = e[u] = 0;
+                    if (i < nrow) {
+                        const int iz = (int)((unsigned)i * inv >> 16), iy = i - iz * ny;
+                        // distance of the row's (eps-widened) face
+                        const float fy = by + (float)iy * h, fz = bz + (float)iz * h;
+                        const float ddy = fmaxf(0.f, fmaxf(fy, -fy - wide));
+                        const float ddz = fmaxf(0.f, fmaxf(fz, -fz - wide));
+                        const float rest = out2 - (ddy * ddy + ddz * ddz);
+                        if (rest >= 0.f) {
+                            const float hx = sqrt_up(rest) + eps;
+                            const int* row = a.cell_start + a.g.G0 * (y0 + iy + a.g.G1 * (z0 + iz));
+                            s[u] = row[cell_coord(qx - hx, a.g.lo0, a.g.inv_h, a.g.G0)];
+                            e[u] = row[cell_coord(qx + hx, a.g.lo0, a.g.inv_h, a.g.G0) + 1];
+                        }
+                    }
+                }
+                // the query's runs as one list, walked by its lanes a point
+                // each: run r holds the points up to run[r].y of the list, at
+                // their position in it + run[r].x
+                int nr = 0, np = 0;
+#pragma unroll
+                for (int u = 0; u < kNearRuns; ++u) {
+                    nr += s[u] < e[u] ? 1 : 0;
+                    np += e[u] - s[u];
+                }
+                int r = nr, all = np;
+#pragma unroll
+                for (int o = 1; o < G; o <<= 1) {
+                    const int pr = __shfl_up_sync(FULL, r, o, G), pp = __shfl_up_sync(FULL, all, o, G);
+                    if (sub >= o) {
+                        r += pr;
+                        all += pp;
+                    }
+                }
+                r -= nr;
+                int at = all - np;
+                all = __shfl_sync(FULL, all, G - 1, G);
+#pragma unroll
+                for (int u = 0; u < kNearRuns; ++u)
+                    if (s[u] < e[u]) {
+                        run[r++] = make_int2(s[u] - at, at + e[u] - s[u]);
+                        at += e[u] - s[u];
+                    }
                 __syncwarp();
-                if (has) {
-                    for (int t = sl; t < staged; t += G) {
-                        const float4 pp = stage[w][t];
-                        const float d2 = sq3_rn(__fsub_rn(pp.x, qx), __fsub_rn(pp.y, qy), __fsub_rn(pp.z, qz));
-                        const unsigned long long v = ((unsigned long long)__float_as_uint(d2) << 32) |
-                                                     (unsigned)__float_as_int(pp.w);
-                        if (v < top.mx) top.push(v, k);
-                    }
+                // the next point is loaded while one is tested
+                int i = sub;
+                float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+                const int2* in_run = run;
+                int2 g = make_int2(0, 0);
+                if (i < all) {
+                    g = *in_run;
+                    while (i >= g.y) g = *++in_run;
+                    p = a.pts[i + g.x];
                 }
-                __syncwarp();
-                staged = 0;
-            };
-            // frontier entries are cells (level 0) or nodes of level fl,
-            // cubes of side 2^fl cells
-            const int side = 1 << fl;
-            const long long per = (long long)side * side * side;
-            const long long total = (long long)nf * per;
-            for (long long b = 0; b < total; b += 32) {
-                const long long t = b + lane;
-                int s0 = 0, cnt = 0;
-                if (t < total) {
-                    int cell;
-                    bool hit = true;
-                    if (fl == 0) {
-                        cell = cur[t];
-                    } else {
-                        const int* D = a.ldim[fl];
-                        const int node = cur[t / per];
-                        const int o = (int)(t % per);
-                        const int ni = node % D[0], nj = (node / D[0]) % D[1], nk = node / (D[0] * D[1]);
-                        const int ui = ni * side + o % side, uj = nj * side + (o / side) % side,
-                                  uk = nk * side + o / (side * side);
-                        hit = cq_node_hit(a, 0, ui, uj, uk, x, y, z, R2, eps);
-                        cell = ui + a.g.G0 * (uj + a.g.G1 * uk);
+                while (__any_sync(FULL, i < all)) {
+                    const float4 c = p;
+                    const bool have = i < all;
+                    i += G;
+                    if (i < all) {
+                        while (i >= g.y) g = *++in_run;
+                        p = a.pts[i + g.x];
                     }
-                    if (hit) {
-                        s0 = a.cell_start[cell];
-                        cnt = a.cell_start[cell + 1] - s0;
-                    }
+                    const float d2 = sq3_rn(__fsub_rn(c.x, qx), __fsub_rn(c.y, qy), __fsub_rn(c.z, qz));
+                    const bool in = have && d2 > lo2 && d2 <= hi2;
+                    const unsigned m = __ballot_sync(FULL, in);
+                    const int pos = found + __popc(m & before);
+                    if (in && pos < kNearKeys)
+                        key[pos] = __hiloint2double(__float_as_int(d2), __float_as_int(c.w));
+                    found += __popc(m & mine);
                 }
-                // the points of the 32 cells as one list that the lanes walk
-                // together, a lane per point (not a lane per cell, which
-                // would idle the warp on the fullest cell)
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const int excl = incl - cnt;
-                const int tot = __shfl_sync(FULL, incl, 31);
-                for (int pb = 0; pb < tot; pb += 32) {
-                    const int tp = pb + lane;
-                    // owner of list position tp: the last lane whose range starts at or before it
-                    int own = 0;
-#pragma unroll
-                    for (int st = 16; st > 0; st >>= 1) {
-                        const int e = __shfl_sync(FULL, excl, own + st);
-                        if (e <= tp) own += st;
-                    }
-                    const int os0 = __shfl_sync(FULL, s0, own);
-                    const int oex = __shfl_sync(FULL, excl, own);
-                    bool keep = false;
-                    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (tp < tot) {
-                        p = a.pts[os0 + (tp - oex)];
-                        const float px = p.x - x, py = p.y - y, pz = p.z - z;
-                        keep = px * px + py * py + pz * pz <= R2;
-                    }
-                    const unsigned bal = __ballot_sync(FULL, keep);
-                    if (keep) stage[w][staged + __popc(bal & below)] = p;
-                    staged += __popc(bal);
-                    if (staged > kCqChunk - 32) rank();
-                }
+                __syncwarp();  // the list is read before the next batch's
             }
-            if (staged > 0) rank();
-            top.sort();
-            if (G == 1) {
-                if (has) {
-#pragma unroll
-                    for (int t = 0; t < KMAX; ++t) {
-                        const int o = t - (KMAX - k);
-                        if (o >= 0)
-                            a.out[qi * k + o] = top.e[t] == NONE ? -1 : (int)(unsigned)(top.e[t] & 0xffffffffu);
+            if (search) {
+                // k points within the radius, or everything was read
+                search = found < k && hi2 < INFINITY;
+                if (search) {
+                    lo2 = hi2;
+                    hi2 *= 2.25f;
+                    if (hi2 > widest * widest) {
+                        wait = true;
+                        search = false;
                     }
-                }
-            } else {
-                // slots >= k hold 0 and sort first: drop them, then k rounds
-                // of the minimum over the G lanes' smallest keys (aligned
-                // groups, so the butterfly stays inside the group); the lane
-                // holding it drops it.  Keys are unique (one index each), the
-                // initial key T and NONE aside, which give -1 as before.
-#pragma unroll 1
-                for (int z = 0; z < KMAX - k; ++z) top.shift_down();
-#pragma unroll 1
-                for (int r = 0; r < k; ++r) {
-                    unsigned long long m = top.e[0];
-                    for (int o = 1; o < G; o <<= 1) {
-                        const unsigned long long v = __shfl_xor_sync(FULL, m, o);
-                        m = v < m ? v : m;
-                    }
-                    if (top.e[0] == m) top.shift_down();
-                    if (has && sl == 0) a.out[qi * k + r] = m == NONE ? -1 : (int)(unsigned)(m & 0xffffffffu);
+                } else if (found > kNearKeys) {
+                    // more than the buffer holds: the far search, from this radius
+                    wait = true;
+                    seed2 = fminf(seed2, hi2);
                 }
             }
         }
         __syncwarp();
-    }
-}
-
-// ------------------------------------------------------------ deep queries --
-// The queries whose per-thread walk ran past its budget (far from every
-// point, so the walk's bound tightens late), one warp per query, level by
-// level down the occupancy pyramid.  The frontier holds the nodes that may
-// contain one of the k nearest; a level's children come from the nodes'
-// child masks, and a child stays when its (eps-widened) box is within the
-// bound U of the query.  After each level U is lowered to the k-th smallest,
-// over the lanes, of each lane's smallest far-corner distance among the
-// children it kept: those are k distinct occupied nodes, so k points lie
-// within it.  At the cells, every lane ranks the points of its share of the
-// cells within U, and the 32 lanes' sets are merged.  A level whose children
-// do not fit the frontier is retried once with the lowered U; if they still
-// do not fit, the cells under the current level's nodes are enumerated.
-constexpr int kDeepWarps = 4;
-constexpr int kDeepNodes = 1024;
-
-// k-th smallest (1 <= k <= 32) of one value per lane, to every lane
-__device__ __forceinline__ float warp_kth_smallest(float v, int k) {
-    const int lane = threadIdx.x & 31;
+        if (wait) found = 0;
+        // a key's rank among the query's keys is its place in the answer
+        for (int b = 0; __any_sync(FULL, b < found); b += 4 * G) {
+            double v[4];
+            int rank[4];
 #pragma unroll
-    for (int size = 2; size <= 32; size <<= 1) {
+            for (int u = 0; u < 4; ++u) {
+                v[u] = b + u * G + sub < found ? key[b + u * G + sub] : 0.0;
+                rank[u] = 0;
+            }
+            for (int i = 0; i < found; ++i) {
+                const double o = key[i];
 #pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            const float o = __shfl_xor_sync(0xffffffffu, v, stride);
-            const bool asc = (lane & size) == 0 || size == 32;
-            const bool low = (lane & stride) == 0;
-            v = (low == asc) ? fminf(v, o) : fmaxf(v, o);
+                for (int u = 0; u < 4; ++u) rank[u] += o < v[u] ? 1 : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (b + u * G + sub < found && rank[u] < k)
+                    a.out[qi * k + rank[u]] = __double2loint(v[u]);
         }
+        if (has && !wait)
+            for (int i = found + sub; i < k; i += G) a.out[qi * k + i] = -1;
+        const unsigned wm = __ballot_sync(FULL, wait && sub == 0);
+        if (wm) {
+            if (wait && sub == 0) {
+                const int o = nfar + __popc(wm & ((1u << lane) - 1u));
+                far[w].q[o] = make_float4(qx, qy, qz, __int_as_float((int)qi));
+                far[w].bound[o] = seed2;
+            }
+            nfar += __popc(wm);
+            __syncwarp();
+            if (nfar >= 32) {
+                far_groups(a, far[w], 32, lane);
+                nfar -= 32;
+                if (lane < nfar) {
+                    far[w].q[lane] = far[w].q[32 + lane];
+                    far[w].bound[lane] = far[w].bound[32 + lane];
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();  // the keys are read before the next queries'
     }
-    return __shfl_sync(0xffffffffu, v, k - 1);
 }
 
-// squared distances from q to the nearest and the farthest point of the
-// eps-widened box of node (ni, nj, nk) of level l
-__device__ __forceinline__ void node_d2(const KnnArgs& a, int l, int ni, int nj, int nk, float qx, float qy, float qz,
-                                        float eps, float& mind2, float& maxd2) {
-    const float h = a.g.h;
-    const float x0 = a.g.lo0 + (float)(ni << l) * h - eps, x1 = a.g.lo0 + (float)((ni + 1) << l) * h + eps;
-    const float y0 = a.g.lo1 + (float)(nj << l) * h - eps, y1 = a.g.lo1 + (float)((nj + 1) << l) * h + eps;
-    const float z0 = a.g.lo2 + (float)(nk << l) * h - eps, z1 = a.g.lo2 + (float)((nk + 1) << l) * h + eps;
-    const float dx = fmaxf(0.f, fmaxf(x0 - qx, qx - x1)), fx = fmaxf(qx - x0, x1 - qx);
-    const float dy = fmaxf(0.f, fmaxf(y0 - qy, qy - y1)), fy = fmaxf(qy - y0, y1 - qy);
-    const float dz = fmaxf(0.f, fmaxf(z0 - qz, qz - z1)), fz = fmaxf(qz - z0, z1 - qz);
-    mind2 = dx * dx + dy * dy + dz * dz;
-    maxd2 = fx * fx + fy * fy + fz * fz;
+// --------------------------------------------------------- far queries --
+// The queries that k_knn_near passed on, in groups of up to 32 near each
+// other, a warp per group and a lane per query.  The warp walks the occupancy
+// pyramid once for the group, depth first, the children nearest to the
+// group's centre first: a node is opened when its (eps-widened) box lies
+// within the k-th distance of some lane's query, tested when it is popped,
+// with the bounds reached by then.  Below level 2 the points of the node's
+// 4x4x4 cells (16 runs, a lane each) are gathered at once, those within the
+// group's reach staged in shared memory, and every lane ranks them for its
+// own query: the walk is a chain of dependent loads, and fewer, wider steps
+// shorten it.  Groups stay narrow (far_groups) because a wide one opens the
+// nodes of all its queries in turn, and the longest group is the launch's
+// time.  A million queries around a 1 M-point torus, a quarter of them off the
+// surface: 5.6 ms here and 1.1 ms in k_knn_near (125 ms with a warp per cell).
+constexpr int kFarWarps = 4;
+constexpr int kFarStack = 8 * KnnIndex::kMaxLevels;  // 7 siblings left per level, and the last 8
+constexpr int kFarLeaf = 2;                          // the level whose nodes are read whole
+
+// (level, child mask) and coordinates (10 bits each) of a node
+__device__ __forceinline__ int2 far_entry(int i, int j, int k, int level, unsigned mask) {
+    return make_int2(i | (j << 10) | (k << 20), level | (int)(mask << 8));
 }
 
-__device__ __forceinline__ int pack3(int i, int j, int k) { return i | (j << 10) | (k << 20); }
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
 
 template <int KMAX>
-__global__ void __launch_bounds__(kDeepWarps * 32) k_knn_deep(KnnArgs a, const int* __restrict__ list,
-                                                             const float* __restrict__ bound,
-                                                             const int* __restrict__ count, int* __restrict__ work) {
-    __shared__ int fco[kDeepWarps][2][kDeepNodes];
-    __shared__ unsigned char fmk[kDeepWarps][2][kDeepNodes];
+__global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned int* __restrict__ work) {
+    __shared__ int2 stack[kFarWarps][kFarStack];
+    __shared__ float4 stage[kFarWarps][32];
     if (a.gate_count && *a.gate_count <= a.gate_min) return;
     const unsigned FULL = 0xffffffffu;
     const unsigned long long NONE = ~0ull;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
-    const int nd = *count;
+    const unsigned ng = a.far_count[1];
     const int k = a.k;
-    const float eps = 1e-4f * a.g.h + 1e-6f;
+    const float h = a.g.h;
+    const float eps = 1e-4f * h + 1e-6f;
     for (;;) {
-        int j = 0;
-        if (lane == 0) j = atomicAdd(work, 1);
-        j = __shfl_sync(FULL, j, 0);
-        if (j >= nd) break;
-        const long long qi = list[j];
+        unsigned g = 0;
+        if (lane == 0) g = atomicAdd(work, 1u);
+        g = __shfl_sync(FULL, g, 0);
+        if (g >= ng) break;
+        const int2 gr = a.far_group[g];
+        const bool has = lane < gr.y;
+        // lanes without a query stand on the group's first
+        const unsigned at = (unsigned)gr.x + (has ? lane : 0);
+        const long long qi = a.far_list[at];
         float qx, qy, qz;
         knn_load_query(a, qi, qx, qy, qz);
-        int* cur = fco[w][0];
-        unsigned char* curm = fmk[w][0];
-        int* nxt = fco[w][1];
-        unsigned char* nxtm = fmk[w][1];
-        int lvl = a.levels;
-        if (lane == 0) {
-            cur[0] = 0;
-            curm[0] = a.occ[a.loff[lvl]];
-        }
-        int nf = 1;
-        float U2 = bound[j];  // from the per-thread walk
-        __syncwarp();
-        while (lvl > 0) {
-            const int nl = lvl - 1;
-            const int* D = a.ldim[nl];
-            int nn = 0;
-            for (int pass = 0; pass < 2; ++pass) {
-                float lmin = INFINITY;
-                nn = 0;
-                for (int b = 0; b < nf * 8; b += 32) {
-                    const int t = b + lane;
-                    bool keep = false;
-                    int cc = 0;
-                    unsigned char cm = 0;
-                    if (t < nf * 8 && ((curm[t >> 3] >> (t & 7)) & 1)) {
-                        const int pc = cur[t >> 3], oc = t & 7;
-                        const int ni = ((pc & 1023) << 1) | (oc & 1), nj = (((pc >> 10) & 1023) << 1) | ((oc >> 1) & 1),
-                                  nk = ((pc >> 20) << 1) | (oc >> 2);
-                        float mind2, maxd2;
-                        node_d2(a, nl, ni, nj, nk, qx, qy, qz, eps, mind2, maxd2);
-                        if (mind2 <= U2) {
-                            keep = true;
-                            lmin = fminf(lmin, maxd2);
-                            cc = pack3(ni, nj, nk);
-                            if (nl > 0) cm = a.occ[a.loff[nl] + ni + (long long)D[0] * (nj + (long long)D[1] * nk)];
-                        }
-                    }
-                    const unsigned bal = __ballot_sync(FULL, keep);
-                    const int pos = nn + __popc(bal & below);
-                    if (keep && pos < kDeepNodes) {
-                        nxt[pos] = cc;
-                        nxtm[pos] = cm;
-                    }
-                    nn += __popc(bal);
-                }
-                const float kth = warp_kth_smallest(lmin, k);
-                if (kth < INFINITY) U2 = fminf(U2, kth * 1.0001f);
-                if (nn <= kDeepNodes) break;
+        const float U2 = a.far_bound[at];
+        SortedK<KMAX> top;
+        // (a lane without a query takes no key)
+        top.init(k, !has ? 0ull
+                         : U2 < INFINITY ? ((unsigned long long)__float_as_uint(U2) << 32) | 0xffffffffull : NONE);
+        // the group's box and its centre
+        float lo[3] = {qx, qy, qz}, hi[3] = {qx, qy, qz};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
+                hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
             }
-            __syncwarp();
-            if (nn > kDeepNodes) break;  // the cells under this level's nodes are enumerated below
-            int* ti = cur;
-            cur = nxt;
-            nxt = ti;
-            unsigned char* tm = curm;
-            curm = nxtm;
-            nxtm = tm;
-            nf = nn;
-            lvl = nl;
-        }
-        // rank the points of the cells within U (cells of the frontier, or
-        // under its nodes of level lvl), a lane per point of 32 cells at a time
-        TopK<KMAX> top;
-        if (U2 < INFINITY)
-            top.init_bound(k, ((unsigned long long)__float_as_uint(U2) << 32) | 0xffffffffull);
-        else
-            top.init(k);
-        const int side = 1 << lvl;
-        const long long per = (long long)side * side * side;
-        const long long total = (long long)nf * per;
-        for (long long b = 0; b < total; b += 32) {
-            const long long t = b + lane;
+        const float mx = 0.5f * (lo[0] + hi[0]), my = 0.5f * (lo[1] + hi[1]), mz = 0.5f * (lo[2] + hi[2]);
+        if (lane == 0) stack[w][0] = far_entry(0, 0, 0, a.levels, a.occ[a.loff[a.levels]]);
+        int sp = 1;
+        float kd2 = U2 * 1.00001f;  // the lane's bound, and the widest of the group
+        float wide = warp_max(has ? kd2 : 0.f);
+        while (sp > 0) {
+            __syncwarp();  // the entries pushed last, and the stage's readers
+            const int2 en = stack[w][--sp];
+            const int lvl = en.y & 0xff;
+            const int ci = en.x & 1023, cj = (en.x >> 10) & 1023, ck = en.x >> 20;
+            {
+                const float x0 = a.g.lo0 + (float)(ci << lvl) * h - eps, x1 = a.g.lo0 + (float)((ci + 1) << lvl) * h + eps;
+                const float y0 = a.g.lo1 + (float)(cj << lvl) * h - eps, y1 = a.g.lo1 + (float)((cj + 1) << lvl) * h + eps;
+                const float z0 = a.g.lo2 + (float)(ck << lvl) * h - eps, z1 = a.g.lo2 + (float)((ck + 1) << lvl) * h + eps;
+                const float dx = fmaxf(0.f, fmaxf(x0 - qx, qx - x1));
+                const float dy = fmaxf(0.f, fmaxf(y0 - qy, qy - y1));
+                const float dz = fmaxf(0.f, fmaxf(z0 - qz, qz - z1));
+                if (!__any_sync(FULL, has && dx * dx + dy * dy + dz * dz <= kd2)) continue;
+            }
+            if (lvl > kFarLeaf) {
+                // push the occupied children within the group's reach, the
+                // nearest to its centre last; a lane per child
+                const int oc = lane & 7;
+                const float half = (float)(1 << (lvl - 1));
+                const int ni = 2 * ci + (oc & 1), nj = 2 * cj + ((oc >> 1) & 1), nk = 2 * ck + (oc >> 2);
+                bool push = lane < 8 && ((en.y >> (8 + oc)) & 1);
+                unsigned cm = 0;
+                float away = -1.f;
+                if (push) {
+                    const int* D = a.ldim[lvl - 1];
+                    cm = a.occ[a.loff[lvl - 1] + ni + (long long)D[0] * (nj + (long long)D[1] * nk)];
+                    const float side = half * h;
+                    const float x0 = a.g.lo0 + (float)ni * side - eps, x1 = a.g.lo0 + (float)(ni + 1) * side + eps;
+                    const float y0 = a.g.lo1 + (float)nj * side - eps, y1 = a.g.lo1 + (float)(nj + 1) * side + eps;
+                    const float z0 = a.g.lo2 + (float)nk * side - eps, z1 = a.g.lo2 + (float)(nk + 1) * side + eps;
+                    const float dx = fmaxf(0.f, fmaxf(x0 - hi[0], lo[0] - x1));
+                    const float dy = fmaxf(0.f, fmaxf(y0 - hi[1], lo[1] - y1));
+                    const float dz = fmaxf(0.f, fmaxf(z0 - hi[2], lo[2] - z1));
+                    push = dx * dx + dy * dy + dz * dz <= wide;
+                    const float ax = 0.5f * (x0 + x1) - mx, ay = 0.5f * (y0 + y1) - my, az = 0.5f * (z0 + z1) - mz;
+                    if (push) away = ax * ax + ay * ay + az * az;
+                }
+                int place = sp;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float o = __shfl_sync(FULL, away, u);
+                    place += o > away || (o == away && u < lane) ? 1 : 0;
+                }
+                if (push) stack[w][place] = far_entry(ni, nj, nk, lvl - 1, cm);
+                sp += __popc(__ballot_sync(FULL, push));
+                continue;
+            }
+            // the rows of the node's cells, a lane each
+            const int side = 1 << lvl;
             int s0 = 0, cnt = 0;
-            if (t < total) {
-                const int pc = cur[t / per];
-                const int o = (int)(t % per);
-                const int ci = (pc & 1023) * side + o % side, cj = ((pc >> 10) & 1023) * side + (o / side) % side,
-                          ck = (pc >> 20) * side + o / (side * side);
-                if (ci < a.g.G0 && cj < a.g.G1 && ck < a.g.G2) {
-                    float mind2, maxd2;
-                    node_d2(a, 0, ci, cj, ck, qx, qy, qz, eps, mind2, maxd2);
-                    if (mind2 <= U2) {
-                        const int cell = ci + a.g.G0 * (cj + a.g.G1 * ck);
-                        s0 = a.cell_start[cell];
-                        cnt = a.cell_start[cell + 1] - s0;
-                    }
+            if (lane < side * side) {
+                const int x = ci << lvl, y = (cj << lvl) + (lane & (side - 1)), z = (ck << lvl) + (lane >> lvl);
+                if (y < a.g.G1 && z < a.g.G2) {
+                    const int row = a.g.G0 * (y + a.g.G1 * z);
+                    s0 = a.cell_start[row + x];
+                    cnt = a.cell_start[row + min(x + side, a.g.G0)] - s0;
                 }
             }
             int incl = cnt;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
+            for (int o = 1; o < 16; o <<= 1) {
                 const int v = __shfl_up_sync(FULL, incl, o);
                 if (lane >= o) incl += v;
             }
-            const int excl = incl - cnt;
-            const int tot = __shfl_sync(FULL, incl, 31);
-            for (int pb = 0; pb < tot; pb += 32) {
-                const int tp = pb + lane;
+            const int excl = incl - cnt, tot = __shfl_sync(FULL, incl, 15);
+            for (int b = 0; b < tot; b += 32) {
+                const int t = b + lane;
+                // the run that holds point t: the last one that starts at or before it
                 int own = 0;
 #pragma unroll
-                for (int st = 16; st > 0; st >>= 1) {
+                for (int st = 8; st > 0; st >>= 1) {
                     const int e = __shfl_sync(FULL, excl, own + st);
-                    if (e <= tp) own += st;
+                    if (e <= t) own += st;
                 }
-                const int os0 = __shfl_sync(FULL, s0, own);
-                const int oex = __shfl_sync(FULL, excl, own);
-                if (tp < tot) {
-                    const float4 pp = a.pts[os0 + (tp - oex)];
-                    const float d2 = sq3_rn(__fsub_rn(pp.x, qx), __fsub_rn(pp.y, qy), __fsub_rn(pp.z, qz));
-                    const unsigned long long v = ((unsigned long long)__float_as_uint(d2) << 32) |
-                                                 (unsigned)__float_as_int(pp.w);
-                    if (v < top.mx) top.push(v, k);
+                const int ps = __shfl_sync(FULL, s0, own), po = __shfl_sync(FULL, excl, own);
+                bool keep = false;
+                float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (t < tot) {
+                    p = a.pts[ps + (t - po)];
+                    const float dx = fmaxf(0.f, fmaxf(lo[0] - p.x, p.x - hi[0]));
+                    const float dy = fmaxf(0.f, fmaxf(lo[1] - p.y, p.y - hi[1]));
+                    const float dz = fmaxf(0.f, fmaxf(lo[2] - p.z, p.z - hi[2]));
+                    keep = dx * dx + dy * dy + dz * dz <= wide;
                 }
-            }
-        }
-        // merge the 32 lanes' sets (as in k_knn_cells)
-        top.sort();
-#pragma unroll 1
-        for (int z = 0; z < KMAX - k; ++z) top.shift_down();
-#pragma unroll 1
-        for (int r = 0; r < k; ++r) {
-            unsigned long long m = top.e[0];
+                const unsigned km = __ballot_sync(FULL, keep);
+                if (keep) stage[w][__popc(km & below)] = p;
+                __syncwarp();
+                // four at a time: their distances do not wait for one another
+                const int m = __popc(km);
+                if (lane < 4 && m < 32) stage[w][m + lane < 32 ? m + lane : 31] = make_float4(INFINITY, 0.f, 0.f, 0.f);
+                __syncwarp();
+                for (int i = 0; i < m; i += 4) {
+                    float d2[4];
+                    int id[4];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long v = __shfl_xor_sync(FULL, m, o);
-                m = v < m ? v : m;
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 c = stage[w][i + u];
+                        d2[u] = sq3_rn(__fsub_rn(c.x, qx), __fsub_rn(c.y, qy), __fsub_rn(c.z, qz));
+                        id[u] = __float_as_int(c.w);
+                    }
+                    if (fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])) <= kd2) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const unsigned long long v =
+                                ((unsigned long long)__float_as_uint(d2[u]) << 32) | (unsigned)id[u];
+                            if (i + u < m && v < top.last()) top.insert(v);
+                        }
+                        kd2 = top.last() == NONE ? INFINITY : top.last_d2() * 1.00001f;
+                    }
+                }
+                __syncwarp();
             }
-            if (top.e[0] == m) top.shift_down();
-            if (lane == 0) a.out[qi * k + r] = m == NONE ? -1 : (int)(unsigned)(m & 0xffffffffu);
+            wide = warp_max(has ? kd2 : 0.f);
         }
-        __syncwarp();
+        if (has) top.store(a.out + qi * k, k);
     }
 }
 
@@ -1410,101 +1167,32 @@ static int knn_launch(const KnnArgs& a, long long nq, cudaStream_t s) {
 }
 
 template <int KMAX>
-static int cells_launch(const KnnIndex& ix, const KnnArgs& a, long long nq, const unsigned int* sbits,
-                        cudaStream_t s) {
+static int near_launch(const KnnIndex& ix, const KnnArgs& a, long long nq, cudaStream_t s) {
     static int bps = 0;
     if (!bps) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_knn_cells<KMAX>, kCqWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_knn_near, kNearThreads, 0);
         if (bps <= 0) bps = 1;
     }
-    const long long grid = (long long)num_sms() * bps;
-    k_knn_cells<KMAX><<<(unsigned)grid, kCqWarps * 32, 0, s>>>(
-        a, ix.c_active.ptr, ix.c_misc.ptr, ix.c_start.ptr, ix.c_count.ptr, ix.c_m.ptr, sbits, ix.kb.ptr, ix.q_order.ptr,
-        ix.c_misc.ptr + 1, ix.c_fb.ptr);
+    long long blocks = (nq + kNearThreads - 1) / kNearThreads;
+    if (blocks > (long long)num_sms() * bps) blocks = (long long)num_sms() * bps;
+    k_knn_near<<<(unsigned)blocks, kNearThreads, 0, s>>>(a, (unsigned int*)ix.q_misc.ptr);
     DWG_CHECK_LAUNCH();
-    // the queries of cells whose candidate sets did not fit, per thread;
-    // those far from every point finish one warp each
-    KnnArgs f = a;
-    f.order = ix.c_fb.ptr;
-    f.nq_dev_i32 = ix.c_misc.ptr + 2;
-    f.kb = ix.kb.ptr;
-    f.deep = ix.levels > 0 ? ix.c_deep.ptr : nullptr;
-    f.deep_bound = ix.c_deep_bound.ptr;
-    f.deep_count = ix.c_misc.ptr + 3;
-    DWG_TRY(knn_launch<KMAX>(f, nq, s));
-    if (f.deep) {
-        static int dbps = 0;
-        if (!dbps) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dbps, k_knn_deep<KMAX>, kDeepWarps * 32, 0);
-            if (dbps <= 0) dbps = 1;
-        }
-        k_knn_deep<KMAX><<<(unsigned)(num_sms() * dbps), kDeepWarps * 32, 0, s>>>(
-            f, ix.c_deep.ptr, ix.c_deep_bound.ptr, ix.c_misc.ptr + 3, ix.c_misc.ptr + 4);
-        DWG_CHECK_LAUNCH();
+    // the queries far from the points, or in sparse neighbourhoods
+    static int fbps = 0;
+    if (!fbps) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fbps, k_knn_far<KMAX>, kFarWarps * 32, 0);
+        if (fbps <= 0) fbps = 1;
     }
+    if (blocks > (long long)num_sms() * fbps) blocks = (long long)num_sms() * fbps;
+    k_knn_far<KMAX><<<(unsigned)blocks, kFarWarps * 32, 0, s>>>(a, (unsigned int*)ix.q_misc.ptr + 3);
+    DWG_CHECK_LAUNCH();
     return DWG_OK;
-}
-
-// queries grouped by cell (k <= 16, no exclusion), see k_knn_cells
-static int knn_query_cells(const KnnIndex& ix, const KnnArgs& a0, long long nq, cudaStream_t s) {
-    if (!ix.kb_per_query && !ix.kb_ready) DWG_TRY(build_kbound(ix, s));
-    const long long ncell = (long long)ix.G[0] * ix.G[1] * ix.G[2];
-    DWG_TRY(ix.c_count.reserve(ncell + 1));
-    DWG_TRY(ix.c_start.reserve(ncell + 1));
-    DWG_TRY(ix.c_fill.reserve(ncell + 1));
-    DWG_TRY(ix.c_m.reserve(ncell));
-    DWG_TRY(ix.c_active.reserve(ncell));
-    DWG_TRY(ix.c_misc.reserve(8));
-    DWG_TRY(ix.q_key.reserve(nq));
-    DWG_TRY(ix.q_order.reserve(nq));
-    DWG_TRY(ix.c_fb.reserve(nq));
-    DWG_TRY(ix.c_deep.reserve(nq));
-    DWG_TRY(ix.c_deep_bound.reserve(nq));
-    DWG_CHECK_CUDA(cudaMemsetAsync(ix.c_count.ptr, 0, sizeof(int) * (ncell + 1), s));
-    DWG_CHECK_CUDA(cudaMemsetAsync(ix.c_m.ptr, 0, sizeof(unsigned int) * ncell, s));
-    unsigned int* sbits = nullptr;
-    if (a0.seed) {
-        DWG_TRY(ix.c_s.reserve(ncell));
-        DWG_CHECK_CUDA(cudaMemsetAsync(ix.c_s.ptr, 0, sizeof(unsigned int) * ncell, s));
-        sbits = ix.c_s.ptr;
-    }
-    DWG_CHECK_CUDA(cudaMemsetAsync(ix.c_misc.ptr, 0, sizeof(int) * 8, s));
-    KnnArgs a = a0;
-    long long blocks = (nq + 255) / 256;
-    const long long cap = (long long)num_sms() * 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    k_cq_key<<<(unsigned)blocks, 256, 0, s>>>(a, ix.q_key.ptr, ix.c_count.ptr, ix.c_m.ptr, sbits);
-    DWG_CHECK_LAUNCH();
-    size_t bytes = 0;
-    int* cin = ix.c_count.ptr;
-    int* cout = ix.c_start.ptr;
-    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, cin, cout, (int)(ncell + 1), s));
-    DWG_TRY(ix.c_scratch.reserve(bytes + 256));
-    bytes = ix.c_scratch.n;
-    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(ix.c_scratch.ptr, bytes, cin, cout, (int)(ncell + 1), s));
-    DWG_CHECK_CUDA(cudaMemcpyAsync(ix.c_fill.ptr, ix.c_start.ptr, sizeof(int) * (ncell + 1), cudaMemcpyDeviceToDevice, s));
-    k_cq_active<<<div_up(ncell, 256), 256, 0, s>>>(ix.c_count.ptr, ncell, ix.c_active.ptr, ix.c_misc.ptr);
-    if (ix.kb_per_query) {
-        DWG_TRY(ix.kb.reserve(ncell));
-        KnnGrid g{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h};
-        const unsigned char* occ1 = ix.levels >= 1 ? ix.occ.ptr + ix.loff[1] : nullptr;
-        k_kb_active<<<num_sms() * 4, 128, 0, s>>>(g, ix.cell_start.ptr, ix.pts.ptr, occ1, ix.ldim[1][0],
-                                                  ix.ldim[1][1], ix.c_active.ptr, ix.c_misc.ptr, sbits, ix.kb.ptr);
-    }
-    k_cq_scatter<<<(unsigned)blocks, 256, 0, s>>>(a, ix.q_key.ptr, ix.c_fill.ptr, ix.q_order.ptr);
-    DWG_CHECK_LAUNCH();
-    // k = 15 (the triangle queries) keeps 15 slots per lane instead of 16 and
-    // k <= 10 (the zero repair) 10: every maximum search and the final sort
-    // are shorter, and the lanes hold fewer registers
-    if (a.k == 15) return cells_launch<15>(ix, a, nq, sbits, s);
-    if (a.k <= 10) return cells_launch<10>(ix, a, nq, sbits, s);
-    return cells_launch<16>(ix, a, nq, sbits, s);
 }
 
 // ------------------------------------------------------------- subsets --
 __global__ void k_sub_count(long long ncell, const int* __restrict__ cs, const float4* __restrict__ pts,
-                            const unsigned char* __restrict__ exclude, int* __restrict__ count) {
+                            const unsigned char* __restrict__ exclude, int* __restrict__ count, Gate gate) {
+    if (gate.closed()) return;
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c > ncell) return;
     int m = 0;
@@ -1517,7 +1205,8 @@ __global__ void k_sub_count(long long ncell, const int* __restrict__ cs, const f
 
 __global__ void k_sub_fill(long long ncell, const int* __restrict__ cs, const float4* __restrict__ pts,
                            const unsigned char* __restrict__ exclude, const int* __restrict__ sub_start,
-                           float4* __restrict__ sub_pts) {
+                           float4* __restrict__ sub_pts, Gate gate) {
+    if (gate.closed()) return;
     const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (c >= ncell) return;
     int o = sub_start[c];
@@ -1528,7 +1217,9 @@ __global__ void k_sub_fill(long long ncell, const int* __restrict__ cs, const fl
     }
 }
 
-int knn_build_subset(const KnnIndex& full, const unsigned char* exclude, KnnIndex& sub, cudaStream_t s) {
+int knn_build_subset(const KnnIndex& full, const unsigned char* exclude, KnnIndex& sub, const int* gate_count,
+                     int gate_min, cudaStream_t s) {
+    const Gate gate{gate_count, gate_min};
     DWG_REQUIRE(exclude && full.n >= 1, "knn subset: bad arguments");
     const long long ncell = (long long)full.G[0] * full.G[1] * full.G[2];
     if (sub.n != full.n || sub.G[0] != full.G[0] || sub.G[1] != full.G[1] || sub.G[2] != full.G[2]) {
@@ -1539,7 +1230,6 @@ int knn_build_subset(const KnnIndex& full, const unsigned char* exclude, KnnInde
         }
         sub.h = full.h;
         sub.inv_h = full.inv_h;
-        sub.morton_shift = full.morton_shift;
         DWG_TRY(sub.cell_start.reserve(ncell + 1));
         DWG_TRY(sub.cell_fill.reserve(ncell + 1));
         DWG_TRY(sub.pts.reserve(full.n));
@@ -1552,27 +1242,17 @@ int knn_build_subset(const KnnIndex& full, const unsigned char* exclude, KnnInde
         DWG_TRY(sub.scratch.reserve(bytes + 256));
     }
     k_sub_count<<<div_up(ncell + 1, 256), 256, 0, s>>>(ncell, full.cell_start.ptr, full.pts.ptr, exclude,
-                                                       sub.cell_fill.ptr);
+                                                       sub.cell_fill.ptr, gate);
     DWG_CHECK_LAUNCH();
     size_t bytes = sub.scratch.n;
     DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(sub.scratch.ptr, bytes, sub.cell_fill.ptr, sub.cell_start.ptr,
                                                  (int)(ncell + 1), s));
     k_sub_fill<<<div_up(ncell, 256), 256, 0, s>>>(ncell, full.cell_start.ptr, full.pts.ptr, exclude,
-                                                  sub.cell_start.ptr, sub.pts.ptr);
+                                                  sub.cell_start.ptr, sub.pts.ptr, gate);
     DWG_CHECK_LAUNCH();
-    DWG_TRY(pyramid_fill(sub, s));
-    // the subset changes between queries.  The whole-grid bound (local blocks
-    // plus min-plus passes) costs in proportion to the grid, empty space
-    // included; past 2^22 cells the bounds of the queried cells alone are
-    // cheaper, at the price of sending the queries of sparse neighbourhoods
-    // to the per-thread search
-    sub.kb_ready = false;
-    sub.kb_per_query = ncell > (1ll << 22);
-    if (!sub.kb_per_query) return build_kbound(sub, s);
+    DWG_TRY(pyramid_fill(sub, gate, s));
     return DWG_OK;
 }
-
-constexpr int kKnnBuckets = 1 << 15;
 
 int knn_query(const KnnIndex& ix, const KnnQuery& q, int k, int* out, cudaStream_t s) {
     DWG_REQUIRE(k >= 1 && k <= 64, "knn: k must be in [1, 64] (got %d)", k);
@@ -1589,12 +1269,11 @@ int knn_query(const KnnIndex& ix, const KnnQuery& q, int k, int* out, cudaStream
     a.nq = q.nq;
     a.nq_dev = q.nq_dev;
     a.nq_dev_i32 = q.nq_dev_i32;
-    a.exclude = q.exclude;
     a.gate_count = q.gate_count;
     a.gate_min = q.gate_min;
     a.k = k;
     a.out = out;
-    a.morton_shift = ix.morton_shift;
+    a.morton_shift = 0;
     a.occ = ix.occ.ptr;
     a.levels = ix.levels;
     for (int l = 0; l < KnnIndex::kMaxLevels; ++l) {
@@ -1602,38 +1281,64 @@ int knn_query(const KnnIndex& ix, const KnnQuery& q, int k, int* out, cudaStream
         for (int t = 0; t < 3; ++t) a.ldim[l][t] = ix.ldim[l][t];
     }
     a.order = nullptr;
-    a.kb = nullptr;
-    a.deep = nullptr;
-    a.deep_bound = nullptr;
-    a.deep_count = nullptr;
+    a.q_key = nullptr;
+    a.q_hist = nullptr;
+    a.far_list = nullptr;
+    a.far_bound = nullptr;
+    a.far_group = nullptr;
+    a.far_count = nullptr;
     a.seed = q.seed;
-    if (k <= kKnnBoundK && !q.exclude && ix.n >= kKnnBoundK && q.use_cells) return knn_query_cells(ix, a, q.nq, s);
-    // bucket the queries spatially (counting sort on device counts, no host sync)
-    DWG_TRY(ix.q_key.reserve(q.nq));
-    DWG_TRY(ix.q_order.reserve(q.nq));
-    DWG_TRY(ix.q_hist.reserve(kKnnBuckets));
-    DWG_TRY(ix.q_fill.reserve(kKnnBuckets));
-    a.q_key = ix.q_key.ptr;
-    a.q_hist = ix.q_hist.ptr;
-    a.order = nullptr;
-    DWG_CHECK_CUDA(cudaMemsetAsync(ix.q_hist.ptr, 0, sizeof(int) * kKnnBuckets, s));
-    long long blocks = (q.nq + 255) / 256;
-    long long cap = (long long)num_sms() * 8;
-    if (blocks > cap) blocks = cap;
-    k_knn_qkey<<<(unsigned)blocks, 256, 0, s>>>(a);
-    DWG_CHECK_LAUNCH();
-    size_t bytes = 0;
-    int* hin = ix.q_hist.ptr;
-    int* hout = ix.q_fill.ptr;
-    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, hin, hout, kKnnBuckets, s));
-    DWG_TRY(ix.q_scratch.reserve(bytes + 256));
-    bytes = ix.q_scratch.n;
-    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(ix.q_scratch.ptr, bytes, hin, hout, kKnnBuckets, s));
-    k_knn_qscatter<<<(unsigned)blocks, 256, 0, s>>>(a, ix.q_fill.ptr, ix.q_order.ptr);
-    DWG_CHECK_LAUNCH();
-    a.order = ix.q_order.ptr;
-    if (k <= 10) return knn_launch<10>(a, q.nq, s);
-    if (k <= 16) return knn_launch<16>(a, q.nq, s);
+    if (!q.coherent) {
+        // bucket the queries spatially (counting sort on device counts, no host sync)
+        DWG_TRY(ix.q_key.reserve(q.nq));
+        DWG_TRY(ix.q_order.reserve(q.nq));
+        // buckets per axis: the grid's cells, at most 128 (32 for few queries,
+        // whose buckets then hold several: clearing and scanning 2^21 counts
+        // takes 10 us)
+        const int gm = max(ix.G[0], max(ix.G[1], ix.G[2]));
+        const int most = q.nq > (1 << 16) ? 7 : 5;
+        int bits = 0;
+        while ((1 << bits) < gm && bits < most) ++bits;
+        a.morton_shift = 0;
+        while ((gm - 1) >> (bits + a.morton_shift)) ++a.morton_shift;
+        const int buckets = 1 << (3 * bits);
+        DWG_TRY(ix.q_hist.reserve(buckets));
+        DWG_TRY(ix.q_fill.reserve(buckets));
+        a.q_key = ix.q_key.ptr;
+        a.q_hist = ix.q_hist.ptr;
+        DWG_CHECK_CUDA(cudaMemsetAsync(ix.q_hist.ptr, 0, sizeof(int) * buckets, s));
+        long long blocks = (q.nq + 255) / 256;
+        const long long cap = (long long)num_sms() * 8;
+        if (blocks > cap) blocks = cap;
+        k_knn_qkey<<<(unsigned)blocks, 256, 0, s>>>(a);
+        DWG_CHECK_LAUNCH();
+        size_t bytes = 0;
+        int* hin = ix.q_hist.ptr;
+        int* hout = ix.q_fill.ptr;
+        DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, hin, hout, buckets, s));
+        DWG_TRY(ix.q_scratch.reserve(bytes + 256));
+        bytes = ix.q_scratch.n;
+        DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(ix.q_scratch.ptr, bytes, hin, hout, buckets, s));
+        k_knn_qscatter<<<(unsigned)blocks, 256, 0, s>>>(a, ix.q_fill.ptr, ix.q_order.ptr);
+        DWG_CHECK_LAUNCH();
+        a.order = ix.q_order.ptr;
+    }
+    if (k <= kKnnNearK) {
+        DWG_TRY(ix.q_misc.reserve(4));
+        DWG_TRY(ix.q_far.reserve(q.nq));
+        DWG_TRY(ix.q_far_bound.reserve(q.nq));
+        DWG_TRY(ix.q_far_group.reserve(q.nq));
+        DWG_CHECK_CUDA(cudaMemsetAsync(ix.q_misc.ptr, 0, sizeof(int) * 4, s));
+        a.far_list = ix.q_far.ptr;
+        a.far_bound = ix.q_far_bound.ptr;
+        a.far_group = ix.q_far_group.ptr;
+        a.far_count = (unsigned int*)ix.q_misc.ptr + 1;
+        // k = 15 (the triangle queries) keeps 15 slots per lane instead of 16
+        // and k <= 10 (the zero repair) 10: shorter insertions, fewer registers
+        if (k == 15) return near_launch<15>(ix, a, q.nq, s);
+        if (k <= 10) return near_launch<10>(ix, a, q.nq, s);
+        return near_launch<16>(ix, a, q.nq, s);
+    }
     if (k <= 32) return knn_launch<32>(a, q.nq, s);
     return knn_launch<64>(a, q.nq, s);
 }

@@ -22,28 +22,18 @@ struct KnnIndex {
     int ldim[kMaxLevels][3] = {};
     long long loff[kMaxLevels] = {};
     DevBuf<unsigned char> occ;
-    // kb[c] >= distance from the centre of cell c to its kKnnBoundK-th
-    // nearest point: over the whole grid on the first cell-grouped query, or
-    // (kb_per_query, indexes rebuilt between queries) for the cells holding
-    // queries only, at every query
-    mutable DevBuf<float> kb, kb_tmp;
-    mutable bool kb_ready = false;
-    bool kb_per_query = false;
-    // workspace of the cell-grouped queries
-    mutable DevBuf<int> c_count, c_start, c_fill, c_active, c_misc, c_fb, c_deep;
-    mutable DevBuf<unsigned int> c_m;
-    mutable DevBuf<unsigned int> c_s;  // per cell: largest |q - x_c| + seed radius (seeded queries)
-    mutable DevBuf<float> c_deep_bound;
-    mutable DevBuf<unsigned char> c_scratch;
     // query bucketing workspace (grown on demand; not thread safe)
-    int morton_shift = 0;
     mutable DevBuf<int> q_key, q_order, q_hist, q_fill;
     mutable DevBuf<unsigned char> q_scratch;
+    // queries handed to the far search, their bounds, and the work counters
+    mutable DevBuf<int> q_far, q_misc;
+    mutable DevBuf<float> q_far_bound;
+    mutable DevBuf<int2> q_far_group;
 };
 
 int knn_build(KnnIndex& ix, const float* points_dev, int n, cudaStream_t s);
 
-constexpr int kKnnBoundK = 16;  // queries with k <= 16 and no exclusion use cell grouping
+constexpr int kKnnNearK = 16;  // queries with k <= 16 take k_knn_near and k_knn_far
 
 struct KnnQuery {
     const float* q = nullptr;              // packed xyz, or ...
@@ -52,10 +42,9 @@ struct KnnQuery {
     long long nq = 0;                      // host count, or
     const unsigned long long* nq_dev = nullptr;  // device count (clamped to nq)
     const int* nq_dev_i32 = nullptr;       // device count as int (clamped to nq)
-    const unsigned char* exclude = nullptr;  // skip candidates with exclude[idx] != 0
     const int* gate_count = nullptr;       // run only when *gate_count > gate_min
     int gate_min = 0;
-    bool use_cells = true;                 // allow the cell-grouped search (k <= 16)
+    bool coherent = false;                 // consecutive queries are near each other: no bucketing
     // per query (null: none): a key above the key of its k-th nearest point
     // (squared distance bits << 32 | index), ~0 where there is none; the
     // searches start from it instead of their own bounds where it is lower
@@ -67,7 +56,8 @@ int knn_query(const KnnIndex& ix, const KnnQuery& q, int k, int* out, cudaStream
 
 // sub = the points of `full` with exclude[id] == 0, on the same grid (no
 // host synchronisation: capturable once sub's buffers exist); indices stay
-// those of full
-int knn_build_subset(const KnnIndex& full, const unsigned char* exclude, KnnIndex& sub, cudaStream_t s);
+// those of full.  Nothing is built unless *gate_count > gate_min (null: always).
+int knn_build_subset(const KnnIndex& full, const unsigned char* exclude, KnnIndex& sub, const int* gate_count,
+                     int gate_min, cudaStream_t s);
 
 }  // namespace dwg

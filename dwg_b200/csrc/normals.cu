@@ -125,7 +125,7 @@ __global__ void k_seed_keys(const int* __restrict__ list, const int* __restrict_
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < z; j += gridDim.x * blockDim.x) {
         const int i = list[j];
         const float qx = P[(size_t)i * 3], qy = P[(size_t)i * 3 + 1], qz = P[(size_t)i * 3 + 2];
-        int ids[kKnnBoundK];
+        int ids[kKnnNearK];
         bool ok = true;
         float mx = 0.f;
         for (int t = 0; t < k && ok; ++t) {
@@ -168,7 +168,7 @@ __global__ void k_zero_apply(const int* __restrict__ list, const int* __restrict
 }
 
 int zero_repair(const KnnIndex& ix, const float* pos, int L, float* N, const unsigned char* is_zero, int k,
-                int min_zero, ZeroRepairWs& ws, cudaStream_t s) {
+                int min_zero, ZeroRepairWs& ws, bool spatial_order, cudaStream_t s) {
     DWG_REQUIRE(pos && N && is_zero && L >= 1 && k >= 1 && k <= 64, "zero_repair: bad arguments");
     DWG_TRY(ws.list.reserve(L));
     DWG_TRY(ws.count.reserve(1));
@@ -183,7 +183,7 @@ int zero_repair(const KnnIndex& ix, const float* pos, int L, float* N, const uns
     DWG_CHECK_CUDA(cub::DeviceSelect::Flagged(ws.scratch.ptr, bytes, it, is_zero, lp, cp, L, s));
     // the neighbours are the k nearest among the unflagged points, in key
     // order: the query runs on the index of those points alone
-    DWG_TRY(knn_build_subset(ix, is_zero, ws.sub, s));
+    DWG_TRY(knn_build_subset(ix, is_zero, ws.sub, ws.count.ptr, min_zero, s));
     KnnQuery q;
     q.q_index = ws.list.ptr;
     q.q_source = pos;
@@ -191,11 +191,12 @@ int zero_repair(const KnnIndex& ix, const float* pos, int L, float* N, const uns
     q.nq_dev_i32 = ws.count.ptr;
     q.gate_count = ws.count.ptr;
     q.gate_min = min_zero;
+    q.coherent = spatial_order;  // the list is in point order
     long long blocks = (long long)num_sms() * 4;
     // seeds from the neighbours recorded by earlier calls (k <= 16: the
     // cell-grouped search); the record starts empty
     int* prev = nullptr;
-    if (k <= kKnnBoundK) {
+    if (k <= kKnnNearK) {
         if (!ws.prev.ptr || ws.prev.n < (size_t)L * k || ws.prev_k != k) {
             DWG_TRY(ws.prev.reserve((size_t)L * k));
             DWG_CHECK_CUDA(cudaMemsetAsync(ws.prev.ptr, 0xff, sizeof(int) * (size_t)L * k, s));

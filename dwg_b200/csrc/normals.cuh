@@ -35,7 +35,7 @@ struct ZeroRepairWs {
     int prev_k = 0;
 };
 int zero_repair(const KnnIndex& ix, const float* positions, int L, float* normals, const unsigned char* is_zero,
-                int k, int min_zero, ZeroRepairWs& ws, cudaStream_t s);
+                int k, int min_zero, ZeroRepairWs& ws, bool spatial_order, cudaStream_t s);
 
 // OutlierFilter + AsFiltertoZero (src/TurboDWG.cu:991-1009, :442-454): the
 // ceil(n * thr) largest areas are divided by 1000; equal areas are taken in

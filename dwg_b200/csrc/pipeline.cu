@@ -611,7 +611,7 @@ int Pipeline::iterate_post() {
                                 is_zero.ptr, zero_count.ptr, s));
     }
     // zero-normal repair when more than knn_zero points are zero (:585-644)
-    DWG_TRY(zero_repair(kidx, leaf_pos.ptr, L, leaf_nrm.ptr, is_zero.ptr, prm.knn_zero, prm.knn_zero, zws, s));
+    DWG_TRY(zero_repair(kidx, leaf_pos.ptr, L, leaf_nrm.ptr, is_zero.ptr, prm.knn_zero, prm.knn_zero, zws, true, s));
     k_iter_end<<<1, 1, 0, s>>>(iter_dev.ptr, ntri.ptr, cap, zero_count.ptr, terms_cur.ptr, tri_hist.ptr,
                                zero_hist.ptr, terms_hist.ptr);
     DWG_CHECK_LAUNCH();

@@ -544,3 +544,28 @@ def test_knn_cell_grouped_queries_dense_and_sparse(oracle_lib, k):
     sparse = ix.query(cu(Q[:5000]), k).cpu().numpy()
     assert np.array_equal(dense[:5000], sparse)
     assert np.array_equal(sparse, oracle_lib.knn(P, Q[:5000], k))
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (15, 15), (16, 16), (17, 10), (40, 16), (300, 15), (5000, 10), (5000, 16)])
+def test_knn_near_and_far_rounds(oracle_lib, n, k):
+    # the ends of the near search's range: clouds of one cell and of a few,
+    # more points at one spot than a query keeps keys, exact ties, queries in
+    # empty space and far outside, a warp's part of queries (1, 3, 33), and
+    # queries that are not numbers (no neighbours)
+    rng = np.random.default_rng(100 * n + k)
+    P = rng.normal(size=(n, 3))
+    P = (0.4 * P / np.linalg.norm(P, axis=1, keepdims=True)).astype(np.float32)
+    P[: n // 5] = P[0]  # one spot
+    P[n // 5: n // 3] = np.round(P[n // 5: n // 3] * 16) / 16  # a lattice
+    Q = np.concatenate([P[rng.integers(0, n, 600)], P[rng.integers(0, n, 400)] * rng.uniform(0, 1.5, (400, 1)),
+                        np.round(rng.uniform(-0.5, 0.5, (200, 3)) * 16) / 16, rng.uniform(-3, 3, (100, 3))])
+    Q = np.ascontiguousarray(Q, np.float32)
+    ix = turbo.KnnIndex(cu(P))
+    ref = oracle_lib.knn(P, Q, k)
+    assert np.array_equal(ix.query(cu(Q), k).cpu().numpy(), ref)
+    for m in (1, 3, 33):
+        assert np.array_equal(ix.query(cu(Q[:m]), k).cpu().numpy(), ref[:m])
+    Q[::7, 1] = np.nan
+    got = ix.query(cu(Q), k).cpu().numpy()
+    bad = np.isnan(Q[:, 1])
+    assert np.array_equal(got[~bad], ref[~bad]) and np.all(got[bad] == -1)
