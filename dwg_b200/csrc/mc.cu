@@ -1,11 +1,11 @@
 // mc.cu -- marching cubes, two passes with cell-ordered (deterministic) output.
 //
 // The reference (src/TurboMC.cu:383-478) launches one 12-thread block per cell
-// and appends triangles at atomicAdd slots.  Here pass 1 classifies 256 cells
-// per block and reduces the triangle counts; a scan over blocks gives every
-// block its output offset; pass 2 re-classifies, scans counts inside the block
-// and writes each triangle at its final position, so the triangle order is
-// the cell order (x fastest) -- identical from run to run.
+// and appends triangles at atomicAdd slots.  Here pass 1 counts the triangles
+// of every 256 cells; a scan gives each such block its output offset; pass 2
+// visits the blocks that have triangles and writes each at its final
+// position, so the triangle order is the cell order (x fastest) -- identical
+// from run to run.
 //
 // Conventions kept from the reference: corner c of cell (x,y,z) sits at
 // (x + (b0 != b1), y + b1, z + !b2) (src/TurboMC.cu:408-413); bit c of the case
@@ -17,15 +17,20 @@
 // against the polygons the cube geometry gives (mc_tables_host).
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <mutex>
 
 #include "mc.cuh"
 
 namespace dwg {
 
-__constant__ signed char c_tri[256][16];
+__constant__ __align__(16) signed char c_tri[256][16];
 __constant__ unsigned char c_ntri[256];
 __constant__ unsigned short c_edges[256];
+// the same in global memory, for blocks that stage them in shared memory (a
+// constant load serves one address at a time)
+__device__ __align__(16) signed char g_tri[256][16];
+__device__ __align__(16) unsigned char g_ntri[256];
 
 static const int kCorner[8][3] = {{0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1},
                                   {0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}};
@@ -434,6 +439,8 @@ int mc_upload_tables() {
     DWG_CHECK_CUDA(cudaMemcpyToSymbol(c_tri, tt, sizeof(tt)));
     DWG_CHECK_CUDA(cudaMemcpyToSymbol(c_ntri, nt, sizeof(nt)));
     DWG_CHECK_CUDA(cudaMemcpyToSymbol(c_edges, es, sizeof(es)));
+    DWG_CHECK_CUDA(cudaMemcpyToSymbol(g_tri, tt, sizeof(tt)));
+    DWG_CHECK_CUDA(cudaMemcpyToSymbol(g_ntri, nt, sizeof(nt)));
     if (dev >= 0 && dev < 64) done[dev] = true;
     return DWG_OK;
 }
@@ -485,15 +492,12 @@ __global__ void __launch_bounds__(kMcThreads) k_mc_count(McArgs a, unsigned int*
     if (threadIdx.x == 0) counts[blockIdx.x] = tot;
 }
 
-__global__ void k_mc_total(const unsigned int* __restrict__ counts, const unsigned int* __restrict__ offs,
-                           long long nb, unsigned long long* __restrict__ total) {
-    *total = (unsigned long long)offs[nb - 1] + counts[nb - 1];
-}
-
 __global__ void __launch_bounds__(kMcThreads)
-    k_mc_emit(McArgs a, const unsigned int* __restrict__ offs, long long cap, float* __restrict__ tris,
-              float* __restrict__ cen, float* __restrict__ nrm) {
+    k_mc_emit_cells(McArgs a, const unsigned int* __restrict__ offs, long long cap, float* __restrict__ tris,
+              float* __restrict__ cen, float* __restrict__ nrm,
+                    long long nb, const unsigned int* __restrict__ counts, unsigned long long* __restrict__ total) {
     const float iso = a.iso_dev ? *a.iso_dev : a.iso;
+    if (total && blockIdx.x == 0 && threadIdx.x == 0) *total = (unsigned long long)offs[nb - 1] + counts[nb - 1];
     long long cell = (long long)blockIdx.x * kMcThreads + threadIdx.x;
     int x = 0, y = 0, z = 0, ci = 0;
     float v[8];
@@ -580,6 +584,343 @@ __global__ void __launch_bounds__(kMcThreads)
     }
 }
 
+// Grids with rows of kMcThinRow cells and more: rows are cut into segments of
+// 31 cells (the 32 samples of a warp's lanes), eight consecutive segments (in
+// cell order) are a unit of the output.
+//
+// Count: a warp marches a segment kMcMarch rows in y.  The comparisons of a
+// row of samples are one ballot, rows z and z + 1 are kept for the next step,
+// and four steps' rows are loaded ahead; a cell's case is eight bits of the
+// four row masks.  The field is read once from HBM (the rows shared by
+// neighbouring z come from L1: the block's warps are consecutive in z).
+constexpr int kMcSeg = 31;
+constexpr int kMcUnit = 8;
+constexpr int kMcMarch = 16;
+constexpr int kMcAhead = 4;
+// below, lanes of a segment would idle: a thread per cell in both passes
+constexpr int kMcThinRow = 16;
+
+// case of the cell at each lane from the masks of its rows (z, y), (z, y + 1),
+// (z + 1, y), (z + 1, y + 1)
+__device__ __forceinline__ unsigned mc_case_bits(unsigned A, unsigned B, unsigned C, unsigned D, int lane) {
+    const unsigned b = B >> lane, d = D >> lane;
+    return ((C >> lane) & 3u) | (((d & 1u) << 3) | ((d & 2u) << 1)) | (((A >> lane) & 3u) << 4) |
+           (((b & 1u) << 7) | ((b & 2u) << 5));
+}
+
+__global__ void __launch_bounds__(kMcThreads) k_mc_count_rows(McArgs a, int segs, unsigned int* __restrict__ counts) {
+    static_assert(kMcThreads == 256, "a case per thread");
+    __shared__ unsigned char ntri[256];
+    ntri[threadIdx.x] = g_ntri[threadIdx.x];
+    __syncthreads();
+    const unsigned FULL = 0xffffffffu;
+    const float iso = a.iso_dev ? *a.iso_dev : a.iso;
+    const int lane = threadIdx.x & 31;
+    const int cx = a.rx - 1, cy = a.ry - 1, cz = a.rz - 1;
+    const long long item = ((long long)blockIdx.x * kMcThreads + threadIdx.x) >> 5;
+    const int z = (int)(item % cz);
+    const long long r = item / cz;
+    const int seg = (int)(r % segs), x0 = seg * kMcSeg, y0 = (int)(r / segs) * kMcMarch;
+    if (y0 >= cy) return;
+    const int y1 = min(y0 + kMcMarch, cy);
+    const int last = min(kMcSeg, cx - x0);  // the segment's last sample
+    const bool in = lane <= last;
+    const unsigned valid = 0xffffffffu >> (31 - last);
+    const size_t plane = (size_t)a.rx * a.ry;
+    const float* row = a.field + (size_t)z * plane + (size_t)y0 * a.rx + x0 + lane;
+    unsigned A = __ballot_sync(FULL, in && row[0] > iso), C = __ballot_sync(FULL, in && row[plane] > iso);
+    for (int y = y0; y < y1; y += kMcAhead) {
+        float v0[kMcAhead], v1[kMcAhead];
+#pragma unroll
+        for (int u = 0; u < kMcAhead; ++u) {
+            row += a.rx;
+            const bool ok = in && y + u < y1;
+            v0[u] = ok ? row[0] : 0.f;
+            v1[u] = ok ? row[plane] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kMcAhead; ++u) {
+            if (y + u >= y1) break;
+            const unsigned B = __ballot_sync(FULL, in && v0[u] > iso), D = __ballot_sync(FULL, in && v1[u] > iso);
+            if ((A | B | C | D) && (A & B & C & D) != valid) {
+                const unsigned n = __reduce_add_sync(FULL, lane < last ? ntri[mc_case_bits(A, B, C, D, lane)] : 0u);
+                if (lane == 0 && n)
+                    atomicAdd(&counts[(seg + (long long)segs * (y + u + (long long)cy * z)) / kMcUnit], n);
+            }
+            A = B;
+            C = D;
+        }
+    }
+}
+
+// Emit: a warp per unit that has triangles (group units at a time are looked
+// at for one).  It finds the cases again by row masks and lists the triangles
+// (case, cell, number, segment) in shared memory; 32 of them at a time, a lane
+// makes one each from the six samples of its edges (L1), and the vertices
+// leave through shared memory as whole rows.  The triangles of consecutive
+// units are consecutive in the output, so what does not fill the lanes waits
+// for the next unit of the group.  Lanes are busy with triangles, not cells,
+// nothing is indexed in local memory, and stores are coalesced.  Also writes
+// the total.  A 384^3 grid with 2.05 M triangles: count 109 and emit 257 us (367
+// and 897 with a thread per cell in both passes); 256^3 at 0.3 M: 30 and 71
+// (91 and 190).  The instructions of the triangles bound it (0.65 of issue).
+constexpr int kMcEmitWarps = 4;
+constexpr int kMcGroup = 4;                       // units a warp takes at a time, at most
+constexpr int kMcPlaces = kMcGroup * kMcUnit;     // segments whose places are kept
+constexpr int kMcList = 32 + 5 * kMcSeg;          // waiting triangles, and a segment's
+
+template <bool POS>
+__global__ void __launch_bounds__(kMcEmitWarps * 32)
+    k_mc_emit(McArgs a, unsigned segs, const unsigned int* __restrict__ counts, const unsigned int* __restrict__ offs,
+              long long units, int group, long long cap, float* __restrict__ tris, float* __restrict__ cen,
+              float* __restrict__ nrm, unsigned long long* __restrict__ total) {
+    __shared__ __align__(16) signed char edges[256][16];
+    __shared__ unsigned char ntri[256];
+    __shared__ size_t corner[8];
+    // case | lane << 8 | number << 13 | segment << 16
+    __shared__ unsigned list[kMcEmitWarps][kMcList];
+    __shared__ int3 place[kMcEmitWarps][kMcPlaces];  // x0, y, z of the listed segments
+    __shared__ float out[kMcEmitWarps][32 * 9];
+    for (int i = threadIdx.x; i < 256; i += kMcEmitWarps * 32) {
+        *reinterpret_cast<int4*>(edges[i]) = *reinterpret_cast<const int4*>(g_tri[i]);
+        ntri[i] = g_ntri[i];
+    }
+    const size_t plane = (size_t)a.rx * a.ry;
+    if (threadIdx.x < 8) {
+        const int c = threadIdx.x;
+        corner[c] = ((c ^ (c >> 1)) & 1) + (size_t)((c >> 1) & 1) * a.rx + (size_t)(1 - (c >> 2)) * plane;
+    }
+    __syncthreads();
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const float iso = a.iso_dev ? *a.iso_dev : a.iso;
+    const int cx = a.rx - 1;
+    const unsigned cy = (unsigned)(a.ry - 1), cz = (unsigned)(a.rz - 1);
+    if (total && blockIdx.x == 0 && threadIdx.x == 0)
+        *total = (unsigned long long)offs[units - 1] + counts[units - 1];
+    // the listed triangles first .. first + n - 1 go to dst rows (width floats)
+    auto store = [&](float* dst, int width, int m, unsigned long long at) {
+        __syncwarp();
+        float* o = dst + at * width;
+        for (int k = lane; k < m * width; k += 32) o[k] = out[w][k];
+        __syncwarp();
+    };
+    auto emit = [&](int n, unsigned long long at) {  // the list's first n (1 to 32) triangles
+        const long long left = cap - (long long)at;  // that still fit
+        if (left <= 0) return;
+        const int m = left < n ? (int)left : n;
+        float P[3][3];
+        if (lane < m) {
+            const unsigned en = list[w][lane];
+            const int3 o = place[w][en >> 16];
+            const int x = o.x + (int)((en >> 8) & 31u), y = o.y, z = o.z;
+            const signed char* tri = &edges[en & 255u][3 * ((en >> 13) & 7u)];
+            const float* f = a.field + ((size_t)x + (size_t)a.rx * y + plane * z);
+            // the cell's coordinates on each axis
+            const float x0 = __fadd_rn(a.ox, __fmul_rn((float)x, a.h)), x1 = __fadd_rn(a.ox, __fmul_rn((float)(x + 1), a.h));
+            const float y0 = __fadd_rn(a.oy, __fmul_rn((float)y, a.h)), y1 = __fadd_rn(a.oy, __fmul_rn((float)(y + 1), a.h));
+            const int gz = z + a.zoff;
+            const float z0 = __fadd_rn(a.oz, __fmul_rn((float)gz, a.h)), z1 = __fadd_rn(a.oz, __fmul_rn((float)(gz + 1), a.h));
+            int ca[3], cb[3];
+            float va[3], vb[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const int e = tri[q];
+                ca[q] = e & 7;
+                cb[q] = e < 4 ? ((e + 1) & 3) : (e < 8 ? 4 + ((e - 3) & 3) : e - 4);
+                va[q] = f[corner[ca[q]]];
+                vb[q] = f[corner[cb[q]]];
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const float num = __fsub_rn(va[q], iso);
+                const float den = __double2float_rn(__dadd_rn((double)__fsub_rn(vb[q], va[q]), 1e-10));
+                const float ell = __fdiv_rn(num, den);
+                float p[2][3];
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int c = s ? cb[q] : ca[q];
+                    if (POS) {
+                        const float* r = a.pos + 3 * ((f - a.field) + corner[c]);
+                        p[s][0] = r[0];
+                        p[s][1] = r[1];
+                        p[s][2] = r[2];
+                    } else {
+                        p[s][0] = (c ^ (c >> 1)) & 1 ? x1 : x0;
+                        p[s][1] = c & 2 ? y1 : y0;
+                        p[s][2] = c & 4 ? z0 : z1;
+                    }
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    P[q][d] = __fsub_rn(p[0][d], __fmul_rn(ell, __fsub_rn(p[1][d], p[0][d])));
+            }
+        }
+        if (tris) {
+            if (lane < m) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) out[w][lane * 9 + q * 3 + d] = P[q][d];
+            }
+            store(tris, 9, m, at);
+        }
+        if (cen) {
+            if (lane < m) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    out[w][lane * 3 + d] = __fdiv_rn(__fadd_rn(__fadd_rn(P[0][d], P[1][d]), P[2][d]), 3.0f);
+            }
+            store(cen, 3, m, at);
+        }
+        if (nrm) {
+            if (lane < m) {
+                float u[3], v[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    u[d] = __fsub_rn(P[1][d], P[0][d]);
+                    v[d] = __fsub_rn(P[2][d], P[0][d]);
+                }
+                const float nx = __fsub_rn(__fmul_rn(u[1], v[2]), __fmul_rn(u[2], v[1]));
+                const float ny = __fsub_rn(__fmul_rn(u[2], v[0]), __fmul_rn(u[0], v[2]));
+                const float nz = __fsub_rn(__fmul_rn(u[0], v[1]), __fmul_rn(u[1], v[0]));
+                const float sc = -inv_len_eps(__fsqrt_rn(sq3_rn(nx, ny, nz)));
+                out[w][lane * 3] = __fmul_rn(nx, sc);
+                out[w][lane * 3 + 1] = __fmul_rn(ny, sc);
+                out[w][lane * 3 + 2] = __fmul_rn(nz, sc);
+            }
+            store(nrm, 3, m, at);
+        }
+    };
+    const long long warps = (long long)gridDim.x * kMcEmitWarps;
+    for (long long g = (long long)blockIdx.x * kMcEmitWarps + w; g * group < units; g += warps) {
+        const long long mine = g * group + lane;
+        const unsigned cnt = lane < group && mine < units ? counts[mine] : 0u;
+        unsigned act = __ballot_sync(FULL, cnt > 0);
+        if (!act) continue;
+        unsigned long long base = offs[g * group + __ffs(act) - 1];  // output place of the list's first triangle
+        int T = 0, ns = 0;                                           // triangles waiting, segments placed
+        while (act) {
+            const long long unit = g * group + __ffs(act) - 1;
+            act &= act - 1;
+            // lane s: the place of the unit's segment s (of a lane past the
+            // grid's segments, z = cz)
+            const unsigned seg = (unsigned)unit * kMcUnit + (lane & (kMcUnit - 1));
+            const unsigned st = seg / segs;
+            const int sx = (int)(seg - st * segs) * kMcSeg;
+            const unsigned sz = st / cy, sy = st - sz * cy;
+            if (lane < kMcUnit) place[w][ns + lane] = make_int3(sx, (int)sy, (int)sz);
+            // the cases of the unit's cells, a byte per segment
+            unsigned long long ci8 = 0;
+#pragma unroll
+            for (int s = 0; s < kMcUnit; ++s) {
+                const int x = __shfl_sync(FULL, sx, s) + lane;
+                const unsigned y = __shfl_sync(FULL, sy, s), z = __shfl_sync(FULL, sz, s);
+                bool va = false, vb = false, vc = false, vd = false;
+                if (x < a.rx && z < cz) {
+                    const float* p = a.field + (size_t)x + (size_t)a.rx * y + plane * z;
+                    va = p[0] > iso;
+                    vb = p[a.rx] > iso;
+                    vc = p[plane] > iso;
+                    vd = p[plane + a.rx] > iso;
+                }
+                const unsigned A = __ballot_sync(FULL, va), B = __ballot_sync(FULL, vb), C = __ballot_sync(FULL, vc),
+                               D = __ballot_sync(FULL, vd);
+                if (lane < kMcSeg && x < cx) ci8 |= (unsigned long long)mc_case_bits(A, B, C, D, lane) << (8 * s);
+            }
+            // (after the group's last unit, once more for what waits)
+#pragma unroll 1
+            for (int s = 0; s < kMcUnit + (act ? 0 : 1); ++s) {
+                if (s < kMcUnit) {
+                    const unsigned ci = (unsigned)(ci8 >> (8 * s)) & 255u;
+                    const int n = ntri[ci];
+                    // n is at most 5: three ballots count the triangles before
+                    const unsigned b0 = __ballot_sync(FULL, n & 1), b1 = __ballot_sync(FULL, n & 2),
+                                   b2 = __ballot_sync(FULL, n & 4);
+                    if (!(b0 | b1 | b2)) continue;
+                    const int at = T + __popc(b0 & below) + 2 * __popc(b1 & below) + 4 * __popc(b2 & below);
+                    for (int k = 0; k < n; ++k) list[w][at + k] = ci | (lane << 8) | (k << 13) | ((ns + s) << 16);
+                    T += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+                }
+                while (T >= 32 || (s == kMcUnit && T > 0)) {
+                    __syncwarp();
+                    const int m = min(T, 32);
+                    emit(m, base);
+                    base += m;
+                    T -= m;
+                    __syncwarp();
+                    // the others move up (in order: a row of lanes at a time)
+                    for (int k = 0; k < T; k += 32) {
+                        const unsigned v = k + lane < T ? list[w][k + 32 + lane] : 0u;
+                        __syncwarp();
+                        if (k + lane < T) list[w][k + lane] = v;
+                        __syncwarp();
+                    }
+                }
+            }
+            ns += kMcUnit;
+        }
+    }
+}
+
+// how a grid is cut: blocks of cells (segs 0) or units of segments
+struct McCut {
+    unsigned segs;
+    long long parts;
+};
+static McCut mc_cut(const McArgs& a, long long most_parts) {
+    const long long cx = a.rx - 1, rows = (long long)(a.ry - 1) * (a.rz - 1);
+    const long long segs = (cx + kMcSeg - 1) / kMcSeg, units = (segs * rows + kMcUnit - 1) / kMcUnit;
+    if (cx >= kMcThinRow && segs * rows < (1ll << 32) - kMcUnit && units <= most_parts)
+        return {(unsigned)segs, units};
+    return {0u, (a.ncell + kMcThreads - 1) / kMcThreads};
+}
+
+// triangles per part of the grid
+static int mc_count(const McArgs& a, const McCut& cut, unsigned int* counts, cudaStream_t s) {
+    if (cut.segs) {
+        const long long marches = (a.ry - 1 + kMcMarch - 1) / kMcMarch;
+        const long long blocks = ((long long)cut.segs * marches * (a.rz - 1) * 32 + kMcThreads - 1) / kMcThreads;
+        DWG_CHECK_CUDA(cudaMemsetAsync(counts, 0, sizeof(unsigned int) * cut.parts, s));
+        k_mc_count_rows<<<(unsigned)blocks, kMcThreads, 0, s>>>(a, (int)cut.segs, counts);
+    } else {
+        k_mc_count<<<(unsigned)cut.parts, kMcThreads, 0, s>>>(a, counts);
+    }
+    DWG_CHECK_LAUNCH();
+    return DWG_OK;
+}
+
+// the triangles at their offsets, and (total not null) their number
+static int mc_emit(const McArgs& a, const McCut& cut, const unsigned int* counts, const unsigned int* offs,
+                   long long cap, float* tris, float* centroids, float* normals, unsigned long long* total,
+                   cudaStream_t s) {
+    if (cut.segs) {
+        static int bps_of[2] = {0, 0};
+        int& bps = bps_of[a.pos != nullptr];
+        if (!bps) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, a.pos ? k_mc_emit<true> : k_mc_emit<false>,
+                                                          kMcEmitWarps * 32, 0);
+            if (bps <= 0) bps = 1;
+        }
+        // several groups per warp, so that clusters of units with triangles
+        // spread over the warps
+        const long long warps = (long long)num_sms() * bps * kMcEmitWarps;
+        const int group = (int)std::max<long long>(1, std::min<long long>(kMcGroup, cut.parts / (4 * warps)));
+        const long long blocks = std::min<long long>((long long)num_sms() * bps,
+                                                     (cut.parts + (long long)group * kMcEmitWarps - 1) /
+                                                         ((long long)group * kMcEmitWarps));
+        auto kernel = a.pos ? k_mc_emit<true> : k_mc_emit<false>;
+        kernel<<<(unsigned)blocks, kMcEmitWarps * 32, 0, s>>>(a, cut.segs, counts, offs, cut.parts, group, cap, tris,
+                                                              centroids, normals, total);
+    } else {
+        k_mc_emit_cells<<<(unsigned)cut.parts, kMcThreads, 0, s>>>(a, offs, cap, tris, centroids, normals, cut.parts,
+                                                                   counts, total);
+    }
+    DWG_CHECK_LAUNCH();
+    return DWG_OK;
+}
+
 int mc_run(const float* field, const McGrid& g, float iso, const float* iso_dev, float* tris,
            float* centroids, float* normals, long long cap, unsigned long long* num_tris_dev,
            McWorkspace& ws, cudaStream_t s) {
@@ -600,12 +941,12 @@ int mc_run(const float* field, const McGrid& g, float iso, const float* iso_dev,
     a.h = g.spacing;
     a.iso = iso;
     a.iso_dev = iso_dev;
-    long long nb = (a.ncell + kMcThreads - 1) / kMcThreads;
-    DWG_REQUIRE(nb < (1ll << 31), "marching cubes: grid too large");
+    DWG_REQUIRE((a.ncell + kMcThreads - 1) / kMcThreads < (1ll << 31), "marching cubes: grid too large");
+    const McCut cut = mc_cut(a, 1ll << 30);
+    const long long nb = cut.parts;
     DWG_TRY(ws.block_counts.reserve(nb));
     DWG_TRY(ws.block_offsets.reserve(nb));
-    k_mc_count<<<(unsigned)nb, kMcThreads, 0, s>>>(a, ws.block_counts.ptr);
-    DWG_CHECK_LAUNCH();
+    DWG_TRY(mc_count(a, cut, ws.block_counts.ptr, s));
     size_t bytes = 0;
     unsigned* cin = ws.block_counts.ptr;
     unsigned* cout = ws.block_offsets.ptr;
@@ -613,10 +954,7 @@ int mc_run(const float* field, const McGrid& g, float iso, const float* iso_dev,
     DWG_TRY(ws.scratch.reserve(bytes + 256));
     bytes = ws.scratch.n;
     DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(ws.scratch.ptr, bytes, cin, cout, (int)nb, s));
-    k_mc_total<<<1, 1, 0, s>>>(cin, cout, nb, num_tris_dev);
-    k_mc_emit<<<(unsigned)nb, kMcThreads, 0, s>>>(a, cout, cap, tris, centroids, normals);
-    DWG_CHECK_LAUNCH();
-    return DWG_OK;
+    return mc_emit(a, cut, cin, cout, cap, tris, centroids, normals, num_tris_dev, s);
 }
 
 }  // namespace dwg
@@ -725,11 +1063,12 @@ extern "C" int dwg_marching_cubes_noalloc(const float* field_dev, const int res[
     a.h = spacing;
     a.iso = iso;
     a.iso_dev = nullptr;
-    const long long nb = (ncell + kMcThreads - 1) / kMcThreads;
-    k_mc_count<<<(unsigned)nb, kMcThreads, 0, s>>>(a, counts);
+    const McCut cut = mc_cut(a, kMcNoAllocMaxBlocks);
+    const long long nb = cut.parts;
+    DWG_TRY(mc_count(a, cut, counts, s));
     k_mc_noalloc_scan<<<1, kMcScanThreads, 0, s>>>(counts, offs, nb, total);
-    k_mc_emit<<<(unsigned)nb, kMcThreads, 0, s>>>(a, offs, capacity, tris_dev, centroids_dev, normals_dev);
     DWG_CHECK_LAUNCH();
+    DWG_TRY(mc_emit(a, cut, counts, offs, capacity, tris_dev, centroids_dev, normals_dev, nullptr, s));
     unsigned long long T = 0;
     DWG_CHECK_CUDA(cudaMemcpyAsync(&T, total, sizeof(T), cudaMemcpyDeviceToHost, s));
     DWG_CHECK_CUDA(cudaStreamSynchronize(s));

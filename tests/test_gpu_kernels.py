@@ -569,3 +569,34 @@ def test_knn_near_and_far_rounds(oracle_lib, n, k):
     got = ix.query(cu(Q), k).cpu().numpy()
     bad = np.isnan(Q[:, 1])
     assert np.array_equal(got[~bad], ref[~bad]) and np.all(got[bad] == -1)
+
+
+@pytest.mark.parametrize("res", [(2, 2, 2), (16, 9, 7), (17, 5, 3), (32, 2, 40), (33, 18, 17), (64, 35, 2), (95, 33, 21)])
+@pytest.mark.parametrize("positions", [False, True])
+def test_marching_cubes_cuts(oracle_lib, dwg_lib, res, positions):
+    # grids below and above the rows' segments of 31 cells, marches of 16 rows
+    # that end early, and noise (every case, up to 5 triangles in every cell,
+    # lists that fill); also a capacity that cuts a run of 32 triangles, and
+    # the allocation-free call
+    import ctypes as C
+    rng = np.random.default_rng(sum(res))
+    res = np.array(res, np.int32)
+    f = rng.normal(size=int(np.prod(res))).astype(np.float32)
+    f[rng.random(f.size) < 0.05] = 0.0  # samples at the iso value
+    org, h = np.array([-0.3, 0.1, -0.6], np.float32), np.float32(0.0371)
+    ref = oracle_lib.marching_cubes(f, res, org, h, np.float32(0.0))
+    T = ref["T"]
+    pos = cu(oracle_lib.grid_points(res, org, h).astype(np.float32)) if positions else None
+    f_d = cu(f)
+    for cap in (T, max(T - 33, 1)):
+        out = [torch.full((T + 1, c), 7.0, device=DEV) for c in (9, 3, 3)]
+        for call in (dwg_lib.dwg_marching_cubes, dwg_lib.dwg_marching_cubes_noalloc):
+            n = C.c_longlong()
+            args = (capi.ptr(f_d), res.ctypes.data, capi.ptr(pos), org.ctypes.data, float(h), 0.0,
+                    *[capi.ptr(t) for t in out], cap)
+            args += (None, C.byref(n), None) if call is dwg_lib.dwg_marching_cubes else (C.byref(n), None)
+            assert call(*args) == (capi.DWG_OK if T <= cap else capi.DWG_ERR_OVERFLOW) and n.value == T
+            for t, name in zip(out, ("tris", "centroids", "normals")):
+                got = t.cpu().numpy()
+                assert np.array_equal(got[:cap].reshape(cap, -1), ref[name][:cap].reshape(cap, -1)), name
+                assert np.all(got[cap:] == 7.0)
