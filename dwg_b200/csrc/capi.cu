@@ -452,7 +452,8 @@ static int gwn_thread_common(dwg_octree* tree, const float* normals_dev, const f
     DWG_REQUIRE(tree && params && (out_w || out_g), "gwn: null argument");
     DWG_TRY(octree_set_point_data(tree->t, normals_dev, areas_dev, radii_dev, S(stream)));
     if (normals_dev || areas_dev) DWG_TRY(octree_update_normals(tree->t, S(stream)));
-    return gwn_eval_thread(tree->t, q, *params, fp64, out_w, out_g, S(stream));
+    if (fp64) return gwn_eval_fp64(tree->t, q, *params, (double*)out_w, (double*)out_g, S(stream));
+    return gwn_eval_grad(tree->t, q, *params, (float*)out_w, (float*)out_g, S(stream));
 }
 
 int dwg_gwn_points_grad(dwg_octree* tree, const float* normals_dev, const float* areas_dev, const float* radii_dev,

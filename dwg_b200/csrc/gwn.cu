@@ -120,6 +120,59 @@ struct AccType<3> {
     using T = CompSum;
 };
 
+// values and gradients (PREC 4): FP32 terms in IEEE arithmetic, summed in FP64
+// (100,000 points, 200,001 queries, screened: 0.59 ms, 1.24 with a thread per
+// query in the caller's order; its divisions, square root and exponential
+// bound it, which the MUFU approximations would shorten at a loss of accuracy)
+struct GradSum {
+    double w, x, y, z;
+    GradSum() = default;
+    __device__ GradSum(int v) : w(v), x(v), y(v), z(v) {}
+    __device__ GradSum(double w_, float gx, float gy, float gz) : w(w_), x(gx), y(gy), z(gz) {}
+    __device__ __forceinline__ GradSum& operator+=(const GradSum& o) {
+        w += o.w;
+        x += o.x;
+        y += o.y;
+        z += o.z;
+        return *this;
+    }
+};
+template <>
+struct AccType<4> {
+    using T = GradSum;
+};
+
+// One term v = G(rho) dot, dot = ne.(p - q), and its gradient with respect to
+// q, added to sum where take is set:
+//   screened  G = |sigma rho + 1| / (e^{sigma rho} 4 pi rho^3 + 1e-7),
+//             rho = max(|p - q|, s), grad v = -G ne + dot G'(rho) grad rho,
+//             grad rho = -(p - q) / r for r > s, 0 where s takes over;
+//   plain     G = 1 / (4 pi r^3 + 1e-8), grad v = -ne G + dot 12 pi r G^2 (p - q).
+template <bool SCREENED>
+__device__ __forceinline__ void grad_term(bool take, float dx, float dy, float dz, float nx, float ny, float nz,
+                                          float s, float sigma, GradSum& sum) {
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float dot = dx * nx + dy * ny + dz * nz;
+    const bool ok = take && (SCREENED ? r2 > 1e-20f : r2 != 0.f);  // else a term of value 0
+    const float r = sqrtf(ok ? r2 : 1.f);
+    if (SCREENED) {
+        const float rho = r > s ? r : s;
+        const float e = expf(sigma * rho);
+        const float r3 = rho * rho * rho;
+        const float den = e * (kFourPi * r3) + 1e-7f;
+        const float up = fabsf(sigma * rho + 1.f);
+        const float G = up / den;
+        const float dden = e * (sigma * kFourPi * r3 + (3.f * kFourPi) * rho * rho);
+        const float Gp = (sigma * den - up * dden) / (den * den);
+        const float k = r > s ? -dot * Gp / r : 0.f;
+        if (ok) sum += GradSum((double)(G * dot), k * dx - G * nx, k * dy - G * ny, k * dz - G * nz);
+    } else {
+        const float den = kFourPi * r * r2 + 1e-8f;
+        const float k = dot * (3.f * kFourPi) * r / (den * den);
+        if (ok) sum += GradSum((double)(dot / den), k * dx - nx / den, k * dy - ny / den, k * dz - nz / den);
+    }
+}
+
 // brick shapes of 32 grid samples (x, y, z extents) a warp evaluates together
 template <int SHAPE>
 struct Brick;
@@ -157,6 +210,7 @@ struct GwnArgs {
     const float* sigma_dev;
     int use_radii;
     const float* __restrict__ q;
+    const int* order;  // point queries in spatial order (null: as they come)
     long long nq;
     int rx, ry, rz;
     int zoff;  // global z index of local sample 0 (grid slabs)
@@ -164,6 +218,7 @@ struct GwnArgs {
     int bx, by;  // bricks per row / column
     long long ngroups;
     float* __restrict__ out;
+    float* out_g;  // gradients, 3 per query (PREC 4)
     unsigned long long* terms_total;
     int* per_query_terms;
     unsigned int* work;  // [0] counter, [1] error flags (sticky)
@@ -336,6 +391,7 @@ __device__ __forceinline__ void group_queries(const GwnArgs& a, unsigned long lo
             valid[u] = qi[u] < a.nq;
             qx[u] = qy[u] = qz[u] = 0.f;
             if (valid[u]) {
+                if (a.order) qi[u] = a.order[qi[u]];
                 qx[u] = a.q[qi[u] * 3];
                 qy[u] = a.q[qi[u] * 3 + 1];
                 qz[u] = a.q[qi[u] * 3 + 2];
@@ -369,12 +425,16 @@ __device__ __forceinline__ void leaf_terms(const GwnArgs& a, int start, int cnt,
         const float4 p = a.pa[j];
         const float4 nn = a.nr[j];
         const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
-        const float d = p.w * fmaf(dx, nn.x, fmaf(dy, nn.y, dz * nn.z));
         const float sc = a.use_radii ? nn.w : a.screen;
-        float v;
-        if (gwn_term<SCREENED, PREC>(dx, dy, dz, d, sc, sigma, sigma_l2e, v)) {
-            sum += (Acc)v;
-            ++nt;
+        if constexpr (PREC == 4) {
+            grad_term<SCREENED>(true, dx, dy, dz, p.w * nn.x, p.w * nn.y, p.w * nn.z, sc, sigma, sum);
+        } else {
+            const float d = p.w * fmaf(dx, nn.x, fmaf(dy, nn.y, dz * nn.z));
+            float v;
+            if (gwn_term<SCREENED, PREC>(dx, dy, dz, d, sc, sigma, sigma_l2e, v)) {
+                sum += (Acc)v;
+                ++nt;
+            }
         }
     }
 }
@@ -391,30 +451,59 @@ template <bool SCREENED, int PREC, typename Acc>
 __device__ __forceinline__ float node_term(const GwnArgs& a, const float4& na, const float4& nb, float dx, float dy,
                                            float dz, float d2, bool take, float sigma, float sigma_l2e, Acc& sum,
                                            int& nt) {
-    // x and y parts first: the samples of a lane share x and y
-    const float dd = node_dot(nb, dx, dy, dz);
-    bool k;
-    float v, g = 0.f;
-    if (SCREENED && PREC != 2) {
-        g = screen_weight_masked(take, d2, a.screen, sigma, sigma_l2e, k);
-        v = __fmul_rn(g, dd);  // never contracted into the sum: a kept g gives the same bits
+    if constexpr (PREC == 4) {
+        grad_term<SCREENED>(take, dx, dy, dz, nb.x, nb.y, nb.z, a.screen, sigma, sum);
+        return 0.f;
     } else {
-        v = gwn_term_masked<SCREENED, PREC>(take, d2, dd, a.screen, sigma, sigma_l2e, k);
+        // x and y parts first: the samples of a lane share x and y
+        const float dd = node_dot(nb, dx, dy, dz);
+        bool k;
+        float v, g = 0.f;
+        if (SCREENED && PREC != 2) {
+            g = screen_weight_masked(take, d2, a.screen, sigma, sigma_l2e, k);
+            v = __fmul_rn(g, dd);  // never contracted into the sum: a kept g gives the same bits
+        } else {
+            v = gwn_term_masked<SCREENED, PREC>(take, d2, dd, a.screen, sigma, sigma_l2e, k);
+        }
+        sum += (Acc)v;  // v is 0 where no term is taken
+        nt += (int)k;
+        return g;
     }
-    sum += (Acc)v;  // v is 0 where no term is taken
-    nt += (int)k;
-    return g;
 }
+
+template <typename Acc>
+__device__ __forceinline__ void put_sum(const GwnArgs& a, long long i, const Acc& sum) {
+    a.out[i] = (float)sum;
+}
+__device__ __forceinline__ void put_sum(const GwnArgs& a, long long i, const GradSum& sum) {
+    if (a.out) a.out[i] = (float)sum.w;
+    if (a.out_g) {
+        a.out_g[i * 3] = (float)sum.x;
+        a.out_g[i * 3 + 1] = (float)sum.y;
+        a.out_g[i * 3 + 2] = (float)sum.z;
+    }
+}
+
+// One of several warps that share a group: the children of the root's
+// children are dealt out in turn (the first warp also takes the terms of the
+// root's own children), and each warp's part of the sums goes to sum and nt.
+template <typename Acc>
+struct GwnPart {
+    int part = 0, parts = 1;
+    Acc sum;
+    int nt = 0;
+};
 
 // MODE 0 sums; MODE 1 counts the group's interaction-list entries (visits
 // where some lane takes a term, and multi-point leaves); MODE 2 writes them:
 // (record, term masks per query slot) in visit order.  Modes 1 and 2 do the
 // traversal only.
-template <bool GRID, bool SCREENED, int PREC, int SHAPE, int NQ, int ORDER, int MODE = 0>
+template <bool GRID, bool SCREENED, int PREC, int SHAPE, int NQ, int ORDER, int MODE = 0, bool SPLIT = false>
 __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g, int lane,
                                          int* __restrict__ stk_node, unsigned* __restrict__ stk_mask,
                                          unsigned* __restrict__ stk_meta, float4* __restrict__ crec, float sigma,
-                                         float sigma_l2e) {
+                                         float sigma_l2e, GwnPart<typename AccType<PREC>::T>* split = nullptr) {
+    static_assert(!SPLIT || (MODE == 0 && NQ == 1), "shared groups: sums of one query per lane");
     const unsigned FULL = 0xffffffffu;
     bool valid[NQ];
     long long qi[NQ];
@@ -448,7 +537,9 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
     // opened (pushed with the queries that need it) otherwise; both use the
     // same d2.  Larger leaves (every leaf when radii apply) are summed point
     // by point.
-    auto child = [&](int cidx, const float4& na, const float4& nb, const bool* act, int& sp) {
+    // (term, push: whether this warp takes the child's terms, and its subtree)
+    auto child = [&](int cidx, const float4& na, const float4& nb, const bool* act, int& sp, bool term = true,
+                     bool push = true) {
         const unsigned meta = (unsigned)__float_as_int(nb.w);
         const bool leaf = (meta & kMetaLeafBit) != 0;
         if (leaf && (!(meta & kMetaSingle) || a.use_radii)) {
@@ -458,7 +549,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
             } else if (MODE == 0) {
 #pragma unroll
                 for (int u = 0; u < NQ; ++u)
-                    if (act[u]) leaf_points(st, cnt, u);
+                    if (act[u] && term) leaf_points(st, cnt, u);
             } else {
                 unsigned m[NQ];
 #pragma unroll
@@ -489,10 +580,10 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
                 anym |= m[u];
             }
             if (anym) record(cidx, m);
-        } else if (__any_sync(FULL, any)) {
+        } else if (__any_sync(FULL, any && term)) {
 #pragma unroll
             for (int u = 0; u < NQ; ++u) {
-                if (ORDER == 0) {
+                if constexpr (ORDER == 0) {
                     node_term<SCREENED, PREC>(a, na, nb, dx[u], dy[u], dz[u], d2[u], take[u], sigma, sigma_l2e, sum[u],
                                               nt[u]);
                 } else {
@@ -518,7 +609,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
             nm[u] = __ballot_sync(FULL, act[u] && !far[u]);
             anym |= nm[u];
         }
-        if (anym) {
+        if (anym && push) {
             if (sp < kGwnStack) {
                 if (lane == 0) {
                     stk_node[sp] = cidx;
@@ -552,28 +643,28 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
             sp = 1;
         }
     }
-    while (sp > 0) {
+    // the children of stack entry i
+    auto open = [&](int i, auto&& each) {
         __syncwarp();
-        --sp;
-        const int node = stk_node[sp];
-        const unsigned pm = stk_meta[sp];
+        const int node = stk_node[i];
+        const unsigned pm = stk_meta[i];
         bool act[NQ];
 #pragma unroll
-        for (int u = 0; u < NQ; ++u) act[u] = (stk_mask[sp * NQ + u] >> lane) & 1u;
+        for (int u = 0; u < NQ; ++u) act[u] = (stk_mask[i * NQ + u] >> lane) & 1u;
         __syncwarp();
         if (node < 0 || node >= a.num_nodes) {
             if (lane == 0) atomicOr(&a.work[1], 2u);
-            continue;
+            return;
         }
         const int first = (int)(pm & kMetaIndex);
         const int nch = (int)((pm >> 28) & 7u) + 1;
         // structural guard: children come after the parent, inside the table
         if ((pm & kMetaLeafBit) || first <= node || first + nch > a.num_nodes) {
             if (lane == 0) atomicOr(&a.work[1], 2u);
-            continue;
+            return;
         }
         // the (at most 8, contiguous) children's records at once, a lane
-        // each, into shared memory; the loop top's __syncwarp ordered the
+        // each, into shared memory; the first __syncwarp above ordered the
         // previous node's reads of them before these writes
         if (lane < nch) {
             crec[lane] = a.node_a[first + lane];
@@ -582,8 +673,34 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
         __syncwarp();
         for (int j = 0; j < nch; ++j) {
             const float4 na = crec[j], nb = crec[8 + j];
-            child(first + j, na, nb, act, sp);
+            each(first + j, na, nb, act);
         }
+    };
+    int low = 0;  // entries below are done
+    if (SPLIT && sp > 0) {
+        const bool lead = split->part == 0;
+        sp = 0;
+        open(0, [&](int c, const float4& na, const float4& nb, const bool* act) { child(c, na, nb, act, sp, lead); });
+        low = sp;
+        int turn = 0;
+        for (int i = 0; i < low; ++i)
+            open(i, [&](int c, const float4& na, const float4& nb, const bool* act) {
+                const bool own = turn == split->part;
+                if (++turn == split->parts) turn = 0;
+                if (own) child(c, na, nb, act, sp);
+            });
+    } else if (SPLIT && split->part > 0) {
+        sum[0] = 0;  // a leaf root is the first warp's
+        nt[0] = 0;
+    }
+    while (sp > low) {
+        --sp;
+        open(sp, [&](int c, const float4& na, const float4& nb, const bool* act) { child(c, na, nb, act, sp); });
+    }
+    if (SPLIT) {
+        split->sum = sum[0];
+        split->nt = nt[0];
+        return 0;
     }
     if (MODE == 1) {
         if (lane == 0) a.list_count[g] = rec;
@@ -594,7 +711,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
 #pragma unroll
     for (int u = 0; u < NQ; ++u) {
         if (valid[u]) {
-            a.out[qi[u]] = (float)sum[u];
+            put_sum(a, qi[u], sum[u]);
             if (a.per_query_terms) a.per_query_terms[qi[u]] = nt[u];
         }
         total += nt[u];
@@ -630,6 +747,52 @@ __global__ void __launch_bounds__(kGwnWarps * 32, (GRID && kNqGrid >= 4) ? 2 : 3
     }
     if (a.terms_total) {
         for (int o = 16; o > 0; o >>= 1) my_terms += __shfl_down_sync(FULL, my_terms, o);
+        if (lane == 0 && my_terms) atomicAdd(a.terms_total, my_terms);
+    }
+}
+
+// Few point queries: parts (8, 4 or 2) warps share each group of 32 (see
+// GwnPart), so that a launch of a few thousand queries uses the whole GPU
+// instead of one warp per SM.  The parts are added in warp order.
+template <bool SCREENED, int PREC>
+__global__ void __launch_bounds__(kGwnWarps * 32, 3) k_gwn_split(GwnArgs a, int parts) {
+    using Acc = typename AccType<PREC>::T;
+    __shared__ int stk_node[kGwnWarps][kGwnStack];
+    __shared__ unsigned stk_mask[kGwnWarps][kGwnStack];
+    __shared__ unsigned stk_meta[kGwnWarps][kGwnStack];
+    __shared__ float4 crec[kGwnWarps][16];
+    __shared__ Acc sums[kGwnWarps][32];
+    __shared__ int terms[kGwnWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const float sigma = a.sigma_dev ? *a.sigma_dev : a.sigma;
+    const unsigned long long g = (unsigned long long)blockIdx.x * (kGwnWarps / parts) + w / parts;
+    GwnPart<Acc> part;
+    part.part = w % parts;
+    part.parts = parts;
+    if ((long long)g < a.ngroups)
+        gwn_group<false, SCREENED, PREC, 0, 1, 0, 0, true>(a, g, lane, stk_node[w], stk_mask[w], stk_meta[w], crec[w],
+                                                           sigma, sigma * 1.4426950408889634f, &part);
+    sums[w][lane] = part.sum;
+    terms[w][lane] = part.nt;
+    __syncthreads();
+    if (w % parts > 0) return;
+    Acc sum = sums[w][lane];
+    int nt = terms[w][lane];
+    for (int i = 1; i < parts; ++i) {
+        sum += sums[w + i][lane];
+        nt += terms[w + i][lane];
+    }
+    const long long j = (long long)g * 32 + lane;
+    if (j < a.nq) {
+        const long long qi = a.order ? a.order[j] : j;
+        put_sum(a, qi, sum);
+        if (a.per_query_terms) a.per_query_terms[qi] = nt;
+    } else {
+        nt = 0;
+    }
+    if (a.terms_total) {
+        unsigned long long my_terms = (unsigned long long)nt;
+        for (int o = 16; o > 0; o >>= 1) my_terms += __shfl_down_sync(0xffffffffu, my_terms, o);
         if (lane == 0 && my_terms) atomicAdd(a.terms_total, my_terms);
     }
 }
@@ -1148,6 +1311,25 @@ static int blocks_for(K kernel) {
 
 template <bool GRID, bool SCREENED, int PREC, int SHAPE, int ORDER>
 static int launch(const GwnArgs& a, cudaStream_t s) {
+    if constexpr (!GRID && ORDER == 0) {
+        // As many warps per group as keep the launch to one wave: a group's
+        // walk is a chain of dependent loads, 8 warps take about a quarter of
+        // its time (each opens the root and its children), and a second wave
+        // takes as long as the first.  14,000 queries, 20,000 points: 101 us
+        // with 8 warps, 182 us with 1; 28,000: 112 us with 4, 168 with 1.
+        if (a.order) {
+            static int bps = 0;
+            if (!bps) bps = blocks_for(k_gwn_split<SCREENED, PREC>);
+            const long long wave = (long long)num_sms() * bps * kGwnWarps;
+            const int parts = a.ngroups * 8 <= wave ? 8 : a.ngroups * 4 <= wave ? 4 : a.ngroups * 2 <= wave ? 2 : 1;
+            if (parts > 1) {
+                const long long blocks = (a.ngroups * parts + kGwnWarps - 1) / kGwnWarps;
+                k_gwn_split<SCREENED, PREC><<<(unsigned)blocks, kGwnWarps * 32, 0, s>>>(a, parts);
+                DWG_CHECK_LAUNCH();
+                return DWG_OK;
+            }
+        }
+    }
     static int blocks_per_sm = 0;
     if (!blocks_per_sm) blocks_per_sm = blocks_for(k_gwn<GRID, SCREENED, PREC, SHAPE, ORDER>);
     long long want = (a.ngroups + kGwnWarps - 1) / kGwnWarps;
@@ -1225,6 +1407,7 @@ static int make_args(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p
     a.screen = p.screen;
     a.use_radii = p.use_radii;
     a.out = out;
+    a.out_g = nullptr;
     a.terms_total = terms_total;
     a.per_query_terms = per_query_terms;
     DWG_TRY(t.work.reserve(2));
@@ -1233,9 +1416,11 @@ static int make_args(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p
     a.num_points = t.n;
     // the counter restarts with every launch; the error word is sticky
     DWG_CHECK_CUDA(cudaMemsetAsync(t.work.ptr, 0, sizeof(unsigned int), s));
+    a.order = nullptr;
     if (q.q) {
         a.q = q.q;
         a.nq = q.nq;
+        if (!q.coherent && q.nq > 0) DWG_TRY(query_order(t.qorder, q.q, q.nq, t.root, s, &a.order));
         a.rx = a.ry = a.rz = 0;
         a.zoff = 0;
         a.ox = a.oy = a.oz = a.h = 0.f;
@@ -1273,6 +1458,23 @@ int gwn_eval(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, float*
     DWG_TRY(make_args(t, q, p, out, terms_total, per_query_terms, s, sigma_dev, a, &empty));
     if (empty) return DWG_OK;
     return q.q ? dispatch<false>(a, p, s) : dispatch<true>(a, p, s);
+}
+
+int gwn_eval_grad(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, float* out_w, float* out_g,
+                  cudaStream_t s) {
+    DWG_REQUIRE(out_w || out_g, "gwn: no output");
+    DWG_REQUIRE(p.order == 0, "gwn: gradients and FP64 sums take the order-0 far field");
+    DWG_REQUIRE(p.beta >= 0.f, "gwn: beta must be >= 0");
+    dwg_gwn_params pp = p;
+    pp.tile = 0;  // tile and precision do not apply
+    GwnArgs a;
+    bool empty = false;
+    DWG_TRY(make_args(t, q, pp, out_w ? out_w : out_g, nullptr, nullptr, s, nullptr, a, &empty));
+    if (empty) return DWG_OK;
+    a.out = out_w;
+    a.out_g = out_g;
+    if (q.q) return p.screened ? launch<false, true, 4, 0, 0>(a, s) : launch<false, false, 4, 0, 0>(a, s);
+    return p.screened ? launch<true, true, 4, 0, 0>(a, s) : launch<true, false, 4, 0, 0>(a, s);
 }
 
 // ------------------------------------------------------ interaction lists --
@@ -1417,6 +1619,7 @@ int gwn_eval_listed(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p,
                     unsigned long long* terms_total, cudaStream_t s, const float* sigma_dev, size_t max_bytes,
                     int wslots) {
     DWG_REQUIRE(p.screened && p.order == 0, "gwn lists: screened sums only");
+    DWG_REQUIRE(!q.q || q.coherent, "gwn lists: point queries in their own order only");
     GwnArgs a;
     bool empty = false;
     DWG_TRY(make_args(t, q, p, out, terms_total, nullptr, s, sigma_dev, a, &empty));
@@ -1463,6 +1666,7 @@ static void fill_args(GwnArgs& a, const Octree& t, const GwnBatchItem& it, const
     a.screen = p.screen;
     a.use_radii = p.use_radii;
     a.q = nullptr;
+    a.order = nullptr;
     a.rx = it.res[0];
     a.ry = it.res[1];
     a.rz = it.res[2];
@@ -1478,6 +1682,7 @@ static void fill_args(GwnArgs& a, const Octree& t, const GwnBatchItem& it, const
     a.by = (a.ry + ey - 1) / ey;
     a.ngroups = (long long)a.bx * a.by * ((a.rz + kNqGrid * ez - 1) / (kNqGrid * ez));
     a.out = it.out;
+    a.out_g = nullptr;
     a.terms_total = it.terms_total;
     a.per_query_terms = nullptr;
     a.work = t.work.ptr;  // error word at [1]

@@ -9,6 +9,7 @@ struct GwnQuery {
     // point queries (packed xyz) ...
     const float* q = nullptr;
     long long nq = 0;
+    bool coherent = false;  // consecutive points lie near each other (else they are taken in spatial order)
     // ... or a regular grid (q == nullptr)
     int res[3] = {0, 0, 0};
     float origin[3] = {0, 0, 0};
@@ -94,12 +95,14 @@ int gwn_eval_listed(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p,
                     unsigned long long* terms_total, cudaStream_t s, const float* sigma_dev, size_t max_bytes,
                     int wslots = 0);
 
-// Values and/or gradients (out_g: 3 per query) of the sums, one thread per
-// query with the decisions of gwn_eval; fp64: terms and sums in double from
-// the FP64 moments (outputs double), else FP32 terms summed in double
-// (outputs float).  Order-0 far field only.
-int gwn_eval_thread(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, bool fp64, void* out_w,
-                    void* out_g, cudaStream_t s);
+// Values and/or gradients (out_g: 3 per query) of the sums with the decisions
+// of gwn_eval: FP32 terms in IEEE arithmetic, summed in double.  Order-0 far
+// field only.
+int gwn_eval_grad(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, float* out_w, float* out_g,
+                  cudaStream_t s);
+// The same in FP64, terms and sums from the FP64 moments, one thread per query.
+int gwn_eval_fp64(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, double* out_w, double* out_g,
+                  cudaStream_t s);
 
 // Frees every weight slot of L (the list itself stays): the kept weights
 // depend on the points' screening radii when use_radii is set, so new radii

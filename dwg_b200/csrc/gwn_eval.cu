@@ -1,27 +1,17 @@
-// gwn_eval.cu -- values and gradients of the winding-number sums, one thread
-// per query, with the Barnes-Hut decisions of the warp kernels (gwn.cu).
-//
-// The DWG loop needs values only, and gwn.cu sums those with one warp per 32
-// coherent queries.  This file serves the two other uses of the same sums:
-//
-//  * the analytic gradient grad_q w (the reference has none): for a term
-//    v = G(rho) dot with dot = ne.(p - q) (ne = A n of a point, sum A n of a
-//    far node),
-//        screened  G = |sigma rho + 1| / (e^{sigma rho} 4 pi rho^3 + 1e-7),
-//                  rho = max(|p - q|, s),
-//                  grad v = -G ne + dot G'(rho) grad rho,
-//                  grad rho = -(p - q) / r for r > s, 0 where s takes over;
-//        plain     G = 1 / (4 pi r^3 + 1e-8),
-//                  grad v = -ne G + dot 12 pi r G^2 (p - q);
-//    the far field is the order-0 dipole, whose gradient this is;
-//  * FP64 sums: terms and sums in double from the FP64 moments (cm_d, ec_d)
-//    and the points' float data, the yardstick a caller checks the FP32 sums
-//    against on the GPU (the CPU oracle does the same on the host).
+// gwn_eval.cu -- the winding-number sums and their gradients in FP64, one
+// thread per query, with the Barnes-Hut decisions of the warp kernels
+// (gwn.cu, which also has the FP32-term gradients): the yardstick a caller
+// checks the FP32 sums against on the GPU, as the CPU oracle does on the
+// host.  Terms and sums are in double, from the FP64 moments (cm_d, ec_d) and
+// the points' float data; the terms' formulas are in gwn.cu (grad_term).
 //
 // Decisions: a child record is far when sq3_rn(CM_f - q) > its open
 // threshold (exactly the warp kernels' test, so the same terms are taken);
 // leaves are always summed point by point.  The traversal walks the level-
-// order records with a per-level (first child, count, next) stack.
+// order records with a per-level (first child, count, next) stack; point
+// queries are taken in spatial order.
+#include <algorithm>
+
 #include "gwn.cuh"
 
 namespace dwg {
@@ -39,71 +29,72 @@ struct ThreadArgs {
     float sigma, screen;
     int use_radii;
     const float* __restrict__ q;
+    const int* order;  // point queries in spatial order (null: as they come)
     long long nq;
     int rx, ry, rz, zoff;
     float ox, oy, oz, h;
     int num_nodes, num_points;
-    void* out_w;
-    void* out_g;
+    double* out_w;
+    double* out_g;
     unsigned int* err;
 };
 
-// One term and its gradient, terms in T (float: IEEE sqrt and division and
-// CUDA's expf; or double), accumulated in double.
-template <typename T, bool SCREENED, bool GRAD>
-__device__ __forceinline__ void add_term(T dx, T dy, T dz, T nx, T ny, T nz, T s, T sigma, double& w, double* g) {
-    const T r2 = dx * dx + dy * dy + dz * dz;
-    const T dot = dx * nx + dy * ny + dz * nz;
+// One term and its gradient.
+template <bool SCREENED, bool GRAD>
+__device__ __forceinline__ void add_term(double dx, double dy, double dz, double nx, double ny, double nz, double s,
+                                         double sigma, double& w, double* g) {
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double dot = dx * nx + dy * ny + dz * nz;
     if (SCREENED) {
-        if (!(r2 > (T)1e-20)) return;  // |p - q| <= 1e-10 is skipped
-        const T r = sqrt(r2);
-        const T rho = r > s ? r : s;
-        const T e = exp(sigma * rho);
-        const T r3 = rho * rho * rho;
-        const T den = e * ((T)kFourPiD * r3) + (T)1e-7;
-        const T up = fabs(sigma * rho + (T)1);
-        const T G = up / den;
-        w += (double)(G * dot);
+        if (!(r2 > 1e-20)) return;  // |p - q| <= 1e-10 is skipped
+        const double r = sqrt(r2);
+        const double rho = r > s ? r : s;
+        const double e = exp(sigma * rho);
+        const double r3 = rho * rho * rho;
+        const double den = e * (kFourPiD * r3) + 1e-7;
+        const double up = fabs(sigma * rho + 1.0);
+        const double G = up / den;
+        w += G * dot;
         if (GRAD) {
-            const T dden = e * (sigma * (T)kFourPiD * r3 + (T)(3.0 * kFourPiD) * rho * rho);
-            const T Gp = (sigma * den - up * dden) / (den * den);
-            const T k = r > s ? -dot * Gp / r : (T)0;
-            g[0] += (double)(k * dx - G * nx);
-            g[1] += (double)(k * dy - G * ny);
-            g[2] += (double)(k * dz - G * nz);
+            const double dden = e * (sigma * kFourPiD * r3 + 3.0 * kFourPiD * rho * rho);
+            const double Gp = (sigma * den - up * dden) / (den * den);
+            const double k = r > s ? -dot * Gp / r : 0.0;
+            g[0] += k * dx - G * nx;
+            g[1] += k * dy - G * ny;
+            g[2] += k * dz - G * nz;
         }
     } else {
-        if (r2 == (T)0) return;  // a zero distance is a term of value 0
-        const T r = sqrt(r2);
-        const T den = (T)kFourPiD * r * r2 + (T)1e-8;
-        w += (double)(dot / den);
+        if (r2 == 0.0) return;  // a zero distance is a term of value 0
+        const double r = sqrt(r2);
+        const double den = kFourPiD * r * r2 + 1e-8;
+        w += dot / den;
         if (GRAD) {
-            const T k = dot * (T)(3.0 * kFourPiD) * r / (den * den);
-            g[0] += (double)(k * dx - nx / den);
-            g[1] += (double)(k * dy - ny / den);
-            g[2] += (double)(k * dz - nz / den);
+            const double k = dot * 3.0 * kFourPiD * r / (den * den);
+            g[0] += k * dx - nx / den;
+            g[1] += k * dy - ny / den;
+            g[2] += k * dz - nz / den;
         }
     }
 }
 
-template <typename T, bool SCREENED, bool GRAD>
+template <bool SCREENED, bool GRAD>
 __device__ __forceinline__ void leaf_points_thread(const ThreadArgs& a, int st, int cnt, float qx, float qy, float qz,
                                                    double& w, double* g) {
-    const T sig = (T)a.sigma;
+    const double sig = (double)a.sigma;
     for (int j = st; j < st + cnt; ++j) {
         const float4 p = a.pa[j];
         const float4 n = a.nr[j];
-        const T s = (T)(a.use_radii ? n.w : a.screen);
-        add_term<T, SCREENED, GRAD>((T)p.x - (T)qx, (T)p.y - (T)qy, (T)p.z - (T)qz, (T)p.w * (T)n.x,
-                                    (T)p.w * (T)n.y, (T)p.w * (T)n.z, s, sig, w, g);
+        const double s = (double)(a.use_radii ? n.w : a.screen);
+        add_term<SCREENED, GRAD>((double)p.x - qx, (double)p.y - qy, (double)p.z - qz, (double)p.w * n.x,
+                                 (double)p.w * n.y, (double)p.w * n.z, s, sig, w, g);
     }
 }
 
-template <typename T, bool SCREENED, bool GRAD>
+template <bool SCREENED, bool GRAD>
 __global__ void __launch_bounds__(128) k_gwn_thread(ThreadArgs a) {
-    using TO = T;  // output type
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.nq; i += stride) {
+    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < a.nq; j += stride) {
+        const long long i = a.order ? a.order[j] : j;
         float qx, qy, qz;
         if (a.q) {
             qx = a.q[i * 3];
@@ -124,7 +115,7 @@ __global__ void __launch_bounds__(128) k_gwn_thread(ThreadArgs a) {
             if (rm & kMetaLeafBit) {
                 const int st = (int)(rm & kMetaIndex), cnt = __float_as_int(a.node_a[0].w);
                 if (cnt >= 0 && st + cnt <= a.num_points)
-                    leaf_points_thread<T, SCREENED, GRAD>(a, st, cnt, qx, qy, qz, w, g);
+                    leaf_points_thread<SCREENED, GRAD>(a, st, cnt, qx, qy, qz, w, g);
                 else
                     atomicOr(a.err, 4u);
             } else {
@@ -154,22 +145,16 @@ __global__ void __launch_bounds__(128) k_gwn_thread(ThreadArgs a) {
                     atomicOr(a.err, 4u);
                     continue;
                 }
-                leaf_points_thread<T, SCREENED, GRAD>(a, st, cnt, qx, qy, qz, w, g);
+                leaf_points_thread<SCREENED, GRAD>(a, st, cnt, qx, qy, qz, w, g);
                 continue;
             }
             const float dxf = __fsub_rn(na.x, qx), dyf = __fsub_rn(na.y, qy), dzf = __fsub_rn(na.z, qz);
             if (sq3_rn(dxf, dyf, dzf) > na.w) {  // far: the node's dipole term
-                if (sizeof(T) == 8) {
-                    const int v = a.level_nodes[c];
-                    const double* cm = a.cm_d + (size_t)v * 3;
-                    const double* ec = a.ec_d + (size_t)v * 3;
-                    add_term<T, SCREENED, GRAD>((T)(cm[0] - (double)qx), (T)(cm[1] - (double)qy),
-                                                (T)(cm[2] - (double)qz), (T)ec[0], (T)ec[1], (T)ec[2],
-                                                (T)a.screen, (T)a.sigma, w, g);
-                } else {
-                    add_term<T, SCREENED, GRAD>((T)dxf, (T)dyf, (T)dzf, (T)nb.x, (T)nb.y, (T)nb.z, (T)a.screen,
-                                                (T)a.sigma, w, g);
-                }
+                const int v = a.level_nodes[c];
+                const double* cm = a.cm_d + (size_t)v * 3;
+                const double* ec = a.ec_d + (size_t)v * 3;
+                add_term<SCREENED, GRAD>(cm[0] - (double)qx, cm[1] - (double)qy, cm[2] - (double)qz, ec[0], ec[1],
+                                         ec[2], a.screen, a.sigma, w, g);
                 continue;
             }
             // opened: its children become the next level
@@ -183,26 +168,25 @@ __global__ void __launch_bounds__(128) k_gwn_thread(ThreadArgs a) {
             next[lev] = 0;
             ++lev;
         }
-        if (a.out_w) static_cast<TO*>(a.out_w)[i] = (TO)w;
+        if (a.out_w) a.out_w[i] = w;
         if (GRAD && a.out_g) {
-            TO* og = static_cast<TO*>(a.out_g) + i * 3;
-            og[0] = (TO)g[0];
-            og[1] = (TO)g[1];
-            og[2] = (TO)g[2];
+            a.out_g[i * 3] = g[0];
+            a.out_g[i * 3 + 1] = g[1];
+            a.out_g[i * 3 + 2] = g[2];
         }
     }
 }
 
-template <typename T, bool SCREENED, bool GRAD>
+template <bool SCREENED, bool GRAD>
 static int launch_thread(const ThreadArgs& a, cudaStream_t s) {
     const long long blocks = std::min<long long>((a.nq + 127) / 128, (long long)num_sms() * 16);
-    k_gwn_thread<T, SCREENED, GRAD><<<(unsigned)(blocks > 0 ? blocks : 1), 128, 0, s>>>(a);
+    k_gwn_thread<SCREENED, GRAD><<<(unsigned)(blocks > 0 ? blocks : 1), 128, 0, s>>>(a);
     DWG_CHECK_LAUNCH();
     return DWG_OK;
 }
 
-int gwn_eval_thread(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, bool fp64, void* out_w,
-                    void* out_g, cudaStream_t s) {
+int gwn_eval_fp64(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, double* out_w, double* out_g,
+                  cudaStream_t s) {
     DWG_REQUIRE(t.M > 0, "gwn: octree is empty");
     DWG_REQUIRE(out_w || out_g, "gwn: no output");
     DWG_REQUIRE(p.order == 0, "gwn: gradients and FP64 sums take the order-0 far field");
@@ -225,9 +209,11 @@ int gwn_eval_thread(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p,
     a.out_w = out_w;
     a.out_g = out_g;
     a.err = t.work.ptr + 1;
+    a.order = nullptr;
     if (q.q) {
         a.q = q.q;
         a.nq = q.nq;
+        if (!q.coherent && q.nq > 0) DWG_TRY(query_order(t.qorder, q.q, q.nq, t.root, s, &a.order));
         a.rx = a.ry = a.rz = a.zoff = 0;
         a.ox = a.oy = a.oz = a.h = 0.f;
     } else {
@@ -245,12 +231,8 @@ int gwn_eval_thread(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p,
     }
     if (a.nq == 0) return DWG_OK;
     const bool grad = out_g != nullptr;
-    if (fp64) {
-        if (p.screened) return grad ? launch_thread<double, true, true>(a, s) : launch_thread<double, true, false>(a, s);
-        return grad ? launch_thread<double, false, true>(a, s) : launch_thread<double, false, false>(a, s);
-    }
-    if (p.screened) return grad ? launch_thread<float, true, true>(a, s) : launch_thread<float, true, false>(a, s);
-    return grad ? launch_thread<float, false, true>(a, s) : launch_thread<float, false, false>(a, s);
+    if (p.screened) return grad ? launch_thread<true, true>(a, s) : launch_thread<true, false>(a, s);
+    return grad ? launch_thread<false, true>(a, s) : launch_thread<false, false>(a, s);
 }
 
 }  // namespace dwg

@@ -27,6 +27,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "order.cuh"
 
 namespace dwg {
 
@@ -63,6 +64,7 @@ struct Octree {
     DevBuf<int> level_nodes, lvl_of, node_meta;
     int level_off[kMaxDepth + 2] = {0};
     DevBuf<unsigned char> scratch;  // CUB temporary storage
+    mutable QueryOrder qorder;          // spatial order of point queries
     mutable DevBuf<unsigned int> work;  // [0] work counter of the persistent GWN kernel, [1] error flag
 };
 

@@ -557,6 +557,7 @@ int Pipeline::iterate_pre() {
     GwnQuery ql;
     ql.q = leaf_pos.ptr;
     ql.nq = L;
+    ql.coherent = true;
     if (prm.grid_lists)
         DWG_TRY(gwn_eval_listed(t2, ql, gp, llist, wleaf.ptr, terms_cur.ptr, s, cur_sigma.ptr, glist_budget,
                                 weight_slots()));
@@ -763,6 +764,7 @@ int Pipeline::finalize() {
     GwnQuery ql;
     ql.q = qpts;
     ql.nq = nqp;
+    ql.coherent = true;
     DWG_TRY(gwn_eval(*tree, ql, gp, wfin.ptr, nullptr, nullptr, s));
     long long ng = (long long)fres[0] * fres[1] * fres[2];
     DWG_REQUIRE(world <= fres[2] - 1, "pipeline: %d ranks for %d final grid cells in z", world, fres[2] - 1);

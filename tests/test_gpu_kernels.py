@@ -600,3 +600,34 @@ def test_marching_cubes_cuts(oracle_lib, dwg_lib, res, positions):
                 got = t.cpu().numpy()
                 assert np.array_equal(got[:cap].reshape(cap, -1), ref[name][:cap].reshape(cap, -1)), name
                 assert np.all(got[cap:] == 7.0)
+
+
+@pytest.mark.parametrize("nq", [1, 31, 33, 3000, 15000, 30000, 70000])
+def test_point_queries_in_any_order(nq):
+    # the spatial order of a caller's queries and the number of warps that
+    # share a group of 32 (8 for few queries, then 4, 2, 1): the same values
+    # whatever order they come in, close to the FP64 sums, gradients too
+    P, N = cloud(6000, seed=3)
+    A = np.full(len(P), 2e-6, np.float32)
+    tree = turbo.TurboLibiGWN(cu(P), max_depth=9, areas=cu(A))
+    tree.UpdateMassNormals(cu(N), cu(A))
+    rng = np.random.default_rng(nq)
+    Q = P[rng.integers(0, len(P), nq)] + rng.normal(0, 0.05, (nq, 3))
+    Q[::5] = rng.uniform(-2, 2, (len(Q[::5]), 3))  # outside the cube too
+    Q = Q.astype(np.float32)
+    perm = rng.permutation(nq)
+    for kw in (dict(screened=True, sigma=10.0), dict(screened=False, sigma=0.0)):
+        def values(q, precision):
+            f = tree.TurboLibiScreenedGWNLaunch if kw["screened"] else tree.TurboLibiGWNLaunch
+            return f(cu(q), precision=precision).cpu().numpy()
+        w64, g64 = (t.cpu().numpy() for t in tree.value_and_gradient(cu(Q), fp64=True, **kw))
+        for precision in (0, 1, 2, 3):
+            w = values(Q, precision)
+            assert np.array_equal(values(Q[perm], precision), w[perm])
+            assert np.abs(w - w64).max() < 2e-5 * np.abs(w64).max()
+        w, g = (t.cpu().numpy() for t in tree.value_and_gradient(cu(Q), **kw))
+        w2, g2 = (t.cpu().numpy() for t in tree.value_and_gradient(cu(Q[perm]), **kw))
+        assert np.array_equal(w2, w[perm]) and np.array_equal(g2, g[perm])
+        assert np.abs(w - w64).max() < 2e-5 * np.abs(w64).max()
+        assert np.abs(g - g64).max() < 1e-4 * np.abs(g64).max()
+    assert tree.status() == 0
