@@ -485,8 +485,9 @@ __device__ __forceinline__ void put_sum(const GwnArgs& a, long long i, const Gra
 }
 
 // One of several warps that share a group: the children of the root's
-// children are dealt out in turn (the first warp also takes the terms of the
-// root's own children), and each warp's part of the sums goes to sum and nt.
+// children are dealt out by their number in the tree (the first warp also
+// takes the terms of the root's own children), so that a query's sum does not
+// depend on the others of its group; each warp's part goes to sum and nt.
 template <typename Acc>
 struct GwnPart {
     int part = 0, parts = 1;
@@ -682,12 +683,9 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
         sp = 0;
         open(0, [&](int c, const float4& na, const float4& nb, const bool* act) { child(c, na, nb, act, sp, lead); });
         low = sp;
-        int turn = 0;
         for (int i = 0; i < low; ++i)
             open(i, [&](int c, const float4& na, const float4& nb, const bool* act) {
-                const bool own = turn == split->part;
-                if (++turn == split->parts) turn = 0;
-                if (own) child(c, na, nb, act, sp);
+                if (c % split->parts == split->part) child(c, na, nb, act, sp);
             });
     } else if (SPLIT && split->part > 0) {
         sum[0] = 0;  // a leaf root is the first warp's
