@@ -617,8 +617,8 @@ int dwg_diffuse_normals(const int* knn_dev, const float* tri_normals_dev, long l
         DevBuf<long long> acc;
         DWG_TRY(acc.reserve((size_t)num_points * 3));
         DWG_CHECK_CUDA(cudaMemsetAsync(acc.ptr, 0, sizeof(long long) * 3 * num_points, S(stream)));
-        DWG_TRY(diffuse_normals(knn_dev, tri_normals_dev, num_tris, nullptr, k, num_points, normals_dev, acc.ptr,
-                                is_zero_dev, zero_count_dev, S(stream)));
+        DWG_TRY(diffuse_normals(knn_dev, tri_normals_dev, num_tris, nullptr, k, num_points, nullptr, normals_dev,
+                                acc.ptr, is_zero_dev, zero_count_dev, S(stream)));
         DWG_CHECK_CUDA(cudaStreamSynchronize(S(stream)));
         return DWG_OK;
     })

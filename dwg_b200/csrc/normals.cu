@@ -9,6 +9,8 @@
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
+#include <algorithm>
+
 #include "normals.cuh"
 #include "octree.cuh"
 
@@ -41,24 +43,89 @@ int gauss_map(const float* P, int n, float* N, cudaStream_t s) {
     return DWG_OK;
 }
 
-// UpdateNormals (src/TurboDWG.cu:179-204), fixed point
-__global__ void k_scatter(const int* __restrict__ knn, const float* __restrict__ tn, long long T,
-                          const unsigned long long* __restrict__ Tdev, int k, int L,
-                          unsigned long long* __restrict__ acc) {
+// UpdateNormals (src/TurboDWG.cu:179-204), fixed point.  A block takes
+// up to kScatterTris triangles that lie together (order: the spatial order their
+// neighbours were found in; null: as they come), whose k neighbours are a few
+// hundred points: their sums are collected in a shared table and leave as one
+// atomic per point, component and block instead of one per triangle.  The
+// table is keyed by point (open addressing); a sum is kept in two 32-bit
+// words, its low 20 bits and the rest, which hold kScatterAdds normals of
+// length 1 even if every neighbour is the same point (longer normals, and
+// points that find no place in kScatterProbes steps, go to global memory at
+// once).  240,000 triangles onto 10,000 points,
+// k = 15: 31 us (93 with an atomic per triangle, neighbour and component);
+// 300,000 onto 830,000: 50 (95).
+constexpr int kScatterTris = 256;
+constexpr int kScatterAdds = 2047;
+constexpr int kScatterSlots = 1024;
+constexpr int kScatterProbes = 8;
+__global__ void __launch_bounds__(256) k_scatter(const int* __restrict__ knn, const float* __restrict__ tn, long long T,
+                                                 const unsigned long long* __restrict__ Tdev, int k, int L,
+                                                 const int* __restrict__ order, unsigned long long* __restrict__ acc) {
+    __shared__ int key[kScatterSlots];
+    __shared__ int low[3][kScatterSlots], high[3][kScatterSlots];
+    __shared__ long long fix[kScatterTris][3];
+    __shared__ int tri[kScatterTris];
     long long nt = T;
     if (Tdev && (long long)*Tdev < nt) nt = (long long)*Tdev;
-    long long total = nt * k;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        long long t = e / k;
-        int i = knn[e];
-        if (i < 0 || i >= L) continue;
-        for (int d = 0; d < 3; ++d) {
-            long long f = __double2ll_rn((double)tn[t * 3 + d] * kFix);
-            atomicAdd(&acc[(size_t)i * 3 + d], (unsigned long long)f);
+    const int each = min(kScatterTris, max(1, kScatterAdds / k));
+    for (long long b = (long long)blockIdx.x * each; b < nt; b += (long long)gridDim.x * each) {
+        const int m = (int)(nt - b < each ? nt - b : each);
+        for (int s = threadIdx.x; s < kScatterSlots; s += blockDim.x) {
+            key[s] = -1;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) low[d][s] = high[d][s] = 0;
         }
+        if (threadIdx.x < m) {
+            const long long t = order ? order[b + threadIdx.x] : b + threadIdx.x;
+            tri[threadIdx.x] = (int)(t - (order ? 0 : b));
+#pragma unroll
+            for (int d = 0; d < 3; ++d) fix[threadIdx.x][d] = __double2ll_rn((double)tn[t * 3 + d] * kFix);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < m * k; e += blockDim.x) {
+            const int j = e / k;
+            const long long t = tri[j] + (order ? 0 : b);
+            const int i = knn[t * k + (e - j * k)];
+            if (i < 0 || i >= L) continue;
+            const long long f[3] = {fix[j][0], fix[j][1], fix[j][2]};
+            int slot = -1;
+            const long long one = 1ll << 40;
+            if (k <= kScatterAdds && f[0] <= one && f[0] >= -one && f[1] <= one && f[1] >= -one && f[2] <= one && f[2] >= -one) {
+                unsigned s = (unsigned)i * 2654435761u >> 22;  // multiplicative hash, 10 bits
+                for (int p = 0; p < kScatterProbes; ++p) {
+                    const int was = atomicCAS(&key[s], -1, i);
+                    if (was == -1 || was == i) {
+                        slot = (int)s;
+                        break;
+                    }
+                    s = (s + 1) & (kScatterSlots - 1);
+                }
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (slot >= 0) {
+                    atomicAdd(&low[d][slot], (int)(f[d] & 0xfffff));
+                    atomicAdd(&high[d][slot], (int)(f[d] >> 20));
+                } else {
+                    atomicAdd(&acc[(size_t)i * 3 + d], (unsigned long long)f[d]);
+                }
+            }
+        }
+        __syncthreads();
+        for (int s = threadIdx.x; s < kScatterSlots; s += blockDim.x) {
+            const int i = key[s];
+            if (i < 0) continue;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const long long f = ((long long)high[d][s] << 20) + low[d][s];
+                if (f) atomicAdd(&acc[(size_t)i * 3 + d], (unsigned long long)f);
+            }
+        }
+        __syncthreads();
     }
 }
+static_assert(kScatterSlots == 1 << 10, "10 bits of hash");
 
 // NormalizeNormals (src/TurboDWG.cu:238-266); also clears the accumulator
 __global__ void k_finalize(long long* __restrict__ acc, int L, float* __restrict__ N,
@@ -84,13 +151,14 @@ __global__ void k_finalize(long long* __restrict__ acc, int L, float* __restrict
 }
 
 int diffuse_scatter(const int* knn, const float* tn, long long T, const unsigned long long* Tdev, int k, int L,
-                    long long* acc, cudaStream_t s) {
+                    const int* order, long long* acc, cudaStream_t s) {
     DWG_REQUIRE(knn && tn && acc && L >= 1 && k >= 1, "diffuse_normals: bad arguments");
     if (T > 0) {
-        long long blocks = (T * k + 255) / 256;
-        long long cap = (long long)num_sms() * 16;
+        const int each = std::min(kScatterTris, std::max(1, kScatterAdds / k));
+        long long blocks = (T + each - 1) / each;
+        const long long cap = (long long)num_sms() * 6;
         if (blocks > cap) blocks = cap;
-        k_scatter<<<(unsigned)blocks, 256, 0, s>>>(knn, tn, T, Tdev, k, L, (unsigned long long*)acc);
+        k_scatter<<<(unsigned)blocks, 256, 0, s>>>(knn, tn, T, Tdev, k, L, order, (unsigned long long*)acc);
         DWG_CHECK_LAUNCH();
     }
     return DWG_OK;
@@ -105,8 +173,9 @@ int diffuse_finish(int L, float* N, long long* acc, unsigned char* is_zero, int*
 }
 
 int diffuse_normals(const int* knn, const float* tn, long long T, const unsigned long long* Tdev, int k, int L,
-                    float* N, long long* acc, unsigned char* is_zero, int* zero_count, cudaStream_t s) {
-    DWG_TRY(diffuse_scatter(knn, tn, T, Tdev, k, L, acc, s));
+                    const int* order, float* N, long long* acc, unsigned char* is_zero, int* zero_count,
+                    cudaStream_t s) {
+    DWG_TRY(diffuse_scatter(knn, tn, T, Tdev, k, L, order, acc, s));
     return diffuse_finish(L, N, acc, is_zero, zero_count, s);
 }
 

@@ -604,12 +604,12 @@ int Pipeline::iterate_post() {
     // normal scatter + normalise (:571-583); sharded: the scatter of this
     // rank's triangles, the sums of all ranks, then the normalisation
     if (world > 1) {
-        DWG_TRY(diffuse_scatter(knn_buf.ptr, tnrm.ptr, cap, ntri.ptr, prm.knn_tri, L, acc.ptr, s));
+        DWG_TRY(diffuse_scatter(knn_buf.ptr, tnrm.ptr, cap, ntri.ptr, prm.knn_tri, L, kidx.q_order.ptr, acc.ptr, s));
         DWG_TRY(exchange_sums());
         DWG_TRY(diffuse_finish(L, leaf_nrm.ptr, acc.ptr, is_zero.ptr, zero_count.ptr, s));
     } else {
-        DWG_TRY(diffuse_normals(knn_buf.ptr, tnrm.ptr, cap, ntri.ptr, prm.knn_tri, L, leaf_nrm.ptr, acc.ptr,
-                                is_zero.ptr, zero_count.ptr, s));
+        DWG_TRY(diffuse_normals(knn_buf.ptr, tnrm.ptr, cap, ntri.ptr, prm.knn_tri, L, kidx.q_order.ptr, leaf_nrm.ptr,
+                                acc.ptr, is_zero.ptr, zero_count.ptr, s));
     }
     // zero-normal repair when more than knn_zero points are zero (:585-644)
     DWG_TRY(zero_repair(kidx, leaf_pos.ptr, L, leaf_nrm.ptr, is_zero.ptr, prm.knn_zero, prm.knn_zero, zws, true, s));

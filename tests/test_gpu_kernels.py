@@ -631,3 +631,25 @@ def test_point_queries_in_any_order(nq):
         assert np.abs(w - w64).max() < 2e-5 * np.abs(w64).max()
         assert np.abs(g - g64).max() < 1e-4 * np.abs(g64).max()
     assert tree.status() == 0
+
+
+@pytest.mark.parametrize("T,k,L", [(1, 1, 1), (136, 15, 40), (137, 15, 5000), (5000, 10, 3), (4000, 15, 200000),
+                                   (40, 64, 30)])
+def test_diffusion_tables(oracle_lib, dwg_lib, T, k, L):
+    # a block's last triangle, tables of a few points and of more than they
+    # hold, one point as every neighbour, absent neighbours (-1), and normals
+    # longer than 1, up and down: the sums are exact, so bit for bit
+    rng = np.random.default_rng(T + k)
+    knn = rng.integers(-1, L, (T, k)).astype(np.int32)
+    knn[: T // 3] = min(2, L - 1)
+    tn = rng.normal(size=(T, 3)).astype(np.float32)
+    tn /= np.linalg.norm(tn, axis=1, keepdims=True)
+    tn[::3] *= rng.choice([1.0, -1.0, 3.0, 1e4, 1e-6], (len(tn[::3]), 1)).astype(np.float32)
+    N0 = rng.normal(size=(L, 3)).astype(np.float32)
+    ref_n, ref_z, ref_c = oracle_lib.diffuse_normals(knn, tn, N0)
+    knn_d, tn_d, n_d = cu(knn), cu(tn), cu(N0)
+    z_d, c_d = torch.zeros(L, dtype=torch.uint8, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    capi.check(dwg_lib.dwg_diffuse_normals(capi.ptr(knn_d), capi.ptr(tn_d), T, k, L, capi.ptr(n_d), capi.ptr(z_d),
+                                           capi.ptr(c_d), None))
+    assert np.array_equal(n_d.cpu().numpy(), ref_n)
+    assert np.array_equal(z_d.cpu().numpy(), ref_z.astype(np.uint8)) and int(c_d.item()) == int(ref_c)
