@@ -295,10 +295,25 @@ int dwg_octree_build(const float* points_dev, int n, int max_depth, const float*
     })
 }
 
-int dwg_octree_destroy(dwg_octree* tree) {
-    delete tree;
+}  // extern "C"
+
+// The library does not know which streams used an octree or an index: the
+// device is waited for, once, and every block goes back to the pool.
+template <typename T>
+static int destroy_idle(T* object) {
+    if (!object) return DWG_OK;
+    if (cudaDeviceSynchronize() == cudaSuccess) {
+        FreeScope idle(nullptr, true);
+        delete object;
+    } else {
+        delete object;
+    }
     return DWG_OK;
 }
+
+extern "C" {
+
+int dwg_octree_destroy(dwg_octree* tree) { return destroy_idle(tree); }
 
 int dwg_octree_num_nodes(const dwg_octree* tree, int* num_nodes) {
     DWG_REQUIRE(tree && num_nodes, "octree_num_nodes: null argument");
@@ -365,7 +380,14 @@ int dwg_octree_export(const dwg_octree* tree, int* depth, int* pt_start, int* pt
         }
         if (cm) DWG_CHECK_CUDA(cudaMemcpy(cm, t.cm_d.ptr, sizeof(double) * 3 * t.M, cudaMemcpyDeviceToHost));
         if (radius) DWG_CHECK_CUDA(cudaMemcpy(radius, t.r_d.ptr, sizeof(double) * t.M, cudaMemcpyDeviceToHost));
-        if (ec) DWG_CHECK_CUDA(cudaMemcpy(ec, t.ec_d.ptr, sizeof(double) * 3 * t.M, cudaMemcpyDeviceToHost));
+        if (ec) {  // kept in level order
+            std::vector<double> e((size_t)t.M * 3);
+            std::vector<int> nodes(t.M);
+            DWG_CHECK_CUDA(cudaMemcpy(e.data(), t.ec_d.ptr, sizeof(double) * 3 * t.M, cudaMemcpyDeviceToHost));
+            DWG_CHECK_CUDA(cudaMemcpy(nodes.data(), t.level_nodes.ptr, sizeof(int) * t.M, cudaMemcpyDeviceToHost));
+            for (int p = 0; p < t.M; ++p)
+                for (int d = 0; d < 3; ++d) ec[(size_t)nodes[p] * 3 + d] = e[(size_t)p * 3 + d];
+        }
         if (perm) DWG_CHECK_CUDA(cudaMemcpy(perm, t.perm.ptr, sizeof(int) * t.n, cudaMemcpyDeviceToHost));
         return DWG_OK;
     })
@@ -577,10 +599,7 @@ int dwg_knn_build(const float* points_dev, int n, void* stream, dwg_knn_index** 
     })
 }
 
-int dwg_knn_destroy(dwg_knn_index* index) {
-    delete index;
-    return DWG_OK;
-}
+int dwg_knn_destroy(dwg_knn_index* index) { return destroy_idle(index); }
 
 int dwg_knn_query(dwg_knn_index* index, const float* queries_dev, long long num_queries, int k, int* out_dev,
                   void* stream) {

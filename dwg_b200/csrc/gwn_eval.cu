@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(128) k_gwn_thread(ThreadArgs a) {
             if (sq3_rn(dxf, dyf, dzf) > na.w) {  // far: the node's dipole term
                 const int v = a.level_nodes[c];
                 const double* cm = a.cm_d + (size_t)v * 3;
-                const double* ec = a.ec_d + (size_t)v * 3;
+                const double* ec = a.ec_d + (size_t)c * 3;
                 add_term<SCREENED, GRAD>(cm[0] - (double)qx, cm[1] - (double)qy, cm[2] - (double)qz, ec[0], ec[1],
                                          ec[2], a.screen, a.sigma, w, g);
                 continue;

@@ -162,34 +162,57 @@ __global__ void k_node_starts(const signed char* __restrict__ lcp, int n, int D,
     nstart[i] = max(0, ld - a);
 }
 
-__global__ void k_level_flags(const signed char* __restrict__ lcp, int n, int d, int* __restrict__ f) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) f[i] = lcp[i] < d ? 1 : 0;
+// the nodes that point i starts, depths lcp_i + 1 .. leaf depth: (i, -, -, depth)
+__global__ void k_node_open(const signed char* __restrict__ lcp, const int* __restrict__ node_base, int n, int D,
+                            int4* __restrict__ info) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int a = lcp[i], ld = min(D, max(a, (int)lcp[i + 1]) + 1);
+    for (int d = a + 1; d <= ld; ++d) info[node_base[i] + (d - a - 1)] = make_int4(i, 0, 0, d);
 }
 
-__global__ void k_level_starts(const signed char* __restrict__ lcp, const int* __restrict__ rank, int n,
-                               int d, int* __restrict__ starts) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int f = lcp[i] < d ? 1 : 0;
-    if (f) starts[rank[i]] = i;
-    if (i == n - 1) starts[rank[i] + f] = n;
-}
-
-__global__ void k_level_nodes(const signed char* __restrict__ lcp, const int* __restrict__ rank,
-                              const int* __restrict__ starts, const int* __restrict__ node_base, int n,
-                              int d, int D, int4* __restrict__ info) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int a = lcp[i];
-    if (a >= d) return;
-    int ld = min(D, max(a, (int)lcp[i + 1]) + 1);
-    if (d > ld) return;
-    int node = node_base[i] + (d - a - 1);
-    int cnt = starts[rank[i] + 1] - i;
-    int skip = node_base[i + cnt];
-    int leaf = (cnt == 1 || d == D) ? kLeafFlag : 0;
-    info[node] = make_int4(i, cnt, skip, d | leaf);
+// A node's points end where the key's first d digits change: found by
+// doubling steps and bisection, so that all nodes of all depths close in one
+// launch (a pass per depth took five launches each): 5 us for 5,000
+// points, 22 for 1.01 M).  Also the depth keys of
+// the level order, the nodes per depth, and the list of big nodes.
+__global__ void __launch_bounds__(256) k_node_close(const unsigned long long* __restrict__ keys,
+                                                    const int* __restrict__ node_base, int n, int D, int M, int big,
+                                                    int4* __restrict__ info, unsigned* __restrict__ depth_key,
+                                                    int* __restrict__ id, int* __restrict__ per_depth,
+                                                    int* __restrict__ big_list) {
+    __shared__ int count[kMaxDepth + 1];
+    if (threadIdx.x <= kMaxDepth) count[threadIdx.x] = 0;
+    __syncthreads();
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < M) {
+        const int4 iv = info[v];
+        const int d = iv.w, sh = 3 * (D - d);
+        const unsigned long long prefix = d > 0 ? keys[iv.x] >> sh : 0ull;
+        int in = iv.x, out = n;  // the last known inside, the first known outside
+        if (d > 0) {
+            for (int step = 1; in + step < n; step *= 2) {
+                if (keys[in + step] >> sh != prefix) {
+                    out = in + step;
+                    break;
+                }
+                in += step;
+            }
+            while (out - in > 1) {
+                const int mid = in + (out - in) / 2;
+                if (keys[mid] >> sh == prefix) in = mid;
+                else out = mid;
+            }
+        }
+        const int cnt = out - iv.x;
+        info[v] = make_int4(iv.x, cnt, node_base[out], d | (cnt == 1 || d == D ? kLeafFlag : 0));
+        depth_key[v] = (unsigned)d;
+        id[v] = v;
+        atomicAdd(&count[d], 1);
+        if (cnt > big) big_list[1 + atomicAdd(big_list, 1)] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x <= kMaxDepth && count[threadIdx.x]) atomicAdd(&per_depth[threadIdx.x], count[threadIdx.x]);
 }
 
 __global__ void k_gather(const float* __restrict__ P, const float* __restrict__ A,
@@ -300,16 +323,19 @@ __global__ void k_centres(const int4* __restrict__ info, const float4* __restric
 // sums, then a fixed tree in shared memory (deterministic), the centre, and
 // the radius as the maximum over the points (exact whatever the order)
 __global__ void __launch_bounds__(kBigThreads) k_centres_big(const int4* __restrict__ info,
-                                                            const float4* __restrict__ pa, int M,
+                                                            const float4* __restrict__ pa,
+                                                            const int* __restrict__ list,
                                                             double* __restrict__ cm_d, double* __restrict__ r_d,
                                                             const int* __restrict__ lvl_of,
                                                             float4* __restrict__ node_a, float* __restrict__ node_r) {
     __shared__ double red[4][kBigThreads];
     const int tid = threadIdx.x;
-    for (long long v = blockIdx.x; v < M; v += gridDim.x) {
+    const int m = list[0];
+    for (int i = blockIdx.x; i < m; i += gridDim.x) {
+        const long long v = list[1 + i];
         const int4 iv = info[v];
-        if (iv.y <= kBigNode) continue;  // the same node for the whole block
         double sa = 0, sx = 0, sy = 0, sz = 0;
+#pragma unroll 8
         for (int j = iv.x + tid; j < iv.x + iv.y; j += kBigThreads) {
             const float4 p = pa[j];
             const double a = p.w;
@@ -333,6 +359,7 @@ __global__ void __launch_bounds__(kBigThreads) k_centres_big(const int4* __restr
                      cz = sa > 0 ? red[3][0] / sa : 0.0;
         __syncthreads();  // every thread has read the sums before the radii reuse the buffer
         double rm = 0;
+#pragma unroll 8
         for (int j = iv.x + tid; j < iv.x + iv.y; j += kBigThreads) {
             const float4 p = pa[j];
             const double dx = (double)p.x - cx, dy = (double)p.y - cy, dz = (double)p.z - cz;
@@ -361,19 +388,18 @@ __global__ void __launch_bounds__(kBigThreads) k_centres_big(const int4* __restr
 
 // sum A n per node, bottom-up one depth level at a time: a leaf sums its
 // points, an internal node its children (in octant order) -- every node's sum
-// has a fixed order, so the result is the same from run to run
-__global__ void k_ec_level(const int* __restrict__ nodes, int p0, int count, const int4* __restrict__ info,
-                           const float4* __restrict__ pa, const float4* __restrict__ nr,
-                           const int* __restrict__ meta, double* __restrict__ ec_d,
-                           float4* __restrict__ node_b) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const int p = p0 + i;
-    const int v = nodes[p];
-    const int4 iv = info[v];
+// has a fixed order, so the result is the same from run to run.  The sums are
+// kept in level order, where a node's children are neighbours: one load after
+// the node's meta word instead of a chain along the children.
+__device__ __forceinline__ void ec_node(int p, const float4* __restrict__ pa, const float4* __restrict__ nr,
+                                        const int* __restrict__ meta, const float4* __restrict__ node_a, double* ec_d,
+                                        float4* __restrict__ node_b) {
+    const unsigned m = (unsigned)meta[p];
+    const int first = (int)(m & kMetaIndex);
     double ex = 0, ey = 0, ez = 0;
-    if (iv.w & kLeafFlag) {
-        for (int j = iv.x; j < iv.x + iv.y; ++j) {
+    if (m & kMetaLeafBit) {
+        const int cnt = (m & kMetaSingle) ? 1 : __float_as_int(node_a[p].w);
+        for (int j = first; j < first + cnt; ++j) {
             const double a = pa[j].w;
             const float4 q = nr[j];
             ex += a * (double)q.x;
@@ -381,16 +407,46 @@ __global__ void k_ec_level(const int* __restrict__ nodes, int p0, int count, con
             ez += a * (double)q.z;
         }
     } else {
-        for (int c = v + 1; c < iv.z; c = info[c].z) {
-            ex += ec_d[(size_t)c * 3];
-            ey += ec_d[(size_t)c * 3 + 1];
-            ez += ec_d[(size_t)c * 3 + 2];
-        }
+        const int nch = (int)((m >> 28) & 7u) + 1;
+        double c[8][3];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) c[j][d] = j < nch ? ec_d[(size_t)(first + j) * 3 + d] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j < nch) {
+                ex += c[j][0];
+                ey += c[j][1];
+                ez += c[j][2];
+            }
     }
-    ec_d[(size_t)v * 3] = ex;
-    ec_d[(size_t)v * 3 + 1] = ey;
-    ec_d[(size_t)v * 3 + 2] = ez;
-    node_b[p] = make_float4((float)ex, (float)ey, (float)ez, __int_as_float(meta[p]));
+    ec_d[(size_t)p * 3] = ex;
+    ec_d[(size_t)p * 3 + 1] = ey;
+    ec_d[(size_t)p * 3 + 2] = ez;
+    node_b[p] = make_float4((float)ex, (float)ey, (float)ez, __int_as_float((int)m));
+}
+
+__global__ void k_ec_level(int p0, int count, const float4* __restrict__ pa, const float4* __restrict__ nr,
+                           const int* __restrict__ meta, const float4* __restrict__ node_a, double* ec_d,
+                           float4* __restrict__ node_b) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) ec_node(p0 + i, pa, nr, meta, node_a, ec_d, node_b);
+}
+
+// a run of small levels by one block, deepest first
+constexpr int kSmallLevel = 2048;
+struct EcRun {
+    int levels, off[kMaxDepth + 2];  // level t of the run: positions off[t + 1] .. off[t]
+};
+__global__ void __launch_bounds__(1024) k_ec_run(EcRun r, const float4* __restrict__ pa, const float4* __restrict__ nr,
+                                                 const int* __restrict__ meta, const float4* __restrict__ node_a,
+                                                 double* ec_d, float4* __restrict__ node_b) {
+    for (int t = 0; t < r.levels; ++t) {
+        for (int p = r.off[t + 1] + (int)threadIdx.x; p < r.off[t]; p += 1024)
+            ec_node(p, pa, nr, meta, node_a, ec_d, node_b);
+        __syncthreads();
+    }
 }
 
 // expansion coefficients about the node's centre c, bottom-up one depth
@@ -403,7 +459,8 @@ __global__ void k_ec_level(const int* __restrict__ nodes, int p0, int count, con
 // with e = sum A n of the child.  Every sum has a fixed order.
 __global__ void k_ho_level(const int* __restrict__ nodes, int p0, int count, const int4* __restrict__ info,
                            const float4* __restrict__ pa, const float4* __restrict__ nr,
-                           const double* __restrict__ cm_d, const double* __restrict__ ec_d, int order,
+                           const double* __restrict__ cm_d, const double* __restrict__ ec_d,
+                           const int* __restrict__ lvl_of, int order,
                            double* __restrict__ ho_d, float4* __restrict__ node_h) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
@@ -437,7 +494,8 @@ __global__ void k_ho_level(const int* __restrict__ nodes, int p0, int count, con
         for (int ch = v + 1; ch < iv.z; ch = info[ch].z) {
             const double d[3] = {cm_d[(size_t)ch * 3] - c0, cm_d[(size_t)ch * 3 + 1] - c1,
                                  cm_d[(size_t)ch * 3 + 2] - c2};
-            const double e[3] = {ec_d[(size_t)ch * 3], ec_d[(size_t)ch * 3 + 1], ec_d[(size_t)ch * 3 + 2]};
+            const double* ce = ec_d + (size_t)lvl_of[ch] * 3;
+            const double e[3] = {ce[0], ce[1], ce[2]};
             const double* hc = ho_d + (size_t)ch * 36;
             double m1c[9];
 #pragma unroll
@@ -514,13 +572,6 @@ __global__ void k_node_meta(const int4* __restrict__ info, const int* __restrict
         m = ((unsigned)lvl_of[v + 1] & kMetaIndex) | ((unsigned)(nch - 1) << 28);
     }
     meta[p] = (int)m;
-}
-
-__global__ void k_depth_key(const int4* __restrict__ info, int M, unsigned* __restrict__ key, int* __restrict__ id) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= M) return;
-    key[v] = (unsigned)(info[v].w & 0xff);
-    id[v] = v;
 }
 
 // Open threshold of a node for opening ratio beta.  With t = beta*R rounded,
@@ -616,6 +667,7 @@ int octree_build(Octree& t, const float* P, int n, int D, const float* A, cudaSt
     DWG_REQUIRE(n >= 1, "octree: need at least one point (n=%d)", n);
     DWG_REQUIRE(D >= 1 && D <= kMaxDepth, "octree: max_depth must be in [1, %d] (got %d)", kMaxDepth, D);
     DWG_REQUIRE(P != nullptr, "octree: null points");
+    FreeScope on_s(s, false);  // the temporaries are used on s alone
     DWG_TRY(require_finite(P, 3ll * n, "octree", s));
     t.n = n;
     t.max_depth = D;
@@ -659,54 +711,39 @@ int octree_build(Octree& t, const float* P, int n, int D, const float* A, cudaSt
     DWG_CHECK_CUDA(cudaStreamSynchronize(s));
     t.M = M;
     DWG_TRY(t.info.reserve(M));
-    DevBuf<int> flags, rank, starts;
-    DWG_TRY(flags.reserve(n));
-    DWG_TRY(rank.reserve(n));
-    DWG_TRY(starts.reserve(n + 1));
-    for (int d = 0; d <= D; d++) {
-        k_level_flags<<<div_up(n, 256), 256, 0, s>>>(lcp.ptr, n, d, flags.ptr);
-        int* fp = flags.ptr;
-        int* rp = rank.ptr;
-        DWG_TRY(cub_call(t.scratch, [&](void* tmp, size_t& bytes) {
-            return cub::DeviceScan::ExclusiveSum(tmp, bytes, fp, rp, n, s);
-        }));
-        k_level_starts<<<div_up(n, 256), 256, 0, s>>>(lcp.ptr, rank.ptr, n, d, starts.ptr);
-        k_level_nodes<<<div_up(n, 256), 256, 0, s>>>(lcp.ptr, rank.ptr, starts.ptr, node_base.ptr, n, d, D,
-                                                      t.info.ptr);
-        DWG_CHECK_LAUNCH();
-    }
-    {
-        // level order: stable radix sort of the nodes by depth
-        DevBuf<unsigned> dkey, dkey2;
-        DevBuf<int> ids;
-        DWG_TRY(dkey.reserve(M));
-        DWG_TRY(dkey2.reserve(M));
-        DWG_TRY(ids.reserve(M));
-        DWG_TRY(t.level_nodes.reserve(M));
-        DWG_TRY(t.lvl_of.reserve(M));
-        DWG_TRY(t.node_meta.reserve(M));
-        k_depth_key<<<div_up(M, 256), 256, 0, s>>>(t.info.ptr, M, dkey.ptr, ids.ptr);
-        DWG_CHECK_LAUNCH();
-        unsigned* k0 = dkey.ptr;
-        unsigned* k1 = dkey2.ptr;
-        int* v0 = ids.ptr;
-        int* v1 = t.level_nodes.ptr;
-        DWG_TRY(cub_call(t.scratch, [&](void* tmp, size_t& bytes) {
-            return cub::DeviceRadixSort::SortPairs(tmp, bytes, k0, k1, v0, v1, M, 0, 5, s);
-        }));
-        std::vector<unsigned> h(M);
-        DWG_CHECK_CUDA(cudaMemcpyAsync(h.data(), dkey2.ptr, sizeof(unsigned) * M, cudaMemcpyDeviceToHost, s));
-        DWG_CHECK_CUDA(cudaStreamSynchronize(s));
-        for (int d = 0; d <= kMaxDepth + 1; ++d) t.level_off[d] = M;
-        for (int p = M - 1; p >= 0; --p) t.level_off[h[p]] = p;
-        t.level_off[0] = 0;
-        for (int d = kMaxDepth; d >= 0; --d)
-            if (t.level_off[d] > t.level_off[d + 1]) t.level_off[d] = t.level_off[d + 1];
-        k_lvl_of<<<div_up(M, 256), 256, 0, s>>>(t.level_nodes.ptr, M, t.lvl_of.ptr);
-        k_node_meta<<<div_up(M, 256), 256, 0, s>>>(t.info.ptr, t.level_nodes.ptr, t.lvl_of.ptr, M, t.node_meta.ptr);
-        DWG_CHECK_LAUNCH();
-        DWG_CHECK_CUDA(cudaStreamSynchronize(s));
-    }
+    // the nodes, and their level order by a stable radix sort on the depth
+    DevBuf<unsigned> dkey, dkey2;
+    DevBuf<int> ids, per_depth;
+    DWG_TRY(dkey.reserve(M));
+    DWG_TRY(dkey2.reserve(M));
+    DWG_TRY(ids.reserve(M));
+    DWG_TRY(per_depth.reserve(kMaxDepth + 1));
+    // disjoint nodes of a depth hold n points, so at most n / kBigNode of them are big
+    DWG_TRY(t.big_nodes.reserve(1 + (size_t)(D + 1) * (n / kBigNode)));
+    DWG_TRY(t.level_nodes.reserve(M));
+    DWG_TRY(t.lvl_of.reserve(M));
+    DWG_TRY(t.node_meta.reserve(M));
+    DWG_CHECK_CUDA(cudaMemsetAsync(per_depth.ptr, 0, sizeof(int) * (kMaxDepth + 1), s));
+    DWG_CHECK_CUDA(cudaMemsetAsync(t.big_nodes.ptr, 0, sizeof(int), s));
+    k_node_open<<<div_up(n, 256), 256, 0, s>>>(lcp.ptr, node_base.ptr, n, D, t.info.ptr);
+    k_node_close<<<div_up(M, 256), 256, 0, s>>>(t.keys.ptr, node_base.ptr, n, D, M, kBigNode, t.info.ptr, dkey.ptr,
+                                                 ids.ptr, per_depth.ptr, t.big_nodes.ptr);
+    DWG_CHECK_LAUNCH();
+    unsigned* k0 = dkey.ptr;
+    unsigned* k1 = dkey2.ptr;
+    int* v0 = ids.ptr;
+    int* v1 = t.level_nodes.ptr;
+    DWG_TRY(cub_call(t.scratch, [&](void* tmp, size_t& bytes) {
+        return cub::DeviceRadixSort::SortPairs(tmp, bytes, k0, k1, v0, v1, M, 0, 5, s);
+    }));
+    int h[kMaxDepth + 1];
+    DWG_CHECK_CUDA(cudaMemcpyAsync(h, per_depth.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
+    k_lvl_of<<<div_up(M, 256), 256, 0, s>>>(t.level_nodes.ptr, M, t.lvl_of.ptr);
+    k_node_meta<<<div_up(M, 256), 256, 0, s>>>(t.info.ptr, t.level_nodes.ptr, t.lvl_of.ptr, M, t.node_meta.ptr);
+    DWG_CHECK_LAUNCH();
+    DWG_CHECK_CUDA(cudaStreamSynchronize(s));
+    t.level_off[0] = 0;
+    for (int d = 0; d <= kMaxDepth; ++d) t.level_off[d + 1] = t.level_off[d] + h[d];
     DWG_TRY(t.pa.reserve(n));
     DWG_TRY(t.nr.reserve(n));
     k_gather<<<div_up(n, 256), 256, 0, s>>>(P, A, t.perm.ptr, n, t.pa.ptr, t.nr.ptr, t.inv_perm.ptr);
@@ -751,7 +788,7 @@ int octree_update_centres(Octree& t, cudaStream_t s) {
                                                   t.node_a.ptr, t.node_r.ptr);
     DWG_CHECK_LAUNCH();
     if (t.n > kBigNode) {
-        k_centres_big<<<num_sms() * 2, kBigThreads, 0, s>>>(t.info.ptr, t.pa.ptr, t.M, t.cm_d.ptr, t.r_d.ptr,
+        k_centres_big<<<num_sms() * 2, kBigThreads, 0, s>>>(t.info.ptr, t.pa.ptr, t.big_nodes.ptr, t.cm_d.ptr, t.r_d.ptr,
                                                             t.lvl_of.ptr, t.node_a.ptr, t.node_r.ptr);
         DWG_CHECK_LAUNCH();
     }
@@ -769,11 +806,23 @@ int octree_set_beta(Octree& t, float beta, cudaStream_t s) {
 }
 
 int octree_update_normals(Octree& t, cudaStream_t s) {
-    for (int d = t.max_depth; d >= 0; --d) {
-        int cnt = t.level_off[d + 1] - t.level_off[d];
-        if (cnt <= 0) continue;
-        k_ec_level<<<div_up(cnt, 128), 128, 0, s>>>(t.level_nodes.ptr, t.level_off[d], cnt, t.info.ptr, t.pa.ptr,
-                                                     t.nr.ptr, t.node_meta.ptr, t.ec_d.ptr, t.node_b.ptr);
+    for (int d = t.max_depth; d >= 0;) {
+        const int cnt = t.level_off[d + 1] - t.level_off[d];
+        // levels of up to kSmallLevel nodes next to each other share a
+        // launch: a launch of its own takes ~4 us, a pass of the block 1 to 2
+        if (cnt <= kSmallLevel) {
+            EcRun r;
+            r.levels = 0;
+            r.off[0] = t.level_off[d + 1];
+            while (d >= 0 && t.level_off[d + 1] - t.level_off[d] <= kSmallLevel) r.off[++r.levels] = t.level_off[d--];
+            if (r.off[0] > r.off[r.levels])
+                k_ec_run<<<1, 1024, 0, s>>>(r, t.pa.ptr, t.nr.ptr, t.node_meta.ptr, t.node_a.ptr, t.ec_d.ptr,
+                                            t.node_b.ptr);
+            continue;
+        }
+        k_ec_level<<<div_up(cnt, 128), 128, 0, s>>>(t.level_off[d], cnt, t.pa.ptr, t.nr.ptr, t.node_meta.ptr,
+                                                     t.node_a.ptr, t.ec_d.ptr, t.node_b.ptr);
+        --d;
     }
     DWG_CHECK_LAUNCH();
     return DWG_OK;
@@ -787,7 +836,7 @@ int octree_update_expansion(Octree& t, int order, cudaStream_t s) {
         int cnt = t.level_off[d + 1] - t.level_off[d];
         if (cnt <= 0) continue;
         k_ho_level<<<div_up(cnt, 64), 64, 0, s>>>(t.level_nodes.ptr, t.level_off[d], cnt, t.info.ptr, t.pa.ptr,
-                                                   t.nr.ptr, t.cm_d.ptr, t.ec_d.ptr, order, t.ho_d.ptr,
+                                                   t.nr.ptr, t.cm_d.ptr, t.ec_d.ptr, t.lvl_of.ptr, order, t.ho_d.ptr,
                                                    t.node_h.ptr);
     }
     DWG_CHECK_LAUNCH();

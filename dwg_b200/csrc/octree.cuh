@@ -10,12 +10,13 @@
 //     info[v] = (pt_start, pt_count, skip, depth | LEAF)   int4
 //     skip[v] = index of the first node after v's subtree, so the children of
 //     v are v+1, skip[v+1], ... while < skip[v]
-//     cm_d, r_d, ec_d: FP64 moments, pre-order
+//     cm_d, r_d: FP64 centres and radii, pre-order
 //   traversal records, numbered p in level order (by depth, then pre-order),
 //   where the children of a node are consecutive:
 //     node_a[p] = (cm.x, cm.y, cm.z, open threshold | leaf point count)  float4
 //     node_b[p] = (sum A n .x, .y, .z, meta)                             float4
 //     node_r[p] = R (max |p - cm|, rounded from FP64)                    float
+//     ec_d[p] = sum A n in FP64
 //     level_nodes[p] = v,  lvl_of[v] = p
 //   meta of an internal node: first child p (bits 0-27) | (children - 1) << 28;
 //   of a leaf: LEAF (bit 31) | SINGLE (bit 30, one point) | pt_start (bits 0-27).
@@ -62,6 +63,7 @@ struct Octree {
     DevBuf<float4> node_h;
     // level order: level d = positions level_off[d] .. level_off[d+1]
     DevBuf<int> level_nodes, lvl_of, node_meta;
+    DevBuf<int> big_nodes;  // [0] number, then the nodes of many points (any order)
     int level_off[kMaxDepth + 2] = {0};
     DevBuf<unsigned char> scratch;  // CUB temporary storage
     mutable QueryOrder qorder;          // spatial order of point queries

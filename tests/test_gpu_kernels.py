@@ -653,3 +653,28 @@ def test_diffusion_tables(oracle_lib, dwg_lib, T, k, L):
                                            capi.ptr(c_d), None))
     assert np.array_equal(n_d.cpu().numpy(), ref_n)
     assert np.array_equal(z_d.cpu().numpy(), ref_z.astype(np.uint8)) and int(c_d.item()) == int(ref_c)
+
+
+@pytest.mark.parametrize("n,depth", [(1, 3), (2, 1), (3, 21), (255, 2), (257, 5), (5000, 4), (9000, 21)])
+def test_octree_nodes_and_moments_at_edges(oracle_lib, n, depth):
+    # every node's range found by bisection over the sorted keys (the last
+    # block's nodes, one point, points at one spot, depth 1 and the deepest),
+    # nodes of more than 4,096 points, and the bottom-up sums over levels of
+    # one node and of thousands
+    rng = np.random.default_rng(n + depth)
+    P = rng.uniform(-0.5, 0.5, (n, 3)).astype(np.float32)
+    P[: n // 3] = P[0]
+    N = rng.normal(size=(n, 3)).astype(np.float32)
+    A = rng.uniform(1e-6, 3e-6, n).astype(np.float32)
+    gt = turbo.TurboLibiGWN(cu(P), max_depth=depth, areas=cu(A))
+    gt.UpdateMassNormals(cu(N), cu(A))
+    g, ot = gt.export(), oracle_lib.Octree(P, depth)
+    idx = match_nodes(g, ot)
+    assert np.array_equal(g["perm"], ot.dfs_order())
+    assert len(idx) == int((ot.counts > 0).sum()) and np.array_equal(g["pt_count"], ot.counts[idx])
+    end = np.array([np.flatnonzero(np.append(g["depth"][v + 1:] <= g["depth"][v], True))[0] + v + 1
+                    for v in range(len(idx))])
+    assert np.array_equal(g["skip"], end)
+    CM, R, EC = ot.moments(P, N, A)
+    assert np.allclose(g["cm"], CM[idx], rtol=0, atol=1e-14) and np.allclose(g["radius"], R[idx], rtol=0, atol=1e-14)
+    assert np.allclose(g["ec"], EC[idx], rtol=1e-11, atol=1e-17)
