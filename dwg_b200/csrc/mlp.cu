@@ -11,9 +11,10 @@
 // is buried in the sampling noise.  The network maps them to a 3-vector
 // that is normalised into an initial normal.
 //
-// GEMMs run on the tensor cores with mma.sync m16n8k16 (BF16 inputs, FP32
-// accumulation); activations are rounded to BF16 where they feed a GEMM and
-// kept in FP32 elsewhere.  Training is mean cosine loss with Adam.
+// The products run on the tensor cores with mma.sync m16n8k16 (BF16 inputs,
+// FP32 accumulation); activations are rounded to BF16 where they feed a
+// product and kept in FP32 elsewhere.  Training is mean cosine loss with Adam.
+#include <algorithm>
 #include <cmath>
 #include <random>
 #include <vector>
@@ -185,196 +186,409 @@ int mlp_features(const KnnIndex& ix, const float* P, int n, float* F, cudaStream
     return DWG_OK;
 }
 
-// ------------------------------------------------------------------- GEMM --
-__device__ __forceinline__ unsigned pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-    return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
+// ---------------------------------------------------------- the network --
+// Two kernels.  k_mlp_rows takes a warp 16 rows through the whole network:
+// the weights sit in shared memory, a layer's product stays in registers, and
+// its activations are the next product's left operand as they stand (the
+// accumulator layout of mma.m16n8k16 is that of its A operand), so a forward
+// pass touches global memory for the features and the outputs only.  Training
+// runs the backward products the same way; what the weight gradients need
+// (activations and dZ in BF16) and gelu' (FP32, read back by the thread that
+// wrote it) go to global memory in the fragments' own order, 512 bytes per
+// warp and store.  k_mlp_weights forms H^T dZ per chunk of rows in shared
+// memory.  Its partial sums, and the bias sums of k_mlp_rows, are added in a
+// fixed order.  65,536 rows, forward and backward: @R@ us and @W@ us (1,030 us
+// with a GEMM, an elementwise and a column-sum kernel per layer, each through
+// global memory with 16-bit loads); the error function and the exponential
+// bound the first.
+__device__ __forceinline__ unsigned pack2(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const unsigned*>(&v);
 }
 
-// C[M x N] (FP32, ldc) (+)= op(A)[M x K] op(B)[K x N], BF16 operands.
-// op(A)(r, c) = TA ? A[c * lda + r] : A[r * lda + c]
-// op(B)(k, c) = TB ? B[c * ldb + k] : B[k * ldb + c]
-// One warp computes a 16 x 32 tile with mma.sync.m16n8k16 (fragment layout of
-// the PTX ISA: lane = 4 g + t holds rows g, g+8 and columns 2t, 2t+1, +8).
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(128) k_gemm(const __nv_bfloat16* __restrict__ A, int lda,
-                                              const __nv_bfloat16* __restrict__ B, int ldb, float* __restrict__ C,
-                                              int ldc, int M, int N, int K, int accumulate, int k_chunk) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int m0 = (blockIdx.x * 4 + warp) * 16;
-    const int n0 = blockIdx.y * 32;
-    if (m0 >= M) return;
-    // split K: slice z covers [kb, ke) and writes its own M x N partial
-    const int kb = blockIdx.z * k_chunk;
-    const int ke = kb + k_chunk < K ? kb + k_chunk : K;
-    C += (size_t)blockIdx.z * M * ldc;
-    const __nv_bfloat16 zero = __float2bfloat16(0.f);
-    auto ldA = [&](int r, int c) -> __nv_bfloat16 {
-        if (r >= M || c >= ke) return zero;
-        return TA ? A[(size_t)c * lda + r] : A[(size_t)r * lda + c];
-    };
-    auto ldB = [&](int k, int c) -> __nv_bfloat16 {
-        if (k >= ke || c >= N) return zero;
-        return TB ? B[(size_t)c * ldb + k] : B[(size_t)k * ldb + c];
-    };
-    float acc[4][4];
+__device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// four 8x8 tiles; lane l gives the row l & 7 of tile l >> 3
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], const __nv_bfloat16* row) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(row);
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a)
+                     : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a)
+                     : "memory");
+}
+
+// gelu (erf form) and its derivative
+__device__ __forceinline__ float gelu_both(float x, float& grad) {
+    const float u = 1.0f + erff(x * 0.7071067811865476f);
+    grad = 0.5f * u + x * 0.3989422804014327f * expf(-0.5f * x * x);
+    return 0.5f * x * u;
+}
+
+constexpr int kRowWarps = 8;
+constexpr int kWPad = kMlpHidden + 8;  // row stride of the weights in shared memory: conflict-free ldmatrix
+constexpr int kW4Pad = 16;             // row stride of the last layer's
+constexpr int kNT = kMlpHidden / 8;    // column tiles of a hidden layer
+// offsets (BF16) of the layers' weights in shared memory
+constexpr int kS1 = 0, kS2 = kS1 + kMlpInPad * kWPad, kS3 = kS2 + kMlpHidden * kWPad, kS4 = kS3 + kMlpHidden * kWPad;
+constexpr int kSBias = kS4 + kMlpHidden * kW4Pad;  // then the biases (FP32): 3 x 128, 8
+constexpr int kBias = 3 * kMlpHidden + kMlpOutPad;
+constexpr int kRowSmem = kSBias * 2 + kBias * 4 + kRowWarps * kBias * 4;  // and the warps' bias sums
+
+struct RowArgs {
+    const float* F;
+    const float* T;
+    long long rows;
+    const __nv_bfloat16* w[kMlpLayers];
+    const float* b[kMlpLayers];
+    float* out;            // forward: raw outputs, 3 per row
+    float4* gp[3];         // training: gelu' of the hidden layers
+    uint4* x;              // the inputs, hidden activations, dZ of the hidden layers and of the outputs
+    uint2* h[3];
+    uint2* dz[3];
+    unsigned* dy;
+    float* bias_part;      // per block: the bias gradients
+    double* loss_part;     // per block
+};
+
+// acc[16 x N] += A[16 x 16 K] op(W): the weights of a layer as they are
+// (TRANS false: B[k][n] = W[n][k], the backward products)
+template <int K, int N, bool FORWARD>
+__device__ __forceinline__ void row_product(float (&acc)[N][4], const unsigned (&A)[K][4], const __nv_bfloat16* w,
+                                            int stride, int lane) {
+    const int t = lane >> 3, r = lane & 7;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int kk = 0; kk < K; ++kk)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
-    for (int k0 = kb; k0 < ke; k0 += 16) {
-        const int r0 = m0 + g, r1 = m0 + g + 8, c0 = k0 + 2 * t, c1 = k0 + 2 * t + 8;
-        const unsigned a0 = pack_bf16(ldA(r0, c0), ldA(r0, c0 + 1));
-        const unsigned a1 = pack_bf16(ldA(r1, c0), ldA(r1, c0 + 1));
-        const unsigned a2 = pack_bf16(ldA(r0, c1), ldA(r0, c1 + 1));
-        const unsigned a3 = pack_bf16(ldA(r1, c1), ldA(r1, c1 + 1));
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = n0 + 8 * j + g;
-            const unsigned b0 = pack_bf16(ldB(c0, col), ldB(c0 + 1, col));
-            const unsigned b1 = pack_bf16(ldB(c1, col), ldB(c1 + 1, col));
-            asm volatile(
-                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                "{%0,%1,%2,%3};\n"
-                : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
-                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        for (int n = 0; n < N; n += 2) {
+            unsigned b[4];
+            if (FORWARD) ldmatrix4<true>(b, w + (kk * 16 + (t & 1) * 8 + r) * stride + n * 8 + (t >> 1) * 8);
+            else ldmatrix4<false>(b, w + (n * 8 + (t >> 1) * 8 + r) * stride + kk * 16 + (t & 1) * 8);
+            mma16816(acc[n], A[kk], b[0], b[1]);
+            mma16816(acc[n + 1], A[kk], b[2], b[3]);
         }
+}
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(kRowWarps * 32, 2) k_mlp_rows(RowArgs a) {
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    __nv_bfloat16* const ws = reinterpret_cast<__nv_bfloat16*>(row_smem);
+    float* const bs = reinterpret_cast<float*>(row_smem + kSBias * 2);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    float* const bsum = bs + kBias + w * kBias;
+    const int stride[kMlpLayers] = {kWPad, kWPad, kWPad, kW4Pad}, at[kMlpLayers] = {kS1, kS2, kS3, kS4};
+#pragma unroll
+    for (int l = 0; l < kMlpLayers; ++l) {
+        const int din = l == 0 ? kMlpInPad : kMlpHidden, dout = l == 3 ? kMlpOutPad : kMlpHidden;
+        for (int i = tid; i < din * stride[l]; i += kRowWarps * 32) {
+            const int r = i / stride[l], c = i % stride[l];
+            ws[at[l] + i] = c < dout ? a.w[l][r * dout + c] : __float2bfloat16(0.f);
+        }
+        for (int i = tid; i < dout; i += kRowWarps * 32) bs[l * kMlpHidden + i] = a.b[l][i];
     }
+    for (int i = lane; i < kBias; i += 32) bsum[i] = 0.f;
+    __syncthreads();
+    double loss = 0.0;
+    const long long tiles = (a.rows + 15) / 16, warps = (long long)gridDim.x * kRowWarps;
+    for (long long tile = (long long)blockIdx.x * kRowWarps + w; tile < tiles; tile += warps) {
+        const long long row[2] = {tile * 16 + g, tile * 16 + g + 8};
+        const bool in[2] = {row[0] < a.rows, row[1] < a.rows};
+        float acc[kNT][4];
+        unsigned A[kMlpHidden / 16][4];
+        {
+            unsigned X[1][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int col = n0 + 8 * j + 2 * t;
-        const int rows[2] = {m0 + g, m0 + g + 8};
+            for (int q = 0; q < 4; ++q) {  // rows g, g + 8; columns 2t, then 2t + 8
+                const int c = 2 * t + (q >> 1) * 8;
+                float2 v = make_float2(0.f, 0.f);
+                if (in[q & 1] && c < kMlpIn) {
+                    const float* f = a.F + row[q & 1] * kMlpIn + c;
+                    v = make_float2(f[0], f[1]);
+                }
+                X[0][q] = pack2(v.x, v.y);
+            }
+            if (TRAIN) a.x[tile * 32 + lane] = make_uint4(X[0][0], X[0][1], X[0][2], X[0][3]);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = rows[h];
-            if (r >= M) continue;
+            for (int n = 0; n < kNT; ++n)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int cc = col + e;
-                if (cc >= N) continue;
-                float* dst = C + (size_t)r * ldc + cc;
-                const float v = acc[j][2 * h + e];
-                *dst = accumulate ? *dst + v : v;
+                for (int q = 0; q < 4; ++q) acc[n][q] = 0.f;
+            row_product<1, kNT, true>(acc, X, ws + kS1, kWPad, lane);
+        }
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            // activations: FP32 pre-activations, BF16 into the next product
+#pragma unroll
+            for (int n = 0; n < kNT; ++n) {
+                const float2 b = *reinterpret_cast<const float2*>(bs + l * kMlpHidden + n * 8 + 2 * t);
+                float4 d;
+                const float h0 = gelu_both(acc[n][0] + b.x, d.x), h1 = gelu_both(acc[n][1] + b.y, d.y);
+                const float h2 = gelu_both(acc[n][2] + b.x, d.z), h3 = gelu_both(acc[n][3] + b.y, d.w);
+                const unsigned lo = pack2(h0, h1), hi = pack2(h2, h3);
+                A[n / 2][(n & 1) * 2] = lo;
+                A[n / 2][(n & 1) * 2 + 1] = hi;
+                if (TRAIN) {
+                    const long long o = (tile * kNT + n) * 32 + lane;
+                    a.gp[l][o] = d;
+                    a.h[l][o] = make_uint2(lo, hi);
+                }
+            }
+            if (l == 2) break;
+#pragma unroll
+            for (int n = 0; n < kNT; ++n)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[n][q] = 0.f;
+            row_product<kMlpHidden / 16, kNT, true>(acc, A, ws + (l == 0 ? kS2 : kS3), kWPad, lane);
+        }
+        // outputs: columns 2t, 2t + 1 of 8 (the second column tile is padding)
+        float y[2][4] = {};
+        row_product<kMlpHidden / 16, 2, true>(y, A, ws + kS4, kW4Pad, lane);
+        const float* b4 = bs + 3 * kMlpHidden + 2 * t;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y[0][q] += b4[q & 1];
+        if (!TRAIN) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+                if (in[s]) {
+                    if (t < 2) a.out[row[s] * 3 + 2 * t] = y[0][2 * s];
+                    if (t == 0) a.out[row[s] * 3 + 1] = y[0][2 * s + 1];
+                }
+            continue;
+        }
+        // cosine loss and dY (BF16) of the two rows
+        unsigned D[1][4] = {};
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const float y0 = __shfl_sync(0xffffffffu, y[0][2 * s], lane & ~3),
+                        y1 = __shfl_sync(0xffffffffu, y[0][2 * s + 1], lane & ~3),
+                        y2 = __shfl_sync(0xffffffffu, y[0][2 * s], (lane & ~3) + 1);
+            float d[3] = {0.f, 0.f, 0.f};
+            if (in[s]) {
+                const float* tr = a.T + row[s] * 3;
+                const float nn = sqrtf(y0 * y0 + y1 * y1 + y2 * y2) + 1e-12f;
+                const float yh[3] = {y0 / nn, y1 / nn, y2 / nn};
+                const float c = yh[0] * tr[0] + yh[1] * tr[1] + yh[2] * tr[2];
+                if (t == 0) loss += (double)(1.0f - c);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) d[q] = -(tr[q] - c * yh[q]) / nn / (float)a.rows;
+            }
+            D[0][s] = t == 0 ? pack2(d[0], d[1]) : t == 1 ? pack2(d[2], 0.f) : 0u;
+        }
+        a.dy[(tile * 32 + lane) * 2] = D[0][0];
+        a.dy[(tile * 32 + lane) * 2 + 1] = D[0][1];
+        // the output bias sums the BF16 dY
+        {
+            float s0 = __uint_as_float(D[0][0] << 16) + __uint_as_float(D[0][1] << 16);
+            float s1 = __uint_as_float(D[0][0] & 0xffff0000u) + __uint_as_float(D[0][1] & 0xffff0000u);
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+            }
+            if (g == 0) {
+                bsum[3 * kMlpHidden + 2 * t] += s0;
+                bsum[3 * kMlpHidden + 2 * t + 1] += s1;
+            }
+        }
+#pragma unroll
+        for (int l = 2; l >= 0; --l) {
+            // dH of layer l's activations, then dZ = dH gelu'
+#pragma unroll
+            for (int n = 0; n < kNT; ++n)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[n][q] = 0.f;
+            if (l == 2) row_product<1, kNT, false>(acc, D, ws + kS4, kW4Pad, lane);
+            else row_product<kMlpHidden / 16, kNT, false>(acc, A, ws + (l == 1 ? kS3 : kS2), kWPad, lane);
+#pragma unroll
+            for (int n = 0; n < kNT; ++n) {
+                const long long o = (tile * kNT + n) * 32 + lane;
+                const float4 d = a.gp[l][o];
+                acc[n][0] *= d.x;
+                acc[n][1] *= d.y;
+                acc[n][2] *= d.z;
+                acc[n][3] *= d.w;
+                const unsigned lo = pack2(acc[n][0], acc[n][1]), hi = pack2(acc[n][2], acc[n][3]);
+                A[n / 2][(n & 1) * 2] = lo;
+                A[n / 2][(n & 1) * 2 + 1] = hi;
+                a.dz[l][o] = make_uint2(lo, hi);
+                // the bias gradient sums the FP32 dZ over the 16 rows
+                float s0 = acc[n][0] + acc[n][2], s1 = acc[n][1] + acc[n][3];
+#pragma unroll
+                for (int x = 4; x < 32; x <<= 1) {
+                    s0 += __shfl_xor_sync(0xffffffffu, s0, x);
+                    s1 += __shfl_xor_sync(0xffffffffu, s1, x);
+                }
+                if (g == 0) {
+                    bsum[l * kMlpHidden + n * 8 + 2 * t] += s0;
+                    bsum[l * kMlpHidden + n * 8 + 2 * t + 1] += s1;
+                }
             }
         }
     }
-}
-
-// sums the partial products of the K slices in slice order (deterministic)
-__global__ void k_sum_slices(const float* __restrict__ part, int slices, long long mn, float* __restrict__ C) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= mn) return;
-    float acc = 0.f;
-    for (int z = 0; z < slices; ++z) acc += part[(size_t)z * mn + i];
-    C[i] = acc;
-}
-
-template <bool TA, bool TB>
-static int gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* C, int ldc, int M, int N, int K,
-                bool accumulate, cudaStream_t s, DevBuf<float>* split_ws = nullptr) {
-    // a long K over a small output (weight gradients: K = batch) is split into
-    // slices of 1024 so that the whole GPU works on it
-    int slices = 1, chunk = K;
-    if (split_ws && !accumulate && ldc == N && (long long)div_up(M, 64) * div_up(N, 32) < 148 && K > 2048) {
-        chunk = 1024;
-        slices = (int)div_up(K, chunk);
-        DWG_TRY(split_ws->reserve((size_t)slices * M * N));
-    }
-    dim3 grid(div_up(M, 64), div_up(N, 32), slices);
-    float* dst = slices > 1 ? split_ws->ptr : C;
-    k_gemm<TA, TB><<<grid, 128, 0, s>>>(A, lda, B, ldb, dst, ldc, M, N, K, accumulate ? 1 : 0, chunk);
-    DWG_CHECK_LAUNCH();
-    if (slices > 1) {
-        const long long mn = (long long)M * N;
-        k_sum_slices<<<div_up(mn, 256), 256, 0, s>>>(split_ws->ptr, slices, mn, C);
-        DWG_CHECK_LAUNCH();
-    }
-    return DWG_OK;
-}
-
-// ------------------------------------------------------------ elementwise --
-__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.7071067811865476f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-    return 0.5f * (1.0f + erff(x * 0.7071067811865476f)) + x * 0.3989422804014327f * expf(-0.5f * x * x);
-}
-
-__global__ void k_pack_x(const float* __restrict__ F, long long n, __nv_bfloat16* __restrict__ X) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n * kMlpInPad) return;
-    const long long r = i / kMlpInPad;
-    const int c = (int)(i % kMlpInPad);
-    X[i] = __float2bfloat16_rn(c < kMlpIn ? F[r * kMlpIn + c] : 0.f);
-}
-
-// z += b; h = bf16(gelu(z)) (hidden layers) -- z keeps the FP32 pre-activation
-__global__ void k_bias_act(float* __restrict__ z, const float* __restrict__ b, __nv_bfloat16* __restrict__ h,
-                           long long rows, int cols, int act) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= rows * cols) return;
-    const float v = z[i] + b[i % cols];
-    z[i] = v;
-    if (act) h[i] = __float2bfloat16_rn(gelu(v));
-}
-
-// cosine loss of the first 3 outputs; dY (BF16, 8 columns) and the loss sum
-__global__ void k_cos_loss(const float* __restrict__ y, const float* __restrict__ tgt, long long rows,
-                           __nv_bfloat16* __restrict__ dy, float* __restrict__ loss) {
-    long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (r < rows) {
-        const float* yr = y + r * kMlpOutPad;
-        const float* tr = tgt + r * 3;
-        const float nn = sqrtf(yr[0] * yr[0] + yr[1] * yr[1] + yr[2] * yr[2]) + 1e-12f;
-        const float yh[3] = {yr[0] / nn, yr[1] / nn, yr[2] / nn};
-        const float c = yh[0] * tr[0] + yh[1] * tr[1] + yh[2] * tr[2];
-        l = (1.0f - c) / (float)rows;
-        for (int d = 0; d < kMlpOutPad; ++d) {
-            float g = 0.f;
-            if (d < 3) g = -(tr[d] - c * yh[d]) / nn / (float)rows;
-            dy[r * kMlpOutPad + d] = __float2bfloat16_rn(g);
+    if (TRAIN) {
+        // the block's warps in order
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
+        __shared__ double losses[kRowWarps];
+        if (lane == 0) losses[w] = loss;
+        __syncthreads();
+        for (int i = tid; i < kBias; i += kRowWarps * 32) {
+            float s = 0.f;
+            for (int k = 0; k < kRowWarps; ++k) s += bs[kBias + k * kBias + i];
+            a.bias_part[(size_t)blockIdx.x * kBias + i] = s;
+        }
+        if (tid == 0) {
+            double s = 0.0;
+            for (int k = 0; k < kRowWarps; ++k) s += losses[k];
+            a.loss_part[blockIdx.x] = s;
         }
     }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(loss, l);
 }
 
-// dZ = dH * gelu'(z): FP32 kept for the bias gradient, BF16 for the GEMMs
-__global__ void k_gelu_back(const float* __restrict__ dh, const float* __restrict__ z, long long n,
-                            float* __restrict__ dz, __nv_bfloat16* __restrict__ dzb) {
-    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = dh[i] * gelu_grad(z[i]);
-    dz[i] = v;
-    dzb[i] = __float2bfloat16_rn(v);
-}
+// Weight gradients of a chunk of row tiles (128 rows at a time): blockIdx.y 0
+// and 1 the two hidden products (a warp 16 of the 128 rows of dW), 2 the first
+// and the last layer's.
+constexpr int kWRows = 128;
+constexpr int kWSmem = (2 * kWRows * kWPad + kWRows * 24 + kWRows * 24) * 2;
+struct WeightArgs {
+    long long tiles;  // of 16 rows
+    const uint4* x;
+    const uint2* h[3];
+    const uint2* dz[3];
+    const unsigned* dy;
+    float* part;  // per chunk: dW of the four layers (16 x 128, 128 x 128 twice, 128 x 8)
+};
+// places of the layers' dW in a part, and its size
+constexpr int kPart1 = kMlpInPad * kMlpHidden, kPart2 = kPart1 + kMlpHidden * kMlpHidden,
+              kPart3 = kPart2 + kMlpHidden * kMlpHidden, kParts = kPart3 + kMlpHidden * kMlpOutPad;
 
-// column sums (bias gradients), one block per column, fixed order
-__global__ void k_colsum_f32(const float* __restrict__ x, long long rows, int cols, float* __restrict__ out) {
-    const int c = blockIdx.x;
-    float acc = 0.f;
-    for (long long r = threadIdx.x; r < rows; r += blockDim.x) acc += x[r * cols + c];
-    __shared__ float sh[256];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+__global__ void __launch_bounds__(kRowWarps * 32) k_mlp_weights(WeightArgs a) {
+    extern __shared__ __align__(16) unsigned char w_smem[];
+    __nv_bfloat16* const hs = reinterpret_cast<__nv_bfloat16*>(w_smem);  // [row][column]
+    __nv_bfloat16* const ds = hs + kWRows * kWPad;
+    __nv_bfloat16* const xs = ds + kWRows * kWPad;  // stride 24: the inputs, and dY
+    __nv_bfloat16* const ys = xs + kWRows * 24;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3, lt = lane >> 3, lr = lane & 7;
+    const int kind = blockIdx.y;
+    const uint2* H = kind == 2 ? a.h[2] : a.h[kind];
+    const uint2* Z = kind == 2 ? a.dz[0] : a.dz[kind + 1];
+    float acc[kNT][4];
+#pragma unroll
+    for (int n = 0; n < kNT; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[n][q] = 0.f;
+    const long long sets = (a.tiles + 7) / 8;
+    for (long long set = blockIdx.x; set < sets; set += gridDim.x) {
+        // the warp's 16 rows, fragments back to rows
+        const long long tile = set * 8 + w;
+        const bool in = tile < a.tiles;
         __syncthreads();
+#pragma unroll 4
+        for (int n = 0; n < kNT; ++n) {
+            const long long o = (tile * kNT + n) * 32 + lane;
+            const uint2 h = in ? H[o] : make_uint2(0u, 0u), z = in ? Z[o] : make_uint2(0u, 0u);
+            const int c = (w * 16 + g) * kWPad + n * 8 + 2 * t;
+            *reinterpret_cast<unsigned*>(hs + c) = h.x;
+            *reinterpret_cast<unsigned*>(hs + c + 8 * kWPad) = h.y;
+            *reinterpret_cast<unsigned*>(ds + c) = z.x;
+            *reinterpret_cast<unsigned*>(ds + c + 8 * kWPad) = z.y;
+        }
+        if (kind == 2) {
+            const uint4 x = in ? a.x[tile * 32 + lane] : make_uint4(0u, 0u, 0u, 0u);
+            const int c = (w * 16 + g) * 24 + 2 * t;
+            *reinterpret_cast<unsigned*>(xs + c) = x.x;
+            *reinterpret_cast<unsigned*>(xs + c + 8 * 24) = x.y;
+            *reinterpret_cast<unsigned*>(xs + c + 8) = x.z;
+            *reinterpret_cast<unsigned*>(xs + c + 8 * 24 + 8) = x.w;
+            *reinterpret_cast<unsigned*>(ys + c) = in ? a.dy[(tile * 32 + lane) * 2] : 0u;
+            *reinterpret_cast<unsigned*>(ys + c + 8 * 24) = in ? a.dy[(tile * 32 + lane) * 2 + 1] : 0u;
+            *reinterpret_cast<unsigned*>(ys + c + 8) = 0u;
+            *reinterpret_cast<unsigned*>(ys + c + 8 * 24 + 8) = 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < kWRows / 16; ++kk) {
+            unsigned A[4], b[4];
+            const int ra = kk * 16 + (lt >> 1) * 8 + lr, rb = kk * 16 + (lt & 1) * 8 + lr;
+            if (kind < 2) {
+                // rows 16 w .. of H^T, all columns of dZ
+                ldmatrix4<true>(A, hs + ra * kWPad + w * 16 + (lt & 1) * 8);
+#pragma unroll
+                for (int n = 0; n < kNT; n += 2) {
+                    ldmatrix4<true>(b, ds + rb * kWPad + n * 8 + (lt >> 1) * 8);
+                    mma16816(acc[n], A, b[0], b[1]);
+                    mma16816(acc[n + 1], A, b[2], b[3]);
+                }
+            } else {
+                // X^T dZ1: the warp's 16 columns; H3^T dY: its 16 rows
+                ldmatrix4<true>(A, xs + ra * 24 + (lt & 1) * 8);
+                ldmatrix4<true>(b, ds + rb * kWPad + w * 16 + (lt >> 1) * 8);
+                mma16816(acc[0], A, b[0], b[1]);
+                mma16816(acc[1], A, b[2], b[3]);
+                ldmatrix4<true>(A, hs + ra * kWPad + w * 16 + (lt & 1) * 8);
+                ldmatrix4<true>(b, ys + rb * 24 + (lt >> 1) * 8);
+                mma16816(acc[2], A, b[0], b[1]);
+            }
+        }
     }
-    if (threadIdx.x == 0) out[c] = sh[0];
+    float* const part = a.part + (size_t)blockIdx.x * kParts;
+    auto put = [&](float* o, int ld, int r, int c, const float (&v)[4]) {
+        *reinterpret_cast<float2*>(o + (size_t)r * ld + c) = make_float2(v[0], v[1]);
+        *reinterpret_cast<float2*>(o + (size_t)(r + 8) * ld + c) = make_float2(v[2], v[3]);
+    };
+    if (kind < 2) {
+#pragma unroll
+        for (int n = 0; n < kNT; ++n) put(part + (kind == 0 ? kPart1 : kPart2), kMlpHidden, w * 16 + g, n * 8 + 2 * t, acc[n]);
+    } else {
+        put(part, kMlpHidden, g, w * 16 + 2 * t, acc[0]);
+        put(part, kMlpHidden, g, w * 16 + 8 + 2 * t, acc[1]);
+        put(part + kPart3, kMlpOutPad, w * 16 + g, 2 * t, acc[2]);
+    }
 }
 
-__global__ void k_colsum_bf16(const __nv_bfloat16* __restrict__ x, long long rows, int cols, float* __restrict__ out) {
-    const int c = blockIdx.x;
-    float acc = 0.f;
-    for (long long r = threadIdx.x; r < rows; r += blockDim.x) acc += __bfloat162float(x[r * cols + c]);
-    __shared__ float sh[256];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
+// the gradients from the chunks' and the blocks' parts, in a fixed order, and
+// the loss
+struct GradOut {
+    float* gw[kMlpLayers];
+    float* gb[kMlpLayers];
+};
+__global__ void __launch_bounds__(128) k_mlp_reduce(const float* __restrict__ part, int chunks,
+                                                    const float* __restrict__ bias_part,
+                                                    const double* __restrict__ loss_part, int blocks, long long rows,
+                                                    GradOut o, float* __restrict__ loss) {
+    static_assert(kParts % 128 == 0, "whole blocks of weights, then a warp per bias");
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i < kParts) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < chunks; ++c) s += part[(size_t)c * kParts + i];
+        const int l = i < kPart1 ? 0 : i < kPart2 ? 1 : i < kPart3 ? 2 : 3;
+        o.gw[l][i - (l == 0 ? 0 : l == 1 ? kPart1 : l == 2 ? kPart2 : kPart3)] = s;
+        return;
     }
-    if (threadIdx.x == 0) out[c] = sh[0];
+    const int k = (i - kParts) >> 5, lane = threadIdx.x & 31;
+    if (k < kBias) {
+        float s = 0.f;
+        for (int b = lane; b < blocks; b += 32) s += bias_part[(size_t)b * kBias + k];
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+        if (lane == 0) o.gb[k / kMlpHidden][k % kMlpHidden] = s;
+    } else if (k == kBias) {
+        double s = 0.0;
+        for (int b = lane; b < blocks; b += 32) s += loss_part[b];
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+        if (lane == 0) *loss = (float)(s / (double)rows);
+    }
 }
 
 __global__ void k_to_bf16(const float* __restrict__ x, long long n, __nv_bfloat16* __restrict__ y) {
@@ -395,23 +609,37 @@ __global__ void k_adam(float* __restrict__ p, float* __restrict__ m, float* __re
     p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-__global__ void k_take3(const float* __restrict__ y, long long rows, float* __restrict__ out) {
-    long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    for (int d = 0; d < 3; ++d) out[r * 3 + d] = y[r * kMlpOutPad + d];
+// --------------------------------------------------------------- host side --
+// blocks of a k_mlp_rows launch over `rows` rows (its shared memory opted into
+// per device)
+template <bool TRAIN>
+static int row_blocks(long long rows, int* blocks) {
+    static int bps_of[64] = {0};
+    int dev = 0;
+    DWG_CHECK_CUDA(cudaGetDevice(&dev));
+    DWG_REQUIRE(dev >= 0 && dev < 64, "mlp: device %d out of range", dev);
+    if (!bps_of[dev]) {
+        DWG_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_rows<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem));
+        DWG_CHECK_CUDA(cudaFuncSetAttribute(k_mlp_weights, cudaFuncAttributeMaxDynamicSharedMemorySize, kWSmem));
+        int bps = 0;
+        DWG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_mlp_rows<TRAIN>, kRowWarps * 32, kRowSmem));
+        bps_of[dev] = bps > 0 ? bps : 1;
+    }
+    const long long tiles = (rows + 15) / 16;
+    *blocks = (int)std::min<long long>((tiles + kRowWarps - 1) / kRowWarps, (long long)num_sms() * bps_of[dev]);
+    return DWG_OK;
 }
 
-// --------------------------------------------------------------- host side --
 static int ensure_cap(Mlp& m, long long B) {
     if (B <= m.cap) return DWG_OK;
-    DWG_TRY(m.x.reserve((size_t)B * kMlpInPad));
-    for (int l = 0; l < kMlpLayers; ++l) {
-        DWG_TRY(m.z[l].reserve((size_t)B * m.dout[l]));
-        DWG_TRY(m.h[l].reserve((size_t)B * m.dout[l]));
+    const size_t rows = (size_t)(B + 15) / 16 * 16;
+    DWG_TRY(m.x.reserve(rows * kMlpInPad));
+    for (int l = 0; l < 3; ++l) {
+        DWG_TRY(m.gp[l].reserve(rows * kMlpHidden));
+        DWG_TRY(m.h[l].reserve(rows * kMlpHidden));
+        DWG_TRY(m.dz[l].reserve(rows * kMlpHidden));
     }
-    DWG_TRY(m.dz.reserve((size_t)B * kMlpHidden));
-    DWG_TRY(m.dzb.reserve((size_t)B * kMlpHidden));
-    DWG_TRY(m.dhb.reserve((size_t)B * kMlpHidden));
+    DWG_TRY(m.dy.reserve(rows * kMlpOutPad));
     m.cap = B;
     return DWG_OK;
 }
@@ -439,8 +667,6 @@ int mlp_init(Mlp& m, unsigned long long seed, cudaStream_t s) {
         DWG_TRY(m.w[l].reserve(w.size()));
         DWG_TRY(m.b[l].reserve(b.size()));
         DWG_TRY(m.wb[l].reserve(w.size()));
-        DWG_TRY(m.gw[l].reserve(w.size()));
-        DWG_TRY(m.gb[l].reserve(b.size()));
         for (auto* buf : {&m.mw[l], &m.vw[l]}) {
             DWG_TRY(buf->reserve(w.size()));
             DWG_CHECK_CUDA(cudaMemsetAsync(buf->ptr, 0, sizeof(float) * w.size(), s));
@@ -453,6 +679,14 @@ int mlp_init(Mlp& m, unsigned long long seed, cudaStream_t s) {
         DWG_CHECK_CUDA(cudaMemcpyAsync(m.b[l].ptr, b.data(), sizeof(float) * b.size(), cudaMemcpyHostToDevice, s));
     }
     DWG_TRY(m.loss.reserve(1));
+    DWG_TRY(m.grad.reserve((size_t)mlp_param_count()));
+    float* g = m.grad.ptr;  // the gradients in the flat order
+    for (int l = 0; l < kMlpLayers; ++l) {
+        m.gw[l] = g;
+        g += (size_t)m.din[l] * m.dout[l];
+        m.gb[l] = g;
+        g += m.dout[l];
+    }
     m.step = 0;
     DWG_TRY(refresh_bf16(m, s));
     DWG_CHECK_CUDA(cudaStreamSynchronize(s));
@@ -481,87 +715,89 @@ int mlp_set_flat(Mlp& m, const float* params_host, cudaStream_t s) {
     return DWG_OK;
 }
 
-static int copy_flat(const DevBuf<float>* w, const DevBuf<float>* b, const Mlp& m, float* dst, cudaStream_t s) {
-    DWG_REQUIRE(dst, "mlp: null output");
+int mlp_get_flat(Mlp& m, float* params_host, cudaStream_t s) {
+    DWG_REQUIRE(params_host, "mlp: null output");
     DWG_CHECK_CUDA(cudaStreamSynchronize(s));
+    float* dst = params_host;
     for (int l = 0; l < kMlpLayers; ++l) {
         const size_t nw = (size_t)m.din[l] * m.dout[l];
-        DWG_CHECK_CUDA(cudaMemcpy(dst, w[l].ptr, sizeof(float) * nw, cudaMemcpyDeviceToHost));
+        DWG_CHECK_CUDA(cudaMemcpy(dst, m.w[l].ptr, sizeof(float) * nw, cudaMemcpyDeviceToHost));
         dst += nw;
-        DWG_CHECK_CUDA(cudaMemcpy(dst, b[l].ptr, sizeof(float) * m.dout[l], cudaMemcpyDeviceToHost));
+        DWG_CHECK_CUDA(cudaMemcpy(dst, m.b[l].ptr, sizeof(float) * m.dout[l], cudaMemcpyDeviceToHost));
         dst += m.dout[l];
     }
     return DWG_OK;
 }
 
-int mlp_get_flat(Mlp& m, float* params_host, cudaStream_t s) { return copy_flat(m.w, m.b, m, params_host, s); }
-int mlp_get_grads_flat(Mlp& m, float* grads_host, cudaStream_t s) { return copy_flat(m.gw, m.gb, m, grads_host, s); }
-
-// forward of rows [0, B) of the packed input m.x; leaves z[3] = outputs
-static int forward_packed(Mlp& m, long long B, cudaStream_t s) {
-    const __nv_bfloat16* in = m.x.ptr;
-    int ld = kMlpInPad;
-    for (int l = 0; l < kMlpLayers; ++l) {
-        DWG_TRY(gemm<false, false>(in, ld, m.wb[l].ptr, m.dout[l], m.z[l].ptr, m.dout[l], (int)B, m.dout[l], m.din[l],
-                                   false, s));
-        const long long nz = B * m.dout[l];
-        k_bias_act<<<div_up(nz, 256), 256, 0, s>>>(m.z[l].ptr, m.b[l].ptr, m.h[l].ptr, B, m.dout[l],
-                                                   l < kMlpLayers - 1 ? 1 : 0);
-        DWG_CHECK_LAUNCH();
-        in = m.h[l].ptr;
-        ld = m.dout[l];
-    }
+int mlp_get_grads_flat(Mlp& m, float* grads_host, cudaStream_t s) {
+    DWG_REQUIRE(grads_host, "mlp: null output");
+    DWG_CHECK_CUDA(cudaStreamSynchronize(s));
+    DWG_CHECK_CUDA(cudaMemcpy(grads_host, m.grad.ptr, sizeof(float) * (size_t)mlp_param_count(), cudaMemcpyDeviceToHost));
     return DWG_OK;
+}
+
+static RowArgs row_args(const Mlp& m, const float* F, long long rows) {
+    RowArgs a{};
+    a.F = F;
+    a.rows = rows;
+    for (int l = 0; l < kMlpLayers; ++l) {
+        a.w[l] = m.wb[l].ptr;
+        a.b[l] = m.b[l].ptr;
+    }
+    return a;
 }
 
 int mlp_forward(Mlp& m, const float* F, long long n, float* out, cudaStream_t s) {
     DWG_REQUIRE(F && out && n >= 0, "mlp_forward: bad arguments");
-    const long long chunk = 1 << 16;
-    DWG_TRY(ensure_cap(m, n < chunk ? (n > 0 ? n : 1) : chunk));
-    for (long long r0 = 0; r0 < n; r0 += chunk) {
-        const long long B = n - r0 < chunk ? n - r0 : chunk;
-        k_pack_x<<<div_up(B * kMlpInPad, 256), 256, 0, s>>>(F + r0 * kMlpIn, B, m.x.ptr);
-        DWG_CHECK_LAUNCH();
-        DWG_TRY(forward_packed(m, B, s));
-        k_take3<<<div_up(B, 256), 256, 0, s>>>(m.z[kMlpLayers - 1].ptr, B, out + r0 * 3);
-        DWG_CHECK_LAUNCH();
-    }
+    if (n == 0) return DWG_OK;
+    RowArgs a = row_args(m, F, n);
+    a.out = out;
+    int blocks = 0;
+    DWG_TRY(row_blocks<false>(n, &blocks));
+    k_mlp_rows<false><<<blocks, kRowWarps * 32, kRowSmem, s>>>(a);
+    DWG_CHECK_LAUNCH();
     return DWG_OK;
 }
 
 int mlp_backward(Mlp& m, const float* F, const float* T, long long B, float* loss_host, cudaStream_t s) {
     DWG_REQUIRE(F && T && B >= 1 && B < (1ll << 31), "mlp_backward: bad arguments");
     DWG_TRY(ensure_cap(m, B));
-    k_pack_x<<<div_up(B * kMlpInPad, 256), 256, 0, s>>>(F, B, m.x.ptr);
-    DWG_CHECK_LAUNCH();
-    DWG_TRY(forward_packed(m, B, s));
-    DWG_CHECK_CUDA(cudaMemsetAsync(m.loss.ptr, 0, sizeof(float), s));
-    // dY in BF16 (8 columns), reusing dzb
-    k_cos_loss<<<div_up(B, 256), 256, 0, s>>>(m.z[kMlpLayers - 1].ptr, T, B, m.dzb.ptr, m.loss.ptr);
-    DWG_CHECK_LAUNCH();
-    const __nv_bfloat16* dzb = m.dzb.ptr;  // dZ of the current layer, BF16
-    for (int l = kMlpLayers - 1; l >= 0; --l) {
-        const int din = m.din[l], dout = m.dout[l];
-        const __nv_bfloat16* hin = l > 0 ? m.h[l - 1].ptr : m.x.ptr;
-        // bias gradient
-        if (l == kMlpLayers - 1)
-            k_colsum_bf16<<<dout, 256, 0, s>>>(dzb, B, dout, m.gb[l].ptr);
-        else
-            k_colsum_f32<<<dout, 256, 0, s>>>(m.dz.ptr, B, dout, m.gb[l].ptr);
-        DWG_CHECK_LAUNCH();
-        // dW = H_in^T dZ
-        DWG_TRY(gemm<true, false>(hin, din, dzb, dout, m.gw[l].ptr, dout, din, dout, (int)B, false, s, &m.split));
-        if (l == 0) break;
-        // dH_in = dZ W^T (FP32 into dz scratch), then dZ_in = dH_in * gelu'(z_in)
-        float* dh = m.dz.ptr;
-        DWG_TRY(gemm<false, true>(dzb, dout, m.wb[l].ptr, dout, dh, din, (int)B, din, dout, false, s));
-        // the BF16 dZ of the layer below must not overwrite the one being read:
-        // alternate between the two BF16 scratch buffers
-        __nv_bfloat16* next = (dzb == m.dzb.ptr) ? m.dhb.ptr : m.dzb.ptr;
-        k_gelu_back<<<div_up(B * din, 256), 256, 0, s>>>(dh, m.z[l - 1].ptr, B * din, m.dz.ptr, next);
-        DWG_CHECK_LAUNCH();
-        dzb = next;
+    int blocks = 0;
+    DWG_TRY(row_blocks<true>(B, &blocks));
+    const long long tiles = (B + 15) / 16, sets = (tiles + 7) / 8;
+    // three blocks per chunk, about two per SM
+    const int chunks = (int)std::min<long long>(sets, std::max(1, num_sms() * 2 / 3));
+    DWG_TRY(m.bias_part.reserve((size_t)blocks * kBias));
+    DWG_TRY(m.loss_part.reserve(blocks));
+    DWG_TRY(m.part.reserve((size_t)chunks * kParts));
+    RowArgs a = row_args(m, F, B);
+    a.T = T;
+    a.x = reinterpret_cast<uint4*>(m.x.ptr);
+    a.dy = reinterpret_cast<unsigned*>(m.dy.ptr);
+    a.bias_part = m.bias_part.ptr;
+    a.loss_part = m.loss_part.ptr;
+    WeightArgs wa{};
+    wa.tiles = tiles;
+    wa.x = a.x;
+    wa.dy = a.dy;
+    wa.part = m.part.ptr;
+    GradOut o;
+    for (int l = 0; l < 3; ++l) {
+        a.gp[l] = reinterpret_cast<float4*>(m.gp[l].ptr);
+        wa.h[l] = a.h[l] = reinterpret_cast<uint2*>(m.h[l].ptr);
+        wa.dz[l] = a.dz[l] = reinterpret_cast<uint2*>(m.dz[l].ptr);
     }
+    for (int l = 0; l < kMlpLayers; ++l) {
+        o.gw[l] = m.gw[l];
+        o.gb[l] = m.gb[l];
+    }
+    k_mlp_rows<true><<<blocks, kRowWarps * 32, kRowSmem, s>>>(a);
+    DWG_CHECK_LAUNCH();
+    k_mlp_weights<<<dim3(chunks, 3), kRowWarps * 32, kWSmem, s>>>(wa);
+    DWG_CHECK_LAUNCH();
+    k_mlp_reduce<<<div_up(kParts + (kBias + 1) * 32, 128), 128, 0, s>>>(m.part.ptr, chunks, m.bias_part.ptr,
+                                                                        m.loss_part.ptr, blocks, B, o, m.loss.ptr);
+    DWG_CHECK_LAUNCH();
     if (loss_host) {
         DWG_CHECK_CUDA(cudaMemcpyAsync(loss_host, m.loss.ptr, sizeof(float), cudaMemcpyDeviceToHost, s));
         DWG_CHECK_CUDA(cudaStreamSynchronize(s));
@@ -574,9 +810,9 @@ int mlp_adam(Mlp& m, float lr, float b1, float b2, float eps, cudaStream_t s) {
     const float c1 = 1.f - std::pow(b1, (float)m.step), c2 = 1.f - std::pow(b2, (float)m.step);
     for (int l = 0; l < kMlpLayers; ++l) {
         const long long nw = (long long)m.din[l] * m.dout[l];
-        k_adam<<<div_up(nw, 256), 256, 0, s>>>(m.w[l].ptr, m.mw[l].ptr, m.vw[l].ptr, m.gw[l].ptr, nw, lr, b1, b2, eps,
+        k_adam<<<div_up(nw, 256), 256, 0, s>>>(m.w[l].ptr, m.mw[l].ptr, m.vw[l].ptr, m.gw[l], nw, lr, b1, b2, eps,
                                                c1, c2);
-        k_adam<<<div_up(m.dout[l], 256), 256, 0, s>>>(m.b[l].ptr, m.mb[l].ptr, m.vb[l].ptr, m.gb[l].ptr, m.dout[l], lr,
+        k_adam<<<div_up(m.dout[l], 256), 256, 0, s>>>(m.b[l].ptr, m.mb[l].ptr, m.vb[l].ptr, m.gb[l], m.dout[l], lr,
                                                       b1, b2, eps, c1, c2);
     }
     DWG_CHECK_LAUNCH();

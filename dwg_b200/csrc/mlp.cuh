@@ -27,17 +27,17 @@ struct Mlp {
     DevBuf<float> w[kMlpLayers], b[kMlpLayers];             // FP32 master
     DevBuf<__nv_bfloat16> wb[kMlpLayers];                   // BF16 copy for the GEMMs
     DevBuf<float> mw[kMlpLayers], vw[kMlpLayers], mb[kMlpLayers], vb[kMlpLayers];  // Adam
-    DevBuf<float> gw[kMlpLayers], gb[kMlpLayers];           // gradients
+    DevBuf<float> grad;                                     // gradients in the flat order,
+    float *gw[kMlpLayers] = {}, *gb[kMlpLayers] = {};       // and the layers' places in it
     long long step = 0;
-    // activations of the last forward (batch capacity)
+    // training workspace (batch capacity), in the fragments' order: inputs,
+    // hidden activations, gelu', dZ of the hidden layers and of the outputs
     long long cap = 0;
-    DevBuf<__nv_bfloat16> x;                                // [B x 16]
-    DevBuf<float> z[kMlpLayers];                            // pre-activations
-    DevBuf<__nv_bfloat16> h[kMlpLayers];                    // post-activations (h[3] unused)
-    DevBuf<float> dz;                                       // [B x 128] scratch
-    DevBuf<__nv_bfloat16> dzb, dhb;
+    DevBuf<__nv_bfloat16> x, h[3], dz[3], dy;
+    DevBuf<float> gp[3];
+    DevBuf<float> part, bias_part;  // partial weight and bias gradients
+    DevBuf<double> loss_part;
     DevBuf<float> loss;
-    DevBuf<float> split;  // partial products of split-K weight-gradient GEMMs
 };
 
 // Flat parameter layout (host and files): for l = 0..3, W_l [din x dout]
