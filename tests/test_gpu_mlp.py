@@ -215,3 +215,41 @@ def test_learned_pipeline_with_zero_network_equals_plain(dwg_lib):
                                            C.byref(p)) == capi.DWG_ERR_INVALID
     finally:
         dwg_lib.dwg_mlp_destroy(h)
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 129, 2047, 4097])
+def test_rows_at_the_edges_of_tiles(dwg_lib, n):
+    # 16 rows per warp tile, 8 tiles per block and turn: a partial tile, a
+    # tile more than the block has warps, partial chunks of the weight sums.
+    # A value on the edge of two BF16 numbers may round either way, by 2^-8 of
+    # itself: two such flips of the largest term bound an output and, as a
+    # share of the gradient, a layer of a few rows.
+    flat = M.init_params(9)
+    h = new_mlp(dwg_lib)
+    try:
+        set_params(dwg_lib, h, flat)
+        F, T = batch(4097, 3)
+        Fd, Td = cu(F), cu(T)
+        out = torch.full((n + 1, 3), 7.0, dtype=torch.float32, device=DEV)
+        capi.check(dwg_lib.dwg_mlp_forward(h, capi.ptr(Fd), n, capi.ptr(out), None))
+        full = torch.empty((len(F), 3), dtype=torch.float32, device=DEV)
+        capi.check(dwg_lib.dwg_mlp_forward(h, capi.ptr(Fd), len(F), capi.ptr(full), None))
+        yo, (layers, acts, _) = M.forward(flat, F[:n])
+        term = np.abs(acts[-1]).max() * np.abs(layers[-1][0]).max()
+        assert np.abs(out[:n].cpu().numpy() - yo).max() <= 2 * 2.0**-8 * term
+        assert torch.equal(out[:n], full[:n]) and bool((out[n] == 7.0).all())
+        got = []
+        for _ in range(2):
+            grads = np.empty(M.param_count(), np.float32)
+            loss = C.c_float()
+            capi.check(dwg_lib.dwg_mlp_gradients(h, capi.ptr(Fd), capi.ptr(Td), n, C.byref(loss),
+                                                 grads.ctypes.data, grads.size, None))
+            got.append((loss.value, grads))
+        assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
+        lo, go = M.loss_and_grads(flat, F[:n], T[:n])
+        assert abs(got[0][0] - lo) <= 2 * 2.0**-8 * term
+        for gl, ol in zip(M.unflatten(got[0][1]), M.unflatten(go)):
+            for a, b in zip(gl, ol):
+                assert np.linalg.norm(a - b) <= 2 * 2.0**-8 * np.linalg.norm(b)
+    finally:
+        dwg_lib.dwg_mlp_destroy(h)
