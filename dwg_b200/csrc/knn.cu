@@ -14,6 +14,7 @@
 #include <cub/cub.cuh>
 
 #include <climits>
+#include <type_traits>
 #include <vector>
 
 #include "knn.cuh"
@@ -638,17 +639,20 @@ __global__ void __launch_bounds__(128) k_knn_thread(KnnArgs a) {
 // trial radius of it: cells are x-fastest, so the cells of one row (y, z)
 // within the radius hold one contiguous run of points.  The lanes list the
 // rows' runs, join them into one list and walk it a point each; the keys
-// within the radius go to shared memory, and when there are k the rank of a
-// key among them (the number below it) is its place in the answer, so
-// nothing is kept sorted.  The first radius follows the density around the
-// query's cell, ~1.35 k points; a round that finds fewer than k is followed
-// by one that reads the shell up to 1.5 times the radius, and past the widest
-// the query goes to k_knn_far, as does one with more keys than are kept (from
-// its radius).  A query with a seed within reach starts from the seed's
-// radius.  The walk's instructions bound it: ~1,780 per warp and 4 queries on
-// 100,000 points of a sphere (k = 15), 80 % of issue slots, 250,000 queries
-// in 150 us (430 us before, one warp per cell streaming the cell's ball);
-// a thread per query keeping a sorted set took 220 us, waiting on its loads.
+// within the radius go to shared memory, and when there are k a bitonic sort
+// over the query's lanes orders them.  The first radius: a query a short way
+// from one that has its k points finds k within that one's radius and the
+// way; else it follows the density around the query's cell, ~1.35 k points.
+// A round that finds fewer than k is followed by one that reads the shell up
+// to 1.5 times the radius, and past the widest the query goes to k_knn_far, as
+// does one with more keys than are kept (from its radius).  A query with a
+// seed within reach starts from the seed's radius.  Instructions bound it
+// (80 % of issue slots): 305,000 queries of a uniform sphere of 10,000 points,
+// up to a cell off it, took 2,310 per warp and 4 queries with the keys' ranks
+// counted (807 of them the ranks), 280 us with the queries' order; sorted
+// 241 us.  250,000 on 100,000 points 242 -> 221 us (430 us with one warp per
+// cell streaming the cell's ball; a thread per query keeping a sorted set
+// waited on its loads).
 constexpr int kNearThreads = 128;
 constexpr int kNearLanes = 8;  // lanes per query
 constexpr int kNearRuns = 4;   // rows a lane lists before it reads their points
@@ -656,6 +660,7 @@ constexpr int kNearKeys = 64;  // keys kept per query
 constexpr int kNearUnit = 64;  // queries a warp takes at a time, at most
 constexpr float kNearFirst = 1.35f * 11.f / 3.14159265f;  // first radius^2 in cells^2: this k / points near
 constexpr float kNearMost = 4.f;                          // at most this
+constexpr float kNearWay = 0.4f;                          // a way to a query with its points, in their radius
 // the widest radius, in cells
 constexpr float kNearWidest = 3.3f;
 
@@ -730,11 +735,48 @@ __device__ __forceinline__ void far_groups(const KnnArgs& a, const FarWait& f, i
     __syncwarp();
 }
 
+// Keys of a query over its lanes, U to a lane (place = lane U + slot).
+// key_none comes after every key.
+__device__ __forceinline__ double key_none() { return __hiloint2double(0x7ff00000, 0); }
+
+// bitonic merge of runs of N places: ascending where (place & N) is 0 or N is
+// everything, descending elsewhere
+template <int U, int N>
+__device__ __forceinline__ void merge_keys(double (&v)[U], int sub) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const bool down = N < U * kNearLanes && N >= U && ((sub * U) & N);
+#pragma unroll
+    for (int d = N / 2; d > 0; d >>= 1) {
+        if (d >= U) {
+            const bool high = (sub & (d / U)) != 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const double x = __shfl_xor_sync(FULL, v[u], d / U);
+                v[u] = (x < v[u]) != (high != down) ? x : v[u];
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (!(u & d)) {
+                    const bool swap = (v[u + d] < v[u]) != (N < U ? (u & N) != 0 : down);
+                    const double x = v[u];
+                    v[u] = swap ? v[u + d] : x;
+                    v[u + d] = swap ? x : v[u + d];
+                }
+        }
+    }
+}
+template <int U, int N = 2>
+__device__ __forceinline__ void sort_keys(double (&v)[U], int sub) {
+    merge_keys<U, N>(v, sub);
+    if constexpr (N < U * kNearLanes) sort_keys<U, 2 * N>(v, sub);
+}
+
 __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned int* __restrict__ work) {
     constexpr int G = kNearLanes, QW = 32 / G;  // lanes per query, queries per warp
     // a key's bits read as a double order like the key (d2 <= +inf: the
     // exponent stays below the NaNs'), and compare in one instruction
-    __shared__ double keys[kNearThreads / G][kNearKeys];
+    __shared__ __align__(16) double keys[kNearThreads / G][kNearKeys];
     __shared__ int2 runs[kNearThreads / G][G * kNearRuns];
     __shared__ FarWait far[kNearThreads / 32];
     if (a.gate_count && *a.gate_count <= a.gate_min) return;
@@ -758,6 +800,8 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
     const unsigned unit = (unsigned)(max((long long)QW, min((long long)kNearUnit, nq / (2 * warps))) / QW * QW);
     unsigned base = 0, end = 0;
     int nfar = 0;  // queries waiting (warp-uniform)
+    // the slot's last query and the radius of its k points
+    float lx = 0.f, ly = 0.f, lz = 0.f, lr = INFINITY;
     for (;;) {
         if (base == end || (long long)base >= nq) {
             if (nfar > 0) {
@@ -790,23 +834,45 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
         // r^2 = 1.35 k 11 / (pi N) cells^2 for N points in the block
         const int cx = cell_coord(qx, a.g.lo0, a.g.inv_h, a.g.G0), cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1),
                   cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2);
-        int near = 0;
-        if (search) {
-            const int x0 = max(cx - 1, 0), x1 = min(cx + 1, a.g.G0 - 1) + 1;
+        float hi2 = INFINITY;
+        // A query a short way from one that has its k points finds k within
+        // their radius and the way; the last four queries are asked
+        if (a.levels > 0) {
+            float r = INFINITY;
 #pragma unroll
-            for (int u = 0; u < (9 + G - 1) / G; ++u) {
-                const int i = u * G + sub, y = cy + i % 3 - 1, z = cz + i / 3 - 1;
-                if (i < 9 && y >= 0 && y < a.g.G1 && z >= 0 && z < a.g.G2) {
-                    const int* row = a.cell_start + a.g.G0 * (y + a.g.G1 * z);
-                    near += row[x1] - row[x0];
+            for (int s = 0; s < 32; s += G) {
+                const float dx = qx - __shfl_sync(FULL, lx, s), dy = qy - __shfl_sync(FULL, ly, s),
+                            dz = qz - __shfl_sync(FULL, lz, s), rs = __shfl_sync(FULL, lr, s);
+                const float way = sqrt_up(dx * dx + dy * dy + dz * dz);
+                if (way <= kNearWay * rs) r = fminf(r, rs + way);
+            }
+            hi2 = r * r;
+            bool need = search && !(hi2 <= widest * widest) && !(seed2 <= widest * widest);
+            if (__any_sync(FULL, need)) {
+                int near = 0;
+                if (need) {
+                    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, a.g.G0 - 1) + 1;
+#pragma unroll
+                    for (int u = 0; u < (9 + G - 1) / G; ++u) {
+                        const int i = u * G + sub, y = cy + i % 3 - 1, z = cz + i / 3 - 1;
+                        if (i < 9 && y >= 0 && y < a.g.G1 && z >= 0 && z < a.g.G2) {
+                            const int* row = a.cell_start + a.g.G0 * (y + a.g.G1 * z);
+                            near += row[x1] - row[x0];
+                        }
+                    }
                 }
+#pragma unroll
+                for (int o = G / 2; o > 0; o >>= 1) near += __shfl_xor_sync(FULL, near, o);
+                if (need) hi2 = fminf(__fdividef(kNearFirst * (float)k, (float)near), kNearMost) * (h * h);
             }
         }
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) near += __shfl_xor_sync(FULL, near, o);
-        // (a one-cell grid is read whole)
-        float hi2 = a.levels > 0 ? fminf(__fdividef(kNearFirst * (float)k, (float)near), kNearMost) * (h * h) : INFINITY;
         if (seed2 <= widest * widest) hi2 = seed2;
+        // (cells so wide that their squares overflow: the far search reads no
+        // rows of a square's width)
+        if (search && a.levels > 0 && !(widest * widest < INFINITY)) {
+            wait = true;
+            search = false;
+        }
         float lo2 = -1.f;  // the round reads the points with lo2 < d2 <= hi2
         while (__any_sync(FULL, search)) {
             // the rows (y, z) of cells within the radius
@@ -902,7 +968,7 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
                 search = found < k && hi2 < INFINITY;
                 if (search) {
                     lo2 = hi2;
-                    hi2 *= 2.25f;
+                    hi2 = fmaxf(hi2 * 2.25f, eps * eps);  // (a radius of 0 grows too)
                     if (hi2 > widest * widest) {
                         wait = true;
                         search = false;
@@ -916,25 +982,56 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
         }
         __syncwarp();
         if (wait) found = 0;
-        // a key's rank among the query's keys is its place in the answer
-        for (int b = 0; __any_sync(FULL, b < found); b += 4 * G) {
+        // the keys in order: 2, 4 or twice 4 to a lane
+        float kth = INFINITY;
+        const int most = __reduce_max_sync(FULL, found);
+        auto put = [&](auto& v) {
+            constexpr int U = sizeof(v) / sizeof(double);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (sub * U + u < min(found, k)) {
+                    a.out[qi * k + sub * U + u] = __double2loint(v[u]);
+                    if (sub * U + u == k - 1) kth = __int_as_float(__double2hiint(v[u]));
+                }
+        };
+        auto get = [&](auto& v, int b) {
+            constexpr int U = sizeof(v) / sizeof(double);
+#pragma unroll
+            for (int u = 0; u < U; u += 2) {
+                const double2 o = *reinterpret_cast<const double2*>(key + b + sub * U + u);
+                v[u] = b + sub * U + u < found ? o.x : key_none();
+                v[u + 1] = b + sub * U + u + 1 < found ? o.y : key_none();
+            }
+        };
+        if (most <= 2 * G) {
+            double v[2];
+            get(v, 0);
+            sort_keys<2>(v, sub);
+            put(v);
+        } else {
             double v[4];
-            int rank[4];
+            get(v, 0);
+            sort_keys<4>(v, sub);
+            if (most > 4 * G) {
+                double o[4];
+                get(o, 4 * G);
+                sort_keys<4>(o, sub);
+                // the smaller of each pair (i, 31 - i) are the smallest 32
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                v[u] = b + u * G + sub < found ? key[b + u * G + sub] : 0.0;
-                rank[u] = 0;
+                for (int u = 0; u < 4; ++u) {
+                    const double x = __shfl_xor_sync(FULL, o[3 - u], G - 1);
+                    v[u] = x < v[u] ? x : v[u];
+                }
+                merge_keys<4, 4 * G>(v, sub);
             }
-            for (int i = 0; i < found; ++i) {
-                const double o = key[i];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) rank[u] += o < v[u] ? 1 : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (b + u * G + sub < found && rank[u] < k)
-                    a.out[qi * k + rank[u]] = __double2loint(v[u]);
+            put(v);
         }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) kth = fminf(kth, __shfl_xor_sync(FULL, kth, o));
+        lx = qx;
+        ly = qy;
+        lz = qz;
+        lr = sqrt_up(kth);
         if (has && !wait)
             for (int i = found + sub; i < k; i += G) a.out[qi * k + i] = -1;
         const unsigned wm = __ballot_sync(FULL, wait && sub == 0);

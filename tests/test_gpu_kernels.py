@@ -678,3 +678,32 @@ def test_octree_nodes_and_moments_at_edges(oracle_lib, n, depth):
     CM, R, EC = ot.moments(P, N, A)
     assert np.allclose(g["cm"], CM[idx], rtol=0, atol=1e-14) and np.allclose(g["radius"], R[idx], rtol=0, atol=1e-14)
     assert np.allclose(g["ec"], EC[idx], rtol=1e-11, atol=1e-17)
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 300])
+@pytest.mark.parametrize("k", [1, 15, 16])
+def test_knn_keys_sorted_over_lanes(n, k):
+    # whole-number coordinates: distances are exact, many are equal and the
+    # smaller index comes first; 2, 4 and twice 4 keys a lane, and more keys
+    # than are kept
+    rng = np.random.default_rng(n * 20 + k)
+    P = rng.integers(-3, 4, (n, 3)).astype(np.float32)
+    Q = np.concatenate([P[rng.integers(0, n, 70)], rng.integers(-5, 6, (71, 3)).astype(np.float32)])
+    kk = min(k, n)
+    got = turbo.KnnIndex(cu(P)).query(cu(Q), kk).cpu().numpy()
+    d2 = ((Q[:, None, :].astype(np.int64) - P[None, :, :].astype(np.int64)) ** 2).sum(-1)
+    ref = np.argsort(d2 * n + np.arange(n)[None, :], axis=1, kind="stable")[:, :kk]
+    assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("scale", [3e-20, 1e-24])
+def test_knn_of_clouds_with_vanishing_squares(scale):
+    # squared distances below the normal numbers, and all of them 0: a radius
+    # of 0 has to grow, a cell whose square is 0 goes to the far search
+    rng = np.random.default_rng(4)
+    P = (rng.integers(-3, 4, (400, 3)).astype(np.float32) * np.float32(scale)).astype(np.float32)
+    got = turbo.KnnIndex(cu(P)).query(cu(P), 15).cpu().numpy()
+    d = P[:, None, :] - P[None, :, :]
+    q = d * d
+    d2 = ((q[..., 0] + q[..., 1]) + q[..., 2]).astype(np.float32)
+    assert np.array_equal(got, np.argsort(d2, axis=1, kind="stable")[:, :15])
