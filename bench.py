@@ -585,10 +585,10 @@ def knn_roofline(a, lib, capi, turbo, torch, dev, P, peaks):
     t = float(np.median(times)) * 1e-3
     nbytes = 12.0 * n + 12.0 * T + 4.0 * k * T
     hbm = float(peaks.get("hbm_gbs", 6650.0))
-    return {"kernel": "dwg_knn_query (k_cq_key/k_cq_scatter + k_knn_cells, k_knn_thread for overflow): "
+    return {"kernel": "dwg_knn_query (k_knn_qkey/k_knn_qscatter, k_knn_near, k_knn_far for what lies further): "
                       f"15 nearest of {n} leaves for the {T} triangle centroids of iteration 0",
             "bound": "hbm", "achieved": nbytes / t / 1e9, "peak": hbm, "unit": "GB/s",
-            "frac": nbytes / t / 1e9 / hbm, "traffic": _traffic("knn_cells", a.workload),
+            "frac": nbytes / t / 1e9 / hbm, "traffic": _traffic("knn_near", a.workload),
             "peak_source": "of measured: hbm_gbs of MEASURED_PEAKS.json" if "hbm_gbs" in peaks else "of fallback 6650",
             "launch_ms": t * 1e3, "algorithmic_bytes": nbytes, "queries": int(T), "points": int(n), "k": k,
             "algorithmic": "12 B per point + 12 B per query + 4 k B per query (ids written)",

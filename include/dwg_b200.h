@@ -171,8 +171,8 @@ int dwg_gwn_grid(dwg_octree* tree, const float* normals_dev, const float* areas_
  * derivative of each term with respect to the query -- of the point terms
  * and of the far nodes' order-0 dipoles, with the opening decisions of
  * dwg_gwn_points -- and out_dev (nullable) the values.  FP32 terms summed in
- * FP64, one thread per query (slower than dwg_gwn_points, which the DWG loop
- * uses); params->order must be 0; lists, tile and precision are ignored. */
+ * FP64, in the warp walk of dwg_gwn_points; params->order must be 0; lists,
+ * tile and precision are ignored. */
 int dwg_gwn_points_grad(dwg_octree* tree, const float* normals_dev, const float* areas_dev,
                         const float* radii_dev, const float* queries_dev, long long num_queries,
                         const dwg_gwn_params* params, float* out_dev, float* grad_dev, void* stream);
