@@ -707,3 +707,27 @@ def test_knn_of_clouds_with_vanishing_squares(scale):
     q = d * d
     d2 = ((q[..., 0] + q[..., 1]) + q[..., 2]).astype(np.float32)
     assert np.array_equal(got, np.argsort(d2, axis=1, kind="stable")[:, :15])
+
+
+@pytest.mark.parametrize("n,depth", [(1, 3), (300, 21), (3000, 4), (20000, 8)])
+def test_fwn_coefficients_at_edges(oracle_lib, n, depth):
+    # one node, chains of one child, leaves of many points, levels on both
+    # sides of those that share a launch; tolerance as for the torus
+    rng = np.random.default_rng(n)
+    P = rng.uniform(-0.5, 0.5, (n, 3)).astype(np.float32)
+    P[: n // 10] = P[0]
+    N = rng.normal(size=(n, 3)).astype(np.float32)
+    N /= np.linalg.norm(N, axis=1, keepdims=True)
+    A = rng.uniform(1e-6, 2e-6, n).astype(np.float32)
+    gt, ot = turbo.TurboLibiGWN(cu(P), max_depth=depth, areas=cu(A)), oracle_lib.Octree(P, depth)
+    gt.UpdateMassNormals(cu(N), cu(A))
+    g = gt.export()
+    idx = match_nodes(g, ot)
+    # about the same centres: coefficients of coincident points are those of
+    # the centre's rounding
+    CM = np.zeros((ot.num_nodes, 3))
+    CM[idx] = g["cm"]
+    ref, got = ot.expansion(P, N, A, CM)[idx], gt.expansion()
+    mass = g["pt_count"][:, None] * 2e-6
+    assert np.all(np.abs(got[:, :9] - ref[:, :9]) <= 1e-11 * mass * g["radius"][:, None] + 1e-30)
+    assert np.all(np.abs(got[:, 9:] - ref[:, 9:]) <= 1e-11 * mass * g["radius"][:, None] ** 2 + 1e-30)
