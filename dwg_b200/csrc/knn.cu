@@ -1126,7 +1126,8 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
                 hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
             }
         const float mx = 0.5f * (lo[0] + hi[0]), my = 0.5f * (lo[1] + hi[1]), mz = 0.5f * (lo[2] + hi[2]);
-        if (lane == 0) stack[w][0] = far_entry(0, 0, 0, a.levels, a.occ[a.loff[a.levels]]);
+        // (a grid of one cell has no pyramid: the cell is the root)
+        if (lane == 0) stack[w][0] = far_entry(0, 0, 0, a.levels, a.levels > 0 ? a.occ[a.loff[a.levels]] : 0);
         int sp = 1;
         float kd2 = U2 * 1.00001f;  // the lane's bound, and the widest of the group
         float wide = warp_max(has ? kd2 : 0.f);

@@ -731,3 +731,15 @@ def test_fwn_coefficients_at_edges(oracle_lib, n, depth):
     mass = g["pt_count"][:, None] * 2e-6
     assert np.all(np.abs(got[:, :9] - ref[:, :9]) <= 1e-11 * mass * g["radius"][:, None] + 1e-30)
     assert np.all(np.abs(got[:, 9:] - ref[:, 9:]) <= 1e-11 * mass * g["radius"][:, None] ** 2 + 1e-30)
+
+
+@pytest.mark.parametrize("n", [14, 64, 65, 1000])
+@pytest.mark.parametrize("k", [1, 10, 16])
+def test_knn_of_one_cell(n, k):
+    # points at one spot: a grid of one cell without a pyramid, with more
+    # points than the near round keeps
+    P = np.tile(np.array([[0.25, -0.5, 0.125]], np.float32), (n, 1))
+    Q = np.array([[0.25, -0.5, 0.125], [0.0, 0.0, 0.0], [9.0, 9.0, 9.0]], np.float32)
+    kk = min(k, n)
+    got = turbo.KnnIndex(cu(P)).query(cu(Q), kk).cpu().numpy()
+    assert np.array_equal(got, np.tile(np.arange(kk, dtype=got.dtype), (3, 1)))
