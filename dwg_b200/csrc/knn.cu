@@ -29,14 +29,32 @@ struct Gate {
     __device__ __forceinline__ bool closed() const { return count && *count <= min; }
 };
 
+// The searches compare a query with cells and nodes in coordinates relative
+// to the grid's corner lo: a point's cell is that of fl(p - lo), so the
+// rounding of every step is a part of the grid's extent, however far from the
+// origin the cloud lies (faces at lo + i h would be rounded at |lo|, which
+// moves them by cells).  In units of 2^-24 extents, a point's cell carries at
+// most 3 (the difference, 1 / h, the product), a face i h - eps 2 and a
+// query's difference 1, and the extent is at most max(G) cells: eps widens
+// boxes and reaches by 8 of them, and 1e-4 cells.
 struct KnnGrid {
     int G0, G1, G2;
-    float lo0, lo1, lo2, h, inv_h;
+    float lo0, lo1, lo2, h, inv_h, eps;
 };
 
-__device__ __forceinline__ int cell_coord(float p, float lo, float inv_h, int G) {
-    int c = (int)floorf(__fmul_rn(__fsub_rn(p, lo), inv_h));
+static KnnGrid grid_of(const KnnIndex& ix) {
+    const int most = max(ix.G[0], max(ix.G[1], ix.G[2]));
+    const float eps = (1e-4f + (float)most * (1.f / 2097152.f)) * ix.h + 1e-6f;  // (8 * 2^-24 = 2^-21)
+    return KnnGrid{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h, eps};
+}
+
+// the cell of a relative coordinate, and of a point's
+__device__ __forceinline__ int cell_at(float u, float inv_h, int G) {
+    const int c = (int)floorf(__fmul_rn(u, inv_h));
     return c < 0 ? 0 : (c >= G ? G - 1 : c);
+}
+__device__ __forceinline__ int cell_coord(float p, float lo, float inv_h, int G) {
+    return cell_at(__fsub_rn(p, lo), inv_h, G);
 }
 
 __global__ void k_knn_hist(const float* __restrict__ P, int n, KnnGrid g, int* __restrict__ counts,
@@ -196,7 +214,7 @@ int knn_build(KnnIndex& ix, const float* P, int n, cudaStream_t s) {
     ix.inv_h = 1.0f / h;
     for (int d = 0; d < 3; ++d) ix.lo[d] = bb[d];
     long long ncell = (long long)ix.G[0] * ix.G[1] * ix.G[2];
-    KnnGrid g{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h};
+    const KnnGrid g = grid_of(ix);
     DevBuf<int> counts, cell_of;
     DWG_TRY(counts.reserve(ncell + 1));
     DWG_TRY(cell_of.reserve(n));
@@ -477,7 +495,8 @@ __device__ __forceinline__ void knn_pyramid(const KnnArgs& a, float qx, float qy
                                             TopK<KMAX>& top) {
     const unsigned long long NONE = ~0ull;
     const float h = a.g.h;
-    const float eps = 1e-4f * h + 1e-6f;
+    const float eps = a.g.eps;
+    const float ux = __fsub_rn(qx, a.g.lo0), uy = __fsub_rn(qy, a.g.lo1), uz = __fsub_rn(qz, a.g.lo2);
     const int top_l = a.levels;
     int lvl = top_l, ci = 0, cj = 0, ck = 0;
     unsigned long long ctr = 0;
@@ -503,22 +522,22 @@ __device__ __forceinline__ void knn_pyramid(const KnnArgs& a, float qx, float qy
         ctr += 1ull << sh;
         // octant of the query about the node's midpoint
         const int half = 1 << (lvl - 1);
-        const float mx = a.g.lo0 + (float)((ci << lvl) + half) * h;
-        const float my = a.g.lo1 + (float)((cj << lvl) + half) * h;
-        const float mz = a.g.lo2 + (float)((ck << lvl) + half) * h;
-        const int qo = (qx >= mx ? 1 : 0) | (qy >= my ? 2 : 0) | (qz >= mz ? 4 : 0);
+        const float mx = (float)((ci << lvl) + half) * h;
+        const float my = (float)((cj << lvl) + half) * h;
+        const float mz = (float)((ck << lvl) + half) * h;
+        const int qo = (ux >= mx ? 1 : 0) | (uy >= my ? 2 : 0) | (uz >= mz ? 4 : 0);
         const int oc = qo ^ (int)((0x76534210u >> (4 * c)) & 7u);
         // empty or outside the grid (such children have no bit)
         if (!(((lvl < 8 ? mk0 : mk1) >> (8 * (lvl & 7) + oc)) & 1ull)) continue;
         const int nl = lvl - 1;
         const int ni = (ci << 1) | (oc & 1), nj = (cj << 1) | ((oc >> 1) & 1), nk = (ck << 1) | (oc >> 2);
         const float kd2 = top.mx == NONE ? INFINITY : __uint_as_float((unsigned)(top.mx >> 32)) * 1.00001f;
-        const float x0 = a.g.lo0 + (float)(ni << nl) * h - eps, x1 = a.g.lo0 + (float)((ni + 1) << nl) * h + eps;
-        const float y0 = a.g.lo1 + (float)(nj << nl) * h - eps, y1 = a.g.lo1 + (float)((nj + 1) << nl) * h + eps;
-        const float z0 = a.g.lo2 + (float)(nk << nl) * h - eps, z1 = a.g.lo2 + (float)((nk + 1) << nl) * h + eps;
-        const float ddx = fmaxf(0.f, fmaxf(x0 - qx, qx - x1));
-        const float ddy = fmaxf(0.f, fmaxf(y0 - qy, qy - y1));
-        const float ddz = fmaxf(0.f, fmaxf(z0 - qz, qz - z1));
+        const float x0 = (float)(ni << nl) * h - eps, x1 = (float)((ni + 1) << nl) * h + eps;
+        const float y0 = (float)(nj << nl) * h - eps, y1 = (float)((nj + 1) << nl) * h + eps;
+        const float z0 = (float)(nk << nl) * h - eps, z1 = (float)((nk + 1) << nl) * h + eps;
+        const float ddx = fmaxf(0.f, fmaxf(x0 - ux, ux - x1));
+        const float ddy = fmaxf(0.f, fmaxf(y0 - uy, uy - y1));
+        const float ddz = fmaxf(0.f, fmaxf(z0 - uz, uz - z1));
         if (ddx * ddx + ddy * ddy + ddz * ddz > kd2) continue;
         if (nl == 0) {
             if (abs(ni - cx) <= 1 && abs(nj - cy) <= 1 && abs(nk - cz) <= 1) continue;  // scanned already
@@ -559,15 +578,16 @@ __global__ void __launch_bounds__(128) k_knn_thread(KnnArgs a) {
     const unsigned long long NONE = ~0ull;
     const int k = a.k;
     const float h = a.g.h;
-    const float eps = 1e-4f * h + 1e-6f;
+    const float eps = a.g.eps;
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nq;
          j += (long long)gridDim.x * blockDim.x) {
         const long long qi = a.order ? a.order[j] : j;
         float qx, qy, qz;
         knn_load_query(a, qi, qx, qy, qz);
-        const int cx = cell_coord(qx, a.g.lo0, a.g.inv_h, a.g.G0);
-        const int cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1);
-        const int cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2);
+        const float ux = __fsub_rn(qx, a.g.lo0), uy = __fsub_rn(qy, a.g.lo1), uz = __fsub_rn(qz, a.g.lo2);
+        const int cx = cell_at(ux, a.g.inv_h, a.g.G0);
+        const int cy = cell_at(uy, a.g.inv_h, a.g.G1);
+        const int cz = cell_at(uz, a.g.inv_h, a.g.G2);
         TopK<KMAX> top;
         top.init(k);
         for (int r = 0;; ++r) {
@@ -575,13 +595,13 @@ __global__ void __launch_bounds__(128) k_knn_thread(KnnArgs a) {
             for (int dz = -r; dz <= r; ++dz) {
                 const int z = cz + dz;
                 if (z < 0 || z >= a.g.G2) continue;
-                const float z0 = a.g.lo2 + (float)z * h - eps, z1 = z0 + h + 2.f * eps;
-                const float ddz = fmaxf(0.f, fmaxf(z0 - qz, qz - z1));
+                const float z0 = (float)z * h - eps, z1 = z0 + h + 2.f * eps;
+                const float ddz = fmaxf(0.f, fmaxf(z0 - uz, uz - z1));
                 for (int dy = -r; dy <= r; ++dy) {
                     const int y = cy + dy;
                     if (y < 0 || y >= a.g.G1) continue;
-                    const float y0 = a.g.lo1 + (float)y * h - eps, y1 = y0 + h + 2.f * eps;
-                    const float ddy = fmaxf(0.f, fmaxf(y0 - qy, qy - y1));
+                    const float y0 = (float)y * h - eps, y1 = y0 + h + 2.f * eps;
+                    const float ddy = fmaxf(0.f, fmaxf(y0 - uy, uy - y1));
                     const float dyz = ddy * ddy + ddz * ddz;
                     if (dyz > kd2) continue;
                     const bool face = (dz == -r || dz == r || dy == -r || dy == r);
@@ -589,8 +609,8 @@ __global__ void __launch_bounds__(128) k_knn_thread(KnnArgs a) {
                     for (int dx = -r; dx <= r; dx += step) {
                         const int x = cx + dx;
                         if (x < 0 || x >= a.g.G0) continue;
-                        const float x0 = a.g.lo0 + (float)x * h - eps, x1 = x0 + h + 2.f * eps;
-                        const float ddx = fmaxf(0.f, fmaxf(x0 - qx, qx - x1));
+                        const float x0 = (float)x * h - eps, x1 = x0 + h + 2.f * eps;
+                        const float ddx = fmaxf(0.f, fmaxf(x0 - ux, ux - x1));
                         if (ddx * ddx + dyz > kd2) continue;
                         const int c = x + a.g.G0 * (y + a.g.G1 * z);
                         const int e = a.cell_start[c + 1];
@@ -610,12 +630,12 @@ __global__ void __launch_bounds__(128) k_knn_thread(KnnArgs a) {
                 break;
             if (top.mx != NONE) {
                 float bd = INFINITY;
-                if (cx - r > 0) bd = fminf(bd, qx - (a.g.lo0 + (float)(cx - r) * h));
-                if (cx + r < a.g.G0 - 1) bd = fminf(bd, (a.g.lo0 + (float)(cx + r + 1) * h) - qx);
-                if (cy - r > 0) bd = fminf(bd, qy - (a.g.lo1 + (float)(cy - r) * h));
-                if (cy + r < a.g.G1 - 1) bd = fminf(bd, (a.g.lo1 + (float)(cy + r + 1) * h) - qy);
-                if (cz - r > 0) bd = fminf(bd, qz - (a.g.lo2 + (float)(cz - r) * h));
-                if (cz + r < a.g.G2 - 1) bd = fminf(bd, (a.g.lo2 + (float)(cz + r + 1) * h) - qz);
+                if (cx - r > 0) bd = fminf(bd, ux - (float)(cx - r) * h);
+                if (cx + r < a.g.G0 - 1) bd = fminf(bd, (float)(cx + r + 1) * h - ux);
+                if (cy - r > 0) bd = fminf(bd, uy - (float)(cy - r) * h);
+                if (cy + r < a.g.G1 - 1) bd = fminf(bd, (float)(cy + r + 1) * h - uy);
+                if (cz - r > 0) bd = fminf(bd, uz - (float)(cz - r) * h);
+                if (cz + r < a.g.G2 - 1) bd = fminf(bd, (float)(cz + r + 1) * h - uz);
                 bd -= eps;
                 if (bd > 0.f && __uint_as_float((unsigned)(top.mx >> 32)) < bd * bd * 0.9999f) break;
             }
@@ -791,7 +811,7 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
     const unsigned long long NONE = ~0ull;
     const int k = a.k;
     const float h = a.g.h;
-    const float eps = 1e-4f * h + 1e-6f;
+    const float eps = a.g.eps;
     const float widest = kNearWidest * h;
     // a warp takes a run of consecutive queries at a time, short when the
     // launch would leave warps idle; the far ones among them form the groups
@@ -832,8 +852,9 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
         // The first radius: a surface through the 3x3x3 block around the
         // query's cell covers ~11 faces of cells, so 1.35 k points lie within
         // r^2 = 1.35 k 11 / (pi N) cells^2 for N points in the block
-        const int cx = cell_coord(qx, a.g.lo0, a.g.inv_h, a.g.G0), cy = cell_coord(qy, a.g.lo1, a.g.inv_h, a.g.G1),
-                  cz = cell_coord(qz, a.g.lo2, a.g.inv_h, a.g.G2);
+        const float ux = __fsub_rn(qx, a.g.lo0), uy = __fsub_rn(qy, a.g.lo1), uz = __fsub_rn(qz, a.g.lo2);
+        const int cx = cell_at(ux, a.g.inv_h, a.g.G0), cy = cell_at(uy, a.g.inv_h, a.g.G1),
+                  cz = cell_at(uz, a.g.inv_h, a.g.G2);
         float hi2 = INFINITY;
         // A query a short way from one that has its k points finds k within
         // their radius and the way; the last four queries are asked
@@ -877,13 +898,13 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
         while (__any_sync(FULL, search)) {
             // the rows (y, z) of cells within the radius
             const float out2 = hi2 * 1.00001f, reach = sqrt_up(hi2) + eps;
-            const int y0 = cell_coord(qy - reach, a.g.lo1, a.g.inv_h, a.g.G1);
-            const int ny = cell_coord(qy + reach, a.g.lo1, a.g.inv_h, a.g.G1) - y0 + 1;
-            const int z0 = cell_coord(qz - reach, a.g.lo2, a.g.inv_h, a.g.G2);
-            const int nrow = search ? ny * (cell_coord(qz + reach, a.g.lo2, a.g.inv_h, a.g.G2) - z0 + 1) : 0;
+            const int y0 = cell_at(uy - reach, a.g.inv_h, a.g.G1);
+            const int ny = cell_at(uy + reach, a.g.inv_h, a.g.G1) - y0 + 1;
+            const int z0 = cell_at(uz - reach, a.g.inv_h, a.g.G2);
+            const int nrow = search ? ny * (cell_at(uz + reach, a.g.inv_h, a.g.G2) - z0 + 1) : 0;
             // row i is (i % ny, i / ny), i / ny = i * inv >> 16 (i < 2^8)
             const unsigned inv = (unsigned)__fdividef(65536.f, (float)ny) + 1u;
-            const float by = a.g.lo1 + (float)y0 * h - eps - qy, bz = a.g.lo2 + (float)z0 * h - eps - qz;
+            const float by = (float)y0 * h - eps - uy, bz = (float)z0 * h - eps - uz;
             const float wide = h + 2.f * eps;
             for (int rb = 0; __any_sync(FULL, rb < nrow); rb += G * kNearRuns) {
                 // the lane's runs of this batch of rows
@@ -902,8 +923,8 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
                         if (rest >= 0.f) {
                             const float hx = sqrt_up(rest) + eps;
                             const int* row = a.cell_start + a.g.G0 * (y0 + iy + a.g.G1 * (z0 + iz));
-                            s[u] = row[cell_coord(qx - hx, a.g.lo0, a.g.inv_h, a.g.G0)];
-                            e[u] = row[cell_coord(qx + hx, a.g.lo0, a.g.inv_h, a.g.G0) + 1];
+                            s[u] = row[cell_at(ux - hx, a.g.inv_h, a.g.G0)];
+                            e[u] = row[cell_at(ux + hx, a.g.inv_h, a.g.G0) + 1];
                         }
                     }
                 }
@@ -1098,7 +1119,7 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
     const unsigned ng = a.far_count[1];
     const int k = a.k;
     const float h = a.g.h;
-    const float eps = 1e-4f * h + 1e-6f;
+    const float eps = a.g.eps;
     for (;;) {
         unsigned g = 0;
         if (lane == 0) g = atomicAdd(work, 1u);
@@ -1116,7 +1137,8 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
         // (a lane without a query takes no key)
         top.init(k, !has ? 0ull
                          : U2 < INFINITY ? ((unsigned long long)__float_as_uint(U2) << 32) | 0xffffffffull : NONE);
-        // the group's box and its centre
+        const float ux = __fsub_rn(qx, a.g.lo0), uy = __fsub_rn(qy, a.g.lo1), uz = __fsub_rn(qz, a.g.lo2);
+        // the group's box, relative to the grid's too (rl, rh), and its centre
         float lo[3] = {qx, qy, qz}, hi[3] = {qx, qy, qz};
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -1125,7 +1147,9 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
                 lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
                 hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
             }
-        const float mx = 0.5f * (lo[0] + hi[0]), my = 0.5f * (lo[1] + hi[1]), mz = 0.5f * (lo[2] + hi[2]);
+        const float rl[3] = {lo[0] - a.g.lo0, lo[1] - a.g.lo1, lo[2] - a.g.lo2};
+        const float rh[3] = {hi[0] - a.g.lo0, hi[1] - a.g.lo1, hi[2] - a.g.lo2};
+        const float mx = 0.5f * (rl[0] + rh[0]), my = 0.5f * (rl[1] + rh[1]), mz = 0.5f * (rl[2] + rh[2]);
         // (a grid of one cell has no pyramid: the cell is the root)
         if (lane == 0) stack[w][0] = far_entry(0, 0, 0, a.levels, a.levels > 0 ? a.occ[a.loff[a.levels]] : 0);
         int sp = 1;
@@ -1137,12 +1161,12 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
             const int lvl = en.y & 0xff;
             const int ci = en.x & 1023, cj = (en.x >> 10) & 1023, ck = en.x >> 20;
             {
-                const float x0 = a.g.lo0 + (float)(ci << lvl) * h - eps, x1 = a.g.lo0 + (float)((ci + 1) << lvl) * h + eps;
-                const float y0 = a.g.lo1 + (float)(cj << lvl) * h - eps, y1 = a.g.lo1 + (float)((cj + 1) << lvl) * h + eps;
-                const float z0 = a.g.lo2 + (float)(ck << lvl) * h - eps, z1 = a.g.lo2 + (float)((ck + 1) << lvl) * h + eps;
-                const float dx = fmaxf(0.f, fmaxf(x0 - qx, qx - x1));
-                const float dy = fmaxf(0.f, fmaxf(y0 - qy, qy - y1));
-                const float dz = fmaxf(0.f, fmaxf(z0 - qz, qz - z1));
+                const float x0 = (float)(ci << lvl) * h - eps, x1 = (float)((ci + 1) << lvl) * h + eps;
+                const float y0 = (float)(cj << lvl) * h - eps, y1 = (float)((cj + 1) << lvl) * h + eps;
+                const float z0 = (float)(ck << lvl) * h - eps, z1 = (float)((ck + 1) << lvl) * h + eps;
+                const float dx = fmaxf(0.f, fmaxf(x0 - ux, ux - x1));
+                const float dy = fmaxf(0.f, fmaxf(y0 - uy, uy - y1));
+                const float dz = fmaxf(0.f, fmaxf(z0 - uz, uz - z1));
                 if (!__any_sync(FULL, has && dx * dx + dy * dy + dz * dz <= kd2)) continue;
             }
             if (lvl > kFarLeaf) {
@@ -1158,12 +1182,12 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
                     const int* D = a.ldim[lvl - 1];
                     cm = a.occ[a.loff[lvl - 1] + ni + (long long)D[0] * (nj + (long long)D[1] * nk)];
                     const float side = half * h;
-                    const float x0 = a.g.lo0 + (float)ni * side - eps, x1 = a.g.lo0 + (float)(ni + 1) * side + eps;
-                    const float y0 = a.g.lo1 + (float)nj * side - eps, y1 = a.g.lo1 + (float)(nj + 1) * side + eps;
-                    const float z0 = a.g.lo2 + (float)nk * side - eps, z1 = a.g.lo2 + (float)(nk + 1) * side + eps;
-                    const float dx = fmaxf(0.f, fmaxf(x0 - hi[0], lo[0] - x1));
-                    const float dy = fmaxf(0.f, fmaxf(y0 - hi[1], lo[1] - y1));
-                    const float dz = fmaxf(0.f, fmaxf(z0 - hi[2], lo[2] - z1));
+                    const float x0 = (float)ni * side - eps, x1 = (float)(ni + 1) * side + eps;
+                    const float y0 = (float)nj * side - eps, y1 = (float)(nj + 1) * side + eps;
+                    const float z0 = (float)nk * side - eps, z1 = (float)(nk + 1) * side + eps;
+                    const float dx = fmaxf(0.f, fmaxf(x0 - rh[0], rl[0] - x1));
+                    const float dy = fmaxf(0.f, fmaxf(y0 - rh[1], rl[1] - y1));
+                    const float dz = fmaxf(0.f, fmaxf(z0 - rh[2], rl[2] - z1));
                     push = dx * dx + dy * dy + dz * dz <= wide;
                     const float ax = 0.5f * (x0 + x1) - mx, ay = 0.5f * (y0 + y1) - my, az = 0.5f * (z0 + z1) - mz;
                     if (push) away = ax * ax + ay * ay + az * az;
@@ -1359,7 +1383,7 @@ int knn_query(const KnnIndex& ix, const KnnQuery& q, int k, int* out, cudaStream
     DWG_REQUIRE(q.q || (q.q_index && q.q_source), "knn: no queries");
     if (q.nq <= 0) return DWG_OK;
     KnnArgs a;
-    a.g = KnnGrid{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h};
+    a.g = grid_of(ix);
     a.pts = ix.pts.ptr;
     a.cell_start = ix.cell_start.ptr;
     a.q = q.q;

@@ -1,0 +1,49 @@
+"""Exact neighbours whatever the cloud's place and size: clouds far from the
+origin, against brute force over all keys on the GPU."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from dwg_b200 import turbo  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def brute(P, Q, k):
+    """The k smallest keys (bits of the squared distance, rounded operation by
+    operation in FP32, then the index) of every query."""
+    idx = torch.arange(len(P), device=P.device, dtype=torch.int64)
+    out = []
+    for q in Q.split(max(1, 200_000_000 // len(P))):
+        d = [P[None, :, c] - q[:, c, None] for c in range(3)]
+        d2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2]
+        key = (d2.contiguous().view(torch.int32).to(torch.int64) << 32) | idx[None, :]
+        out.append((key.topk(k, dim=1, largest=False, sorted=True).values & 0xffffffff).to(torch.int32))
+    return torch.cat(out)
+
+
+def torus(n, seed):
+    """About 1 wide."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    th, ph = (torch.rand(n, generator=g, device="cuda", dtype=torch.float64) * (2 * np.pi) for _ in range(2))
+    ring = 0.37 + 0.13 * ph.cos()
+    return torch.stack([ring * th.cos(), ring * th.sin(), 0.13 * ph.sin()], 1), g
+
+
+@pytest.mark.parametrize("n,offset,k", [(1000000, 5e3, 15), (1000000, 1e4, 10), (100000, 4e4, 15), (100000, 9e4, 16),
+                                        (100000, 9e4, 1), (100000, 9e4, 32), (20000, -3e5, 8)])
+def test_knn_far_from_the_origin(n, offset, k):
+    # coordinates whose rounding is a cell's thousandth up to cells: cells,
+    # faces and reaches have to be those of the points as they are stored.
+    # Queries on the points, near them, and off the surface
+    P, g = torus(n, seed=k)
+    off = torch.tensor([offset, -0.7 * offset, 0.9 * offset], device="cuda", dtype=torch.float64)
+    m = 6000
+    sel = torch.randint(n, (3 * m,), generator=g, device="cuda")
+    Q = P[sel]
+    Q[m:] += torch.randn(2 * m, 3, generator=g, device="cuda", dtype=torch.float64) * 3e-3
+    Q[2 * m:] *= torch.rand(m, 1, generator=g, device="cuda", dtype=torch.float64) * 1.5
+    P, Q = (P + off).float().contiguous(), (Q + off).float().contiguous()
+    got = turbo.KnnIndex(P).query(Q, k)
+    assert torch.equal(got, brute(P, Q, k))
