@@ -36,7 +36,8 @@ struct Gate {
 // moves them by cells).  In units of 2^-24 extents, a point's cell carries at
 // most 3 (the difference, 1 / h, the product), a face i h - eps 2 and a
 // query's difference 1, and the extent is at most max(G) cells: eps widens
-// boxes and reaches by 8 of them, and 1e-4 cells.
+// boxes and reaches by 8 of them, and 1e-4 cells: below a thousandth of a cell
+// (max(G) <= 1024) whatever the cloud's size, so a reach stays a few cells.
 struct KnnGrid {
     int G0, G1, G2;
     float lo0, lo1, lo2, h, inv_h, eps;
@@ -44,7 +45,7 @@ struct KnnGrid {
 
 static KnnGrid grid_of(const KnnIndex& ix) {
     const int most = max(ix.G[0], max(ix.G[1], ix.G[2]));
-    const float eps = (1e-4f + (float)most * (1.f / 2097152.f)) * ix.h + 1e-6f;  // (8 * 2^-24 = 2^-21)
+    const float eps = (1e-4f + (float)most * (1.f / 2097152.f)) * ix.h;  // (8 * 2^-24 = 2^-21)
     return KnnGrid{ix.G[0], ix.G[1], ix.G[2], ix.lo[0], ix.lo[1], ix.lo[2], ix.h, ix.inv_h, eps};
 }
 
@@ -198,7 +199,9 @@ int knn_build(KnnIndex& ix, const float* P, int n, cudaStream_t s) {
     double gm = ceil(sqrt((double)n / 14.0));
     if (gm < 1) gm = 1;
     if (gm > 1024) gm = 1024;
-    float h = (float)(emax / gm) * 1.0001f;
+    // (no cell below 1e-12: eps and the radii, thousandths of a cell, keep
+    // normal squares; the points of a cloud that small share a few cells)
+    float h = fmaxf((float)(emax / gm) * 1.0001f, 1e-12f);
     for (;;) {
         long long tot = 1;
         for (int d = 0; d < 3; ++d) {
@@ -683,6 +686,9 @@ constexpr float kNearMost = 4.f;                          // at most this
 constexpr float kNearWay = 0.4f;                          // a way to a query with its points, in their radius
 // the widest radius, in cells
 constexpr float kNearWidest = 3.3f;
+// a window of cells about a query is at most 15 wide then, so a row's number
+// stays below 2^8
+static_assert(kNearWidest < 6.9f, "rows of a window are numbered below 2^8");
 
 // the KMAX smallest keys, ascending (k < KMAX: the first KMAX - k slots hold
 // 0); an insertion is 2 compares and 2 selects of 64 bits per slot, without
@@ -902,7 +908,8 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
             const int ny = cell_at(uy + reach, a.g.inv_h, a.g.G1) - y0 + 1;
             const int z0 = cell_at(uz - reach, a.g.inv_h, a.g.G2);
             const int nrow = search ? ny * (cell_at(uz + reach, a.g.inv_h, a.g.G2) - z0 + 1) : 0;
-            // row i is (i % ny, i / ny), i / ny = i * inv >> 16 (i < 2^8)
+            // row i is (i % ny, i / ny), i / ny = i * inv >> 16 (exact for
+            // ny <= 15, i < 2^8)
             const unsigned inv = (unsigned)__fdividef(65536.f, (float)ny) + 1u;
             const float by = (float)y0 * h - eps - uy, bz = (float)z0 * h - eps - uz;
             const float wide = h + 2.f * eps;

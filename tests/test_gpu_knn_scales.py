@@ -1,5 +1,5 @@
 """Exact neighbours whatever the cloud's place and size: clouds far from the
-origin, against brute force over all keys on the GPU."""
+origin and clouds far smaller than 1, against brute force over all keys on the GPU."""
 import numpy as np
 import pytest
 
@@ -45,5 +45,20 @@ def test_knn_far_from_the_origin(n, offset, k):
     Q[m:] += torch.randn(2 * m, 3, generator=g, device="cuda", dtype=torch.float64) * 3e-3
     Q[2 * m:] *= torch.rand(m, 1, generator=g, device="cuda", dtype=torch.float64) * 1.5
     P, Q = (P + off).float().contiguous(), (Q + off).float().contiguous()
+    got = turbo.KnnIndex(P).query(Q, k)
+    assert torch.equal(got, brute(P, Q, k))
+
+
+@pytest.mark.parametrize("n,width,k", [(300000, 2e-6, 15), (100000, 2e-6, 10), (1000000, 1e-5, 16), (100000, 1e-9, 1),
+                                       (100000, 2e-6, 32), (3000, 3e-12, 15)])
+def test_knn_of_tiny_clouds(n, width, k):
+    # many cells an axis, each far below 1e-6: a reach has to stay a few cells
+    P, g = torus(n, seed=k)
+    m = 3000
+    sel = torch.randint(n, (3 * m,), generator=g, device="cuda")
+    Q = P[sel]
+    Q[m:] += torch.randn(2 * m, 3, generator=g, device="cuda", dtype=torch.float64) * 3e-3
+    Q[2 * m:] *= torch.rand(m, 1, generator=g, device="cuda", dtype=torch.float64) * 1.5
+    P, Q = (P * width).float().contiguous(), (Q * width).float().contiguous()
     got = turbo.KnnIndex(P).query(Q, k)
     assert torch.equal(got, brute(P, Q, k))
