@@ -13,6 +13,7 @@
 // dist^2 = (dx*dx + dy*dy) + dz*dz in round-to-nearest single precision.
 #include <cub/cub.cuh>
 
+#include <cfloat>
 #include <climits>
 #include <type_traits>
 #include <vector>
@@ -1197,7 +1198,9 @@ __global__ void __launch_bounds__(kFarWarps * 32) k_knn_far(KnnArgs a, unsigned 
                     const float dz = fmaxf(0.f, fmaxf(z0 - rh[2], rl[2] - z1));
                     push = dx * dx + dy * dy + dz * dz <= wide;
                     const float ax = 0.5f * (x0 + x1) - mx, ay = 0.5f * (y0 + y1) - my, az = 0.5f * (z0 + z1) - mz;
-                    if (push) away = ax * ax + ay * ay + az * az;
+                    // (the limit takes a NaN too, of coordinates whose sums
+                    // overflow: it has to order like the others)
+                    if (push) away = fminf(ax * ax + ay * ay + az * az, FLT_MAX);
                 }
                 int place = sp;
 #pragma unroll

@@ -1,5 +1,5 @@
 """Exact neighbours whatever the cloud's place and size: clouds far from the
-origin and clouds far smaller than 1, against brute force over all keys on the GPU."""
+origin, and clouds far smaller and far larger than 1, against brute force over all keys on the GPU."""
 import numpy as np
 import pytest
 
@@ -60,5 +60,20 @@ def test_knn_of_tiny_clouds(n, width, k):
     Q[m:] += torch.randn(2 * m, 3, generator=g, device="cuda", dtype=torch.float64) * 3e-3
     Q[2 * m:] *= torch.rand(m, 1, generator=g, device="cuda", dtype=torch.float64) * 1.5
     P, Q = (P * width).float().contiguous(), (Q * width).float().contiguous()
+    got = turbo.KnnIndex(P).query(Q, k)
+    assert torch.equal(got, brute(P, Q, k))
+
+
+@pytest.mark.parametrize("width,offset", [(4e19, 0.0), (1e21, 0.0), (1e38, 0.0), (1e38, 2.5e38), (6e37, -3e38)])
+@pytest.mark.parametrize("k", [10, 15])
+def test_knn_of_huge_clouds(width, offset, k):
+    # squares, and sums of two coordinates, beyond the largest number: such
+    # distances are all equal, and the smaller index comes first
+    P, g = torus(6000, seed=k)
+    Q = torch.cat([P[:500], P[500:1000] * 1.3, -P[1000:1100]])
+    P, Q = (P * width + offset).float().contiguous(), (Q * width + offset).float().contiguous()
+    assert torch.isfinite(P).all() and torch.isfinite(Q).all()
+    Q[-20:, 1] = 3.4e38
+    Q[-10:, 2] = -3.4e38
     got = turbo.KnnIndex(P).query(Q, k)
     assert torch.equal(got, brute(P, Q, k))
