@@ -928,7 +928,9 @@ __global__ void __launch_bounds__(kNearThreads) k_knn_near(KnnArgs a, unsigned i
                         const float ddy = fmaxf(0.f, fmaxf(fy, -fy - wide));
                         const float ddz = fmaxf(0.f, fmaxf(fz, -fz - wide));
                         const float rest = out2 - (ddy * ddy + ddz * ddz);
-                        if (rest >= 0.f) {
+                        // (all rows within an infinite radius, whose rest
+                        // is a NaN for a query at infinity)
+                        if (!(rest < 0.f)) {
                             const float hx = sqrt_up(rest) + eps;
                             const int* row = a.cell_start + a.g.G0 * (y0 + iy + a.g.G1 * (z0 + iz));
                             s[u] = row[cell_at(ux - hx, a.g.inv_h, a.g.G0)];

@@ -77,3 +77,16 @@ def test_knn_of_huge_clouds(width, offset, k):
     Q[-10:, 2] = -3.4e38
     got = turbo.KnnIndex(P).query(Q, k)
     assert torch.equal(got, brute(P, Q, k))
+
+
+@pytest.mark.parametrize("n", [14, 100, 6000])
+@pytest.mark.parametrize("k", [5, 14])
+def test_knn_of_queries_at_infinity(n, k):
+    # every distance is infinite: the smallest indices, in a grid of one cell
+    # (points at one spot) as in one of many
+    P = torch.full((n, 3), 0.25, device="cuda") if n < 1000 else torus(n, 1)[0].float().contiguous()
+    inf = float("inf")
+    Q = torch.tensor([[inf, 0, 0], [0, inf, 0], [0, 0, inf], [-inf, 0, 0], [0, -inf, 0], [0, 0, -inf],
+                      [inf, -inf, inf]], device="cuda")
+    got = turbo.KnnIndex(P).query(Q, k)
+    assert torch.equal(got, torch.arange(k, device="cuda", dtype=torch.int32).expand(len(Q), k))
