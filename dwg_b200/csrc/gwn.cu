@@ -217,6 +217,7 @@ struct GwnArgs {
     float ox, oy, oz, h;
     int bx, by;  // bricks per row / column
     long long ngroups;
+    int lanes;  // point queries of a group
     float* __restrict__ out;
     float* out_g;  // gradients, 3 per query (PREC 4)
     unsigned long long* terms_total;
@@ -378,7 +379,7 @@ __device__ __forceinline__ void grid_queries(const GwnArgs& a, unsigned long lon
     }
 }
 
-// the samples of group g: a grid brick, or 32 * NQ consecutive points
+// the samples of group g: a grid brick, or a.lanes * NQ consecutive points
 template <bool GRID, int SHAPE, int NQ>
 __device__ __forceinline__ void group_queries(const GwnArgs& a, unsigned long long g, int lane, bool* valid,
                                               long long* qi, float* qx, float* qy, float* qz) {
@@ -387,8 +388,8 @@ __device__ __forceinline__ void group_queries(const GwnArgs& a, unsigned long lo
     } else {
 #pragma unroll
         for (int u = 0; u < NQ; ++u) {
-            qi[u] = (long long)g * (32 * NQ) + u * 32 + lane;
-            valid[u] = qi[u] < a.nq;
+            qi[u] = (long long)g * (a.lanes * NQ) + u * a.lanes + lane;
+            valid[u] = lane < a.lanes && qi[u] < a.nq;
             qx[u] = qy[u] = qz[u] = 0.f;
             if (valid[u]) {
                 if (a.order) qi[u] = a.order[qi[u]];
@@ -484,27 +485,15 @@ __device__ __forceinline__ void put_sum(const GwnArgs& a, long long i, const Gra
     }
 }
 
-// One of several warps that share a group: the children of the root's
-// children are dealt out by their number in the tree (the first warp also
-// takes the terms of the root's own children), so that a query's sum does not
-// depend on the others of its group; each warp's part goes to sum and nt.
-template <typename Acc>
-struct GwnPart {
-    int part = 0, parts = 1;
-    Acc sum;
-    int nt = 0;
-};
-
 // MODE 0 sums; MODE 1 counts the group's interaction-list entries (visits
 // where some lane takes a term, and multi-point leaves); MODE 2 writes them:
 // (record, term masks per query slot) in visit order.  Modes 1 and 2 do the
 // traversal only.
-template <bool GRID, bool SCREENED, int PREC, int SHAPE, int NQ, int ORDER, int MODE = 0, bool SPLIT = false>
+template <bool GRID, bool SCREENED, int PREC, int SHAPE, int NQ, int ORDER, int MODE = 0>
 __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g, int lane,
                                          int* __restrict__ stk_node, unsigned* __restrict__ stk_mask,
                                          unsigned* __restrict__ stk_meta, float4* __restrict__ crec, float sigma,
-                                         float sigma_l2e, GwnPart<typename AccType<PREC>::T>* split = nullptr) {
-    static_assert(!SPLIT || (MODE == 0 && NQ == 1), "shared groups: sums of one query per lane");
+                                         float sigma_l2e) {
     const unsigned FULL = 0xffffffffu;
     bool valid[NQ];
     long long qi[NQ];
@@ -538,9 +527,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
     // opened (pushed with the queries that need it) otherwise; both use the
     // same d2.  Larger leaves (every leaf when radii apply) are summed point
     // by point.
-    // (term, push: whether this warp takes the child's terms, and its subtree)
-    auto child = [&](int cidx, const float4& na, const float4& nb, const bool* act, int& sp, bool term = true,
-                     bool push = true) {
+    auto child = [&](int cidx, const float4& na, const float4& nb, const bool* act, int& sp) {
         const unsigned meta = (unsigned)__float_as_int(nb.w);
         const bool leaf = (meta & kMetaLeafBit) != 0;
         if (leaf && (!(meta & kMetaSingle) || a.use_radii)) {
@@ -550,7 +537,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
             } else if (MODE == 0) {
 #pragma unroll
                 for (int u = 0; u < NQ; ++u)
-                    if (act[u] && term) leaf_points(st, cnt, u);
+                    if (act[u]) leaf_points(st, cnt, u);
             } else {
                 unsigned m[NQ];
 #pragma unroll
@@ -581,7 +568,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
                 anym |= m[u];
             }
             if (anym) record(cidx, m);
-        } else if (__any_sync(FULL, any && term)) {
+        } else if (__any_sync(FULL, any)) {
 #pragma unroll
             for (int u = 0; u < NQ; ++u) {
                 if constexpr (ORDER == 0) {
@@ -610,7 +597,7 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
             nm[u] = __ballot_sync(FULL, act[u] && !far[u]);
             anym |= nm[u];
         }
-        if (anym && push) {
+        if (anym) {
             if (sp < kGwnStack) {
                 if (lane == 0) {
                     stk_node[sp] = cidx;
@@ -644,28 +631,28 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
             sp = 1;
         }
     }
-    // the children of stack entry i
-    auto open = [&](int i, auto&& each) {
+    while (sp > 0) {
         __syncwarp();
-        const int node = stk_node[i];
-        const unsigned pm = stk_meta[i];
+        --sp;
+        const int node = stk_node[sp];
+        const unsigned pm = stk_meta[sp];
         bool act[NQ];
 #pragma unroll
-        for (int u = 0; u < NQ; ++u) act[u] = (stk_mask[i * NQ + u] >> lane) & 1u;
+        for (int u = 0; u < NQ; ++u) act[u] = (stk_mask[sp * NQ + u] >> lane) & 1u;
         __syncwarp();
         if (node < 0 || node >= a.num_nodes) {
             if (lane == 0) atomicOr(&a.work[1], 2u);
-            return;
+            continue;
         }
         const int first = (int)(pm & kMetaIndex);
         const int nch = (int)((pm >> 28) & 7u) + 1;
         // structural guard: children come after the parent, inside the table
         if ((pm & kMetaLeafBit) || first <= node || first + nch > a.num_nodes) {
             if (lane == 0) atomicOr(&a.work[1], 2u);
-            return;
+            continue;
         }
         // the (at most 8, contiguous) children's records at once, a lane
-        // each, into shared memory; the first __syncwarp above ordered the
+        // each, into shared memory; the loop top's __syncwarp ordered the
         // previous node's reads of them before these writes
         if (lane < nch) {
             crec[lane] = a.node_a[first + lane];
@@ -674,31 +661,8 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
         __syncwarp();
         for (int j = 0; j < nch; ++j) {
             const float4 na = crec[j], nb = crec[8 + j];
-            each(first + j, na, nb, act);
+            child(first + j, na, nb, act, sp);
         }
-    };
-    int low = 0;  // entries below are done
-    if (SPLIT && sp > 0) {
-        const bool lead = split->part == 0;
-        sp = 0;
-        open(0, [&](int c, const float4& na, const float4& nb, const bool* act) { child(c, na, nb, act, sp, lead); });
-        low = sp;
-        for (int i = 0; i < low; ++i)
-            open(i, [&](int c, const float4& na, const float4& nb, const bool* act) {
-                if (c % split->parts == split->part) child(c, na, nb, act, sp);
-            });
-    } else if (SPLIT && split->part > 0) {
-        sum[0] = 0;  // a leaf root is the first warp's
-        nt[0] = 0;
-    }
-    while (sp > low) {
-        --sp;
-        open(sp, [&](int c, const float4& na, const float4& nb, const bool* act) { child(c, na, nb, act, sp); });
-    }
-    if (SPLIT) {
-        split->sum = sum[0];
-        split->nt = nt[0];
-        return 0;
     }
     if (MODE == 1) {
         if (lane == 0) a.list_count[g] = rec;
@@ -745,52 +709,6 @@ __global__ void __launch_bounds__(kGwnWarps * 32, (GRID && kNqGrid >= 4) ? 2 : 3
     }
     if (a.terms_total) {
         for (int o = 16; o > 0; o >>= 1) my_terms += __shfl_down_sync(FULL, my_terms, o);
-        if (lane == 0 && my_terms) atomicAdd(a.terms_total, my_terms);
-    }
-}
-
-// Few point queries: parts (8, 4 or 2) warps share each group of 32 (see
-// GwnPart), so that a launch of a few thousand queries uses the whole GPU
-// instead of one warp per SM.  The parts are added in warp order.
-template <bool SCREENED, int PREC>
-__global__ void __launch_bounds__(kGwnWarps * 32, 3) k_gwn_split(GwnArgs a, int parts) {
-    using Acc = typename AccType<PREC>::T;
-    __shared__ int stk_node[kGwnWarps][kGwnStack];
-    __shared__ unsigned stk_mask[kGwnWarps][kGwnStack];
-    __shared__ unsigned stk_meta[kGwnWarps][kGwnStack];
-    __shared__ float4 crec[kGwnWarps][16];
-    __shared__ Acc sums[kGwnWarps][32];
-    __shared__ int terms[kGwnWarps][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const float sigma = a.sigma_dev ? *a.sigma_dev : a.sigma;
-    const unsigned long long g = (unsigned long long)blockIdx.x * (kGwnWarps / parts) + w / parts;
-    GwnPart<Acc> part;
-    part.part = w % parts;
-    part.parts = parts;
-    if ((long long)g < a.ngroups)
-        gwn_group<false, SCREENED, PREC, 0, 1, 0, 0, true>(a, g, lane, stk_node[w], stk_mask[w], stk_meta[w], crec[w],
-                                                           sigma, sigma * 1.4426950408889634f, &part);
-    sums[w][lane] = part.sum;
-    terms[w][lane] = part.nt;
-    __syncthreads();
-    if (w % parts > 0) return;
-    Acc sum = sums[w][lane];
-    int nt = terms[w][lane];
-    for (int i = 1; i < parts; ++i) {
-        sum += sums[w + i][lane];
-        nt += terms[w + i][lane];
-    }
-    const long long j = (long long)g * 32 + lane;
-    if (j < a.nq) {
-        const long long qi = a.order ? a.order[j] : j;
-        put_sum(a, qi, sum);
-        if (a.per_query_terms) a.per_query_terms[qi] = nt;
-    } else {
-        nt = 0;
-    }
-    if (a.terms_total) {
-        unsigned long long my_terms = (unsigned long long)nt;
-        for (int o = 16; o > 0; o >>= 1) my_terms += __shfl_down_sync(0xffffffffu, my_terms, o);
         if (lane == 0 && my_terms) atomicAdd(a.terms_total, my_terms);
     }
 }
@@ -1309,25 +1227,6 @@ static int blocks_for(K kernel) {
 
 template <bool GRID, bool SCREENED, int PREC, int SHAPE, int ORDER>
 static int launch(const GwnArgs& a, cudaStream_t s) {
-    if constexpr (!GRID && ORDER == 0) {
-        // As many warps per group as keep the launch to one wave: a group's
-        // walk is a chain of dependent loads, 8 warps take about a quarter of
-        // its time (each opens the root and its children), and a second wave
-        // takes as long as the first.  14,000 queries, 20,000 points: 101 us
-        // with 8 warps, 182 us with 1; 28,000: 112 us with 4, 168 with 1.
-        if (a.order) {
-            static int bps = 0;
-            if (!bps) bps = blocks_for(k_gwn_split<SCREENED, PREC>);
-            const long long wave = (long long)num_sms() * bps * kGwnWarps;
-            const int parts = a.ngroups * 8 <= wave ? 8 : a.ngroups * 4 <= wave ? 4 : a.ngroups * 2 <= wave ? 2 : 1;
-            if (parts > 1) {
-                const long long blocks = (a.ngroups * parts + kGwnWarps - 1) / kGwnWarps;
-                k_gwn_split<SCREENED, PREC><<<(unsigned)blocks, kGwnWarps * 32, 0, s>>>(a, parts);
-                DWG_CHECK_LAUNCH();
-                return DWG_OK;
-            }
-        }
-    }
     static int blocks_per_sm = 0;
     if (!blocks_per_sm) blocks_per_sm = blocks_for(k_gwn<GRID, SCREENED, PREC, SHAPE, ORDER>);
     long long want = (a.ngroups + kGwnWarps - 1) / kGwnWarps;
@@ -1369,6 +1268,20 @@ static int dispatch(const GwnArgs& a, const dwg_gwn_params& p, cudaStream_t s) {
     if (prec == 1) return launch_plain<GRID, 1>(a, p, s);
     if (prec == 3) return launch_plain<GRID, 3>(a, p, s);
     return launch_plain<GRID, 2>(a, p, s);
+}
+
+// Point queries of a group: 32, or as few as keep the launch to one wave of
+// warps (three blocks an SM, the kernels' bound).  A group's walk is a chain
+// of dependent loads over the nodes that any of its queries opens, so on a GPU
+// that would idle small groups are done sooner; no query's sum changes, its
+// terms keep their order in any group.  10,000 queries around 100,000 points
+// (values; gradients): 152 and 248 us by 4, 277 and 464 by 32; 100,000: 467
+// and 776 by 4, 221 and 373 by 32.
+static int point_lanes(long long nq) {
+    const long long wave = (long long)num_sms() * 3 * kGwnWarps;
+    int lanes = 1;
+    while (lanes < 32 && (nq + lanes - 1) / lanes > wave) lanes *= 2;
+    return lanes;
 }
 
 // the kernel arguments of a sum (everything but the launch); *empty is set
@@ -1418,17 +1331,21 @@ static int make_args(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p
     if (q.q) {
         a.q = q.q;
         a.nq = q.nq;
-        if (!q.coherent && q.nq > 0) DWG_TRY(query_order(t.qorder, q.q, q.nq, t.root, s, &a.order));
+        // (interaction lists are those of groups of 32; a group of one query
+        // needs no order)
+        a.lanes = q.coherent ? 32 : point_lanes(q.nq);
+        if (!q.coherent && a.lanes > 1) DWG_TRY(query_order(t.qorder, q.q, q.nq, t.root, s, &a.order));
         a.rx = a.ry = a.rz = 0;
         a.zoff = 0;
         a.ox = a.oy = a.oz = a.h = 0.f;
         a.bx = a.by = 1;
-        a.ngroups = (q.nq + 31) / 32;  // one point per lane
+        a.ngroups = (q.nq + a.lanes - 1) / a.lanes;  // one point per lane
         *empty = a.ngroups == 0;
         return DWG_OK;
     }
     DWG_REQUIRE(q.res[0] > 0 && q.res[1] > 0 && q.res[2] > 0, "gwn: bad grid resolution");
     a.q = nullptr;
+    a.lanes = 32;
     a.nq = (long long)q.res[0] * q.res[1] * q.res[2];
     a.rx = q.res[0];
     a.ry = q.res[1];
@@ -1665,6 +1582,7 @@ static void fill_args(GwnArgs& a, const Octree& t, const GwnBatchItem& it, const
     a.use_radii = p.use_radii;
     a.q = nullptr;
     a.order = nullptr;
+    a.lanes = 32;
     a.rx = it.res[0];
     a.ry = it.res[1];
     a.rz = it.res[2];

@@ -78,3 +78,31 @@ def test_grid_fp64_and_gradient_match_points(oracle_lib, case):
     w32 = tree.grid(res, org, h, sigma=20.0).cpu().numpy().astype(np.float64)
     w64 = wg.cpu().numpy()
     assert np.abs(w32 - w64).max() <= 1e-5 * np.abs(w64).max()
+
+
+@pytest.mark.parametrize("screened", [True, False])
+def test_sums_do_not_depend_on_the_call(case, screened):
+    # a query's value and gradient are the same bits alone and in any call:
+    # groups of 1, 2, 4, 8, 16 and 32 queries and their last, partial groups
+    # (3,552 warps fill the GPU: up to 3,552, 7,104, ... queries)
+    Pn, N, A, R, Q = case
+    tree = turbo.TurboLibiGWN(cu(Pn), max_depth=8, areas=cu(A))
+    tree.UpdateMassNormals(cu(N), cu(A))
+    rng = np.random.default_rng(8)
+    q = np.concatenate([Q, Pn[rng.integers(0, len(Pn), 115000)] + rng.normal(0, 0.02, (115000, 3))])
+    q = cu(q[rng.permutation(len(q))].astype(np.float32))
+    kw = dict(sigma=20.0 if screened else 0.0, screened=screened)
+
+    def values(x, precision):
+        if screened:
+            return tree.TurboLibiScreenedGWNLaunch(x, sigma=20.0, precision=precision)
+        return tree.TurboLibiGWNLaunch(x, precision=precision)
+    full = [values(q, p) for p in (0, 1, 2, 3)]
+    w, g = tree.value_and_gradient(q, **kw)
+    for m in (1, 2, 33, 3552, 3553, 10000, 20001, 50000, 60001):
+        x = q[:m].contiguous()
+        for p in (0, 1, 2, 3):
+            assert torch.equal(values(x, p), full[p][:m]), (m, p)
+        w2, g2 = tree.value_and_gradient(x, **kw)
+        assert torch.equal(w2, w[:m]) and torch.equal(g2, g[:m]), m
+    assert tree.status() == 0
