@@ -223,6 +223,9 @@ struct GwnArgs {
     unsigned long long* terms_total;
     int* per_query_terms;
     unsigned int* work;  // [0] counter, [1] error flags (sticky)
+    // the launch's counter: the sums' is work[0]; the gradients, whose calls
+    // may overlap, have the call's own, or none (a block per 8 groups)
+    unsigned int* next;
     int num_nodes, num_points;
     const float4* __restrict__ node_h;  // expansion records, 8 float4 each (plain sums, order >= 1)
     // interaction lists (grids): per-group entry counts (counting pass), the
@@ -701,11 +704,16 @@ __global__ void __launch_bounds__(kGwnWarps * 32, (GRID && kNqGrid >= 4) ? 2 : 3
     unsigned long long my_terms = 0;
     for (;;) {
         unsigned g = 0;
-        if (lane == 0) g = atomicAdd(&a.work[0], 1u);
-        g = __shfl_sync(FULL, g, 0);
+        if (PREC == 4 && !a.next) {
+            g = blockIdx.x * kGwnWarps + w;  // a block per 8 groups
+        } else {
+            if (lane == 0) g = atomicAdd(a.next, 1u);
+            g = __shfl_sync(FULL, g, 0);
+        }
         if ((long long)g >= a.ngroups) break;
         my_terms += (unsigned long long)gwn_group<GRID, SCREENED, PREC, SHAPE, NQ, ORDER, MODE>(
             a, g, lane, stk_node[w], stk_mask[w], stk_meta[w], crec[w], sigma, sigma_l2e);
+        if (PREC == 4 && !a.next) break;
     }
     if (a.terms_total) {
         for (int o = 16; o > 0; o >>= 1) my_terms += __shfl_down_sync(FULL, my_terms, o);
@@ -1231,7 +1239,7 @@ static int launch(const GwnArgs& a, cudaStream_t s) {
     if (!blocks_per_sm) blocks_per_sm = blocks_for(k_gwn<GRID, SCREENED, PREC, SHAPE, ORDER>);
     long long want = (a.ngroups + kGwnWarps - 1) / kGwnWarps;
     long long grid = (long long)num_sms() * blocks_per_sm;
-    if (want < grid) grid = want > 0 ? want : 1;
+    if (want < grid || (PREC == 4 && !a.next)) grid = want > 0 ? want : 1;
     k_gwn<GRID, SCREENED, PREC, SHAPE, ORDER><<<(unsigned)grid, kGwnWarps * 32, 0, s>>>(a);
     DWG_CHECK_LAUNCH();
     return DWG_OK;
@@ -1284,11 +1292,11 @@ static int point_lanes(long long nq) {
     return lanes;
 }
 
-// the kernel arguments of a sum (everything but the launch); *empty is set
-// for an empty point query set
+// the kernel arguments of a sum (everything but the launch), valid while
+// sorted lives; *empty is set for an empty point query set
 static int make_args(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, float* out,
                      unsigned long long* terms_total, int* per_query_terms, cudaStream_t s, const float* sigma_dev,
-                     GwnArgs& a, bool* empty) {
+                     QueryOrder& sorted, GwnArgs& a, bool* empty, bool counter = true) {
     *empty = false;
     DWG_REQUIRE(t.M > 0, "gwn: octree is empty");
     DWG_REQUIRE(out != nullptr, "gwn: output is null");
@@ -1322,11 +1330,11 @@ static int make_args(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p
     a.terms_total = terms_total;
     a.per_query_terms = per_query_terms;
     DWG_TRY(t.work.reserve(2));
-    a.work = t.work.ptr;
+    a.work = a.next = t.work.ptr;
     a.num_nodes = t.M;
     a.num_points = t.n;
     // the counter restarts with every launch; the error word is sticky
-    DWG_CHECK_CUDA(cudaMemsetAsync(t.work.ptr, 0, sizeof(unsigned int), s));
+    if (counter) DWG_CHECK_CUDA(cudaMemsetAsync(t.work.ptr, 0, sizeof(unsigned int), s));
     a.order = nullptr;
     if (q.q) {
         a.q = q.q;
@@ -1334,7 +1342,7 @@ static int make_args(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p
         // (interaction lists are those of groups of 32; a group of one query
         // needs no order)
         a.lanes = q.coherent ? 32 : point_lanes(q.nq);
-        if (!q.coherent && a.lanes > 1) DWG_TRY(query_order(t.qorder, q.q, q.nq, t.root, s, &a.order));
+        if (!q.coherent && a.lanes > 1) DWG_TRY(query_order(sorted, q.q, q.nq, t.root, s, &a.order));
         a.rx = a.ry = a.rz = 0;
         a.zoff = 0;
         a.ox = a.oy = a.oz = a.h = 0.f;
@@ -1369,8 +1377,9 @@ int gwn_eval(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, float*
              unsigned long long* terms_total, int* per_query_terms, cudaStream_t s,
              const float* sigma_dev) {
     GwnArgs a;
+    QueryOrder sorted;
     bool empty = false;
-    DWG_TRY(make_args(t, q, p, out, terms_total, per_query_terms, s, sigma_dev, a, &empty));
+    DWG_TRY(make_args(t, q, p, out, terms_total, per_query_terms, s, sigma_dev, sorted, a, &empty));
     if (empty) return DWG_OK;
     return q.q ? dispatch<false>(a, p, s) : dispatch<true>(a, p, s);
 }
@@ -1383,11 +1392,16 @@ int gwn_eval_grad(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, f
     dwg_gwn_params pp = p;
     pp.tile = 0;  // tile and precision do not apply
     GwnArgs a;
+    QueryOrder sorted;
     bool empty = false;
-    DWG_TRY(make_args(t, q, pp, out_w ? out_w : out_g, nullptr, nullptr, s, nullptr, a, &empty));
+    DWG_TRY(make_args(t, q, pp, out_w ? out_w : out_g, nullptr, nullptr, s, nullptr, sorted, a, &empty, false));
     if (empty) return DWG_OK;
     a.out = out_w;
     a.out_g = out_g;
+    // (up to 3,552 queries, one wave, need no counter; 200,001 around 100,000
+    // points: 622 us with one, 676 with a block per 8 groups)
+    if (!q.q) DWG_TRY(work_counter(sorted, s));
+    a.next = sorted.counter;
     if (q.q) return p.screened ? launch<false, true, 4, 0, 0>(a, s) : launch<false, false, 4, 0, 0>(a, s);
     return p.screened ? launch<true, true, 4, 0, 0>(a, s) : launch<true, false, 4, 0, 0>(a, s);
 }
@@ -1536,8 +1550,9 @@ int gwn_eval_listed(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p,
     DWG_REQUIRE(p.screened && p.order == 0, "gwn lists: screened sums only");
     DWG_REQUIRE(!q.q || q.coherent, "gwn lists: point queries in their own order only");
     GwnArgs a;
+    QueryOrder sorted;
     bool empty = false;
-    DWG_TRY(make_args(t, q, p, out, terms_total, nullptr, s, sigma_dev, a, &empty));
+    DWG_TRY(make_args(t, q, p, out, terms_total, nullptr, s, sigma_dev, sorted, a, &empty));
     if (empty) return DWG_OK;
     const bool grid = !q.q;
     const bool same = L.ngroups == a.ngroups && L.grid == grid && L.qptr == q.q && L.nq == a.nq &&
@@ -1602,6 +1617,7 @@ static void fill_args(GwnArgs& a, const Octree& t, const GwnBatchItem& it, const
     a.terms_total = it.terms_total;
     a.per_query_terms = nullptr;
     a.work = t.work.ptr;  // error word at [1]
+    a.next = nullptr;
     a.node_h = nullptr;
     a.list_count = nullptr;
     a.list_off = nullptr;

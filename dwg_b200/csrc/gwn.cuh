@@ -2,6 +2,7 @@
 #pragma once
 
 #include "octree.cuh"
+#include "order.cuh"
 
 namespace dwg {
 

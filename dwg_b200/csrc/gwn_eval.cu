@@ -210,10 +210,11 @@ int gwn_eval_fp64(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, d
     a.out_g = out_g;
     a.err = t.work.ptr + 1;
     a.order = nullptr;
+    QueryOrder sorted;
     if (q.q) {
         a.q = q.q;
         a.nq = q.nq;
-        if (!q.coherent && q.nq > 0) DWG_TRY(query_order(t.qorder, q.q, q.nq, t.root, s, &a.order));
+        if (!q.coherent && q.nq > 0) DWG_TRY(query_order(sorted, q.q, q.nq, t.root, s, &a.order));
         a.rx = a.ry = a.rz = a.zoff = 0;
         a.ox = a.oy = a.oz = a.h = 0.f;
     } else {

@@ -28,7 +28,6 @@
 #pragma once
 
 #include "common.cuh"
-#include "order.cuh"
 
 namespace dwg {
 
@@ -66,7 +65,6 @@ struct Octree {
     DevBuf<int> big_nodes;  // [0] number, then the nodes of many points (any order)
     int level_off[kMaxDepth + 2] = {0};
     DevBuf<unsigned char> scratch;  // CUB temporary storage
-    mutable QueryOrder qorder;          // spatial order of point queries
     mutable DevBuf<unsigned int> work;  // [0] work counter of the persistent GWN kernel, [1] error flag
 };
 

@@ -50,11 +50,32 @@ __global__ void k_query_place(const int* __restrict__ key, long long nq, int* __
 
 }  // namespace
 
-int query_order(QueryOrder& w, const float* q, long long nq, const double root[4], cudaStream_t s, const int** order) {
-    *order = nullptr;
+static int call_memory(QueryOrder& w, size_t bytes, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     DWG_CHECK_CUDA(cudaStreamIsCapturing(s, &cs));
-    if (cs != cudaStreamCaptureStatusNone || nq >= (1ll << 31) || !(root[3] > 0)) return DWG_OK;
+    if (cs != cudaStreamCaptureStatusNone) return DWG_OK;
+    const cudaError_t e = cudaMallocAsync(&w.mem, bytes, s);
+    if (e != cudaSuccess) w.mem = nullptr;
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return DWG_OK;
+    }
+    DWG_CHECK_CUDA(e);
+    w.stream = s;
+    return DWG_OK;
+}
+
+int work_counter(QueryOrder& w, cudaStream_t s) {
+    DWG_TRY(call_memory(w, sizeof(int), s));
+    if (!w.mem) return DWG_OK;
+    DWG_CHECK_CUDA(cudaMemsetAsync(w.mem, 0, sizeof(int), s));
+    w.counter = (unsigned int*)w.mem;
+    return DWG_OK;
+}
+
+int query_order(QueryOrder& w, const float* q, long long nq, const double root[4], cudaStream_t s, const int** order) {
+    *order = nullptr;
+    if (nq >= (1ll << 31) || !(root[3] > 0)) return DWG_OK;
     // ~4 queries of a surface per cell, at most 2^21 cells (clearing and
     // scanning their counts takes 10 us)
     int bits = 4;
@@ -64,23 +85,24 @@ int query_order(QueryOrder& w, const float* q, long long nq, const double root[4
     for (int d = 0; d < 3; ++d) c.lo[d] = (float)(root[d] - 0.5 * root[3]);
     c.scale = (float)(cells / root[3]);
     c.cells = cells;
-    DWG_TRY(w.key.reserve(nq));
-    DWG_TRY(w.order.reserve(nq));
-    DWG_TRY(w.hist.reserve(buckets));
-    DWG_TRY(w.fill.reserve(buckets));
-    DWG_CHECK_CUDA(cudaMemsetAsync(w.hist.ptr, 0, sizeof(int) * buckets, s));
+    size_t scan = 0;
+    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan, (int*)nullptr, (int*)nullptr, buckets, s));
+    // keys, order, counts and the counter, places, the scan's storage
+    const size_t keys = ((size_t)nq * sizeof(int) + 255) / 256 * 256, counts = (size_t)buckets * sizeof(int);
+    DWG_TRY(call_memory(w, 2 * keys + 2 * counts + 256 + scan, s));
+    if (!w.mem) return DWG_OK;
+    char* const at = (char*)w.mem;
+    int *key = (int*)at, *out = (int*)(at + keys), *hist = (int*)(at + 2 * keys), *fill = hist + buckets + 64;
+    DWG_CHECK_CUDA(cudaMemsetAsync(hist, 0, counts + sizeof(int), s));
+    w.counter = (unsigned int*)(hist + buckets);
     long long blocks = (nq + 255) / 256;
     if (blocks > (long long)num_sms() * 8) blocks = (long long)num_sms() * 8;
-    k_query_key<<<(unsigned)blocks, 256, 0, s>>>(q, nq, c, w.key.ptr, w.hist.ptr);
+    k_query_key<<<(unsigned)blocks, 256, 0, s>>>(q, nq, c, key, hist);
     DWG_CHECK_LAUNCH();
-    size_t bytes = 0;
-    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, w.hist.ptr, w.fill.ptr, buckets, s));
-    DWG_TRY(w.scratch.reserve(bytes + 256));
-    bytes = w.scratch.n;
-    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(w.scratch.ptr, bytes, w.hist.ptr, w.fill.ptr, buckets, s));
-    k_query_place<<<(unsigned)blocks, 256, 0, s>>>(w.key.ptr, nq, w.fill.ptr, w.order.ptr);
+    DWG_CHECK_CUDA(cub::DeviceScan::ExclusiveSum(at + 2 * keys + 2 * counts + 256, scan, hist, fill, buckets, s));
+    k_query_place<<<(unsigned)blocks, 256, 0, s>>>(key, nq, fill, out);
     DWG_CHECK_LAUNCH();
-    *order = w.order.ptr;
+    *order = out;
     return DWG_OK;
 }
 

@@ -172,7 +172,10 @@ int dwg_gwn_grid(dwg_octree* tree, const float* normals_dev, const float* areas_
  * and of the far nodes' order-0 dipoles, with the opening decisions of
  * dwg_gwn_points -- and out_dev (nullable) the values.  FP32 terms summed in
  * FP64, in the warp walk of dwg_gwn_points; params->order must be 0; lists,
- * tile and precision are ignored. */
+ * tile and precision are ignored.  Calls of one octree, and the FP64 sums
+ * below, may overlap on several streams while they set nothing (normals, areas
+ * and radii NULL, beta that of the call before); the sums of dwg_gwn_points
+ * and dwg_gwn_grid share a work counter and must follow each other. */
 int dwg_gwn_points_grad(dwg_octree* tree, const float* normals_dev, const float* areas_dev,
                         const float* radii_dev, const float* queries_dev, long long num_queries,
                         const dwg_gwn_params* params, float* out_dev, float* grad_dev, void* stream);

@@ -106,3 +106,27 @@ def test_sums_do_not_depend_on_the_call(case, screened):
         w2, g2 = tree.value_and_gradient(x, **kw)
         assert torch.equal(w2, w[:m]) and torch.equal(g2, g[:m]), m
     assert tree.status() == 0
+
+
+def test_gradients_and_fp64_sums_of_two_streams(case):
+    # calls of one octree that overlap: each has its own order of the queries
+    Pn, N, A, R, Q = case
+    tree = turbo.TurboLibiGWN(cu(Pn), max_depth=8, areas=cu(A))
+    tree.UpdateMassNormals(cu(N), cu(A))
+    rng = np.random.default_rng(9)
+    near = (Pn[rng.integers(0, len(Pn), 31000)] + rng.normal(0, 0.02, (31000, 3))).astype(np.float32)
+    sets = [cu(Q[:7001]), cu(near)]
+    ref = [(*tree.value_and_gradient(x, sigma=20.0), *tree.value_and_gradient(x, sigma=20.0, fp64=True)) for x in sets]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in sets]
+    got = [[], []]
+    for _ in range(6):
+        for i in (0, 1):
+            with torch.cuda.stream(streams[i]):
+                got[i].append((*tree.value_and_gradient(sets[i], sigma=20.0),
+                               *tree.value_and_gradient(sets[i], sigma=20.0, fp64=True)))
+    torch.cuda.synchronize()
+    for i in (0, 1):
+        for out in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(out, ref[i]))
+    assert tree.status() == 0
