@@ -217,7 +217,7 @@ struct GwnArgs {
     float ox, oy, oz, h;
     int bx, by;  // bricks per row / column
     long long ngroups;
-    int lanes;  // point queries of a group
+    int lanes;  // point queries, or gradients of a grid, of a group
     float* __restrict__ out;
     float* out_g;  // gradients, 3 per query (PREC 4)
     unsigned long long* terms_total;
@@ -382,11 +382,16 @@ __device__ __forceinline__ void grid_queries(const GwnArgs& a, unsigned long lon
     }
 }
 
-// the samples of group g: a grid brick, or a.lanes * NQ consecutive points
+// the samples of group g: a grid brick (with one sample a lane, a part of
+// one), or a.lanes * NQ consecutive points
 template <bool GRID, int SHAPE, int NQ>
 __device__ __forceinline__ void group_queries(const GwnArgs& a, unsigned long long g, int lane, bool* valid,
                                               long long* qi, float* qx, float* qy, float* qz) {
-    if (GRID) {
+    if (GRID && NQ == 1) {  // a brick's 32 samples in parts of a.lanes
+        const unsigned parts = 32u / a.lanes;
+        grid_queries<SHAPE, NQ>(a, g / parts, ((int)(g % parts) * a.lanes + lane) & 31, valid, qi, qx, qy, qz);
+        valid[0] = valid[0] && lane < a.lanes;
+    } else if (GRID) {
         grid_queries<SHAPE, NQ>(a, g, lane, valid, qi, qx, qy, qz);
     } else {
 #pragma unroll
@@ -684,14 +689,14 @@ __device__ __forceinline__ int gwn_group(const GwnArgs& a, unsigned long long g,
     return total;
 }
 
-template <bool GRID>
+template <bool GRID, int PREC = 1>
 __host__ __device__ constexpr int nq_of() {
-    return GRID ? kNqGrid : 1;
+    return GRID && PREC != 4 ? kNqGrid : 1;
 }
 
 template <bool GRID, bool SCREENED, int PREC, int SHAPE, int ORDER, int MODE = 0>
 __global__ void __launch_bounds__(kGwnWarps * 32, (GRID && kNqGrid >= 4) ? 2 : 3) k_gwn(GwnArgs a) {
-    constexpr int NQ = nq_of<GRID>();
+    constexpr int NQ = nq_of<GRID, PREC>();
     __shared__ int stk_node[kGwnWarps][kGwnStack];
     __shared__ unsigned stk_mask[kGwnWarps][kGwnStack * NQ];
     __shared__ unsigned stk_meta[kGwnWarps][kGwnStack];
@@ -1400,7 +1405,19 @@ int gwn_eval_grad(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, f
     a.out_g = out_g;
     // (up to 3,552 queries, one wave, need no counter; 200,001 around 100,000
     // points: 622 us with one, 676 with a block per 8 groups)
-    if (!q.q) DWG_TRY(work_counter(sorted, s));
+    if (!q.q) {
+        // one sample a lane, and few lanes for few samples: a grid's samples
+        // lie farther apart than points of a surface, and what one opens all
+        // of the warp's IEEE terms wait for (100,000 points, us, with two
+        // samples a lane and with one: 16^3 779 and 154, 64^3 541 and 416, 100^3 1,004 and 908)
+        int ex, ey, ez;
+        brick_extent(0, ex, ey, ez);
+        const long long bricks = (long long)a.bx * a.by * ((a.rz + ez - 1) / ez);
+        a.lanes = point_lanes(bricks * 32);
+        a.ngroups = bricks * (32 / a.lanes);
+        DWG_REQUIRE(a.ngroups < (1ll << 32), "gwn: grid too large");
+        DWG_TRY(work_counter(sorted, s));
+    }
     a.next = sorted.counter;
     if (q.q) return p.screened ? launch<false, true, 4, 0, 0>(a, s) : launch<false, false, 4, 0, 0>(a, s);
     return p.screened ? launch<true, true, 4, 0, 0>(a, s) : launch<true, false, 4, 0, 0>(a, s);

@@ -130,3 +130,23 @@ def test_gradients_and_fp64_sums_of_two_streams(case):
         for out in got[i]:
             assert all(torch.equal(a, b) for a, b in zip(out, ref[i]))
     assert tree.status() == 0
+
+
+@pytest.mark.parametrize("res", [(1, 1, 1), (5, 3, 2), (23, 19, 11), (33, 40, 30), (70, 61, 54)])
+@pytest.mark.parametrize("screened", [True, False])
+def test_grid_gradients_match_fp64(case, res, screened):
+    # FP32 gradients at a grid: bricks cut at its ends, parts of a brick of 1
+    # to 32 samples; tolerances as at points, relative to the sums at points
+    Pn, N, A, R, Q = case
+    tree = turbo.TurboLibiGWN(cu(Pn), max_depth=8, areas=cu(A))
+    tree.UpdateMassNormals(cu(N), cu(A))
+    kw = dict(beta=2.3, sigma=20.0 if screened else 0.0, screened=screened)
+    sw, sg = (float(t.abs().max()) for t in tree.value_and_gradient(cu(Q), fp64=True, **kw))
+    res = np.array(res, np.int32)
+    grid = (res, np.array([-0.52, -0.5, -0.2], np.float32), np.float32(1.0 / max(res.max(), 2)))
+    w64, g64 = tree.value_and_gradient(grid=grid, fp64=True, **kw)
+    w32, g32 = tree.value_and_gradient(grid=grid, **kw)
+    ew, eg = (w32.double() - w64).abs(), (g32.double() - g64).abs()
+    assert float(ew.max()) <= 1e-5 * sw and float((ew ** 2).mean()) ** 0.5 <= 1e-6 * sw
+    assert float(eg.max()) <= 1e-4 * sg and float((eg ** 2).mean()) ** 0.5 <= 1e-5 * sg
+    assert tree.status() == 0
