@@ -214,7 +214,9 @@ int gwn_eval_fp64(const Octree& t, const GwnQuery& q, const dwg_gwn_params& p, d
     if (q.q) {
         a.q = q.q;
         a.nq = q.nq;
-        if (!q.coherent && q.nq > 0) DWG_TRY(query_order(sorted, q.q, q.nq, t.root, s, &a.order));
+        // (few queries are done sooner than sorted: 1 query 74 us with, 61
+        // without; 1,000 around 100,000 points 306 with, 340 without)
+        if (!q.coherent && q.nq > 256) DWG_TRY(query_order(sorted, q.q, q.nq, t.root, s, &a.order));
         a.rx = a.ry = a.rz = a.zoff = 0;
         a.ox = a.oy = a.oz = a.h = 0.f;
     } else {

@@ -150,3 +150,14 @@ def test_grid_gradients_match_fp64(case, res, screened):
     assert float(ew.max()) <= 1e-5 * sw and float((ew ** 2).mean()) ** 0.5 <= 1e-6 * sw
     assert float(eg.max()) <= 1e-4 * sg and float((eg ** 2).mean()) ** 0.5 <= 1e-5 * sg
     assert tree.status() == 0
+
+
+def test_fp64_sums_do_not_depend_on_the_call(case):
+    # with and without a spatial order
+    Pn, N, A, R, Q = case
+    tree = turbo.TurboLibiGWN(cu(Pn), max_depth=8, areas=cu(A))
+    tree.UpdateMassNormals(cu(N), cu(A))
+    w, g = tree.value_and_gradient(cu(Q), sigma=20.0, fp64=True)
+    for m in (1, 256, 257):
+        w2, g2 = tree.value_and_gradient(cu(Q[:m]), sigma=20.0, fp64=True)
+        assert torch.equal(w2, w[:m]) and torch.equal(g2, g[:m])
