@@ -220,7 +220,7 @@ void pool_free(void* p) {
         }
     }
     if (t_free.active) {
-        cudaStream_t s = t_free.stream;
+        cudaStream_t s = t_free.stream ? t_free.stream : cudaStreamLegacy;
         if (t_free.idle) {
             if (dev < 0) cudaGetDevice(&dev);
             s = side_stream(dev);

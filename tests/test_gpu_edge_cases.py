@@ -77,3 +77,21 @@ def test_degenerate_clouds_track_oracle(oracle_lib, kind):
         assert np.all(np.isfinite(got[k])), k
     assert np.allclose(got["iso"][:1], ref["iso"][:1], rtol=1e-4, atol=1e-9)
     assert abs(len(got["tris"]) - len(ref["tris"])) <= 0.01 * len(ref["tris"]) + 4
+
+
+def test_builds_on_the_default_stream_wait_for_it_alone(dwg_lib):
+    # temporaries of an index and of a tree go back in the order of the
+    # caller's stream, the default one too: a build does not wait for another
+    # stream's work (a kernel that counts ~0.5 s of cycles)
+    P, _ = D.sphere(3000, seed=6)
+    Pd = cu(P.astype(np.float32))
+    side, done = torch.cuda.Stream(), torch.cuda.Event()
+    for build in (lambda: turbo.KnnIndex(Pd), lambda: turbo.TurboLibiGWN(Pd, max_depth=8)):
+        keep = [build() for _ in range(2)]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(1000000000)
+            done.record(side)
+        keep.append(build())
+        assert not done.query()
+        torch.cuda.synchronize()
