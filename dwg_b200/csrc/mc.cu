@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kMcThreads)
     }
 }
 
-// Grids with rows of kMcThinRow cells and more: rows are cut into segments of
+// Grids with rows of kMcThinRow cells and more, and more than kMcFewCells: rows are cut into segments of
 // 31 cells (the 32 samples of a warp's lanes), eight consecutive segments (in
 // cell order) are a unit of the output.
 //
@@ -599,6 +599,11 @@ constexpr int kMcMarch = 16;
 constexpr int kMcAhead = 4;
 // below, lanes of a segment would idle: a thread per cell in both passes
 constexpr int kMcThinRow = 16;
+// so do grids of up to as many cells: their units are a few hundred, and a warp
+// takes a unit's triangles in turn while most of the GPU idles (whole calls by
+// rows and by cells, us, a surface and noise: 40^3 60 and 94, 56 and 69; 48^3 60
+// and 84, 56 and 80; 64^3 63 and 95, 70 and 132)
+constexpr long long kMcFewCells = 1 << 17;
 
 // case of the cell at each lane from the masks of its rows (z, y), (z, y + 1),
 // (z + 1, y), (z + 1, y + 1)
@@ -872,7 +877,7 @@ struct McCut {
 static McCut mc_cut(const McArgs& a, long long most_parts) {
     const long long cx = a.rx - 1, rows = (long long)(a.ry - 1) * (a.rz - 1);
     const long long segs = (cx + kMcSeg - 1) / kMcSeg, units = (segs * rows + kMcUnit - 1) / kMcUnit;
-    if (cx >= kMcThinRow && segs * rows < (1ll << 32) - kMcUnit && units <= most_parts)
+    if (cx >= kMcThinRow && a.ncell > kMcFewCells && segs * rows < (1ll << 32) - kMcUnit && units <= most_parts)
         return {(unsigned)segs, units};
     return {0u, (a.ncell + kMcThreads - 1) / kMcThreads};
 }

@@ -743,3 +743,12 @@ def test_knn_of_one_cell(n, k):
     kk = min(k, n)
     got = turbo.KnnIndex(cu(P)).query(cu(Q), kk).cpu().numpy()
     assert np.array_equal(got, np.tile(np.arange(kk, dtype=got.dtype), (3, 1)))
+
+
+@pytest.mark.parametrize("res", [(65, 65, 33), (66, 65, 33), (17, 120, 80), (32, 81, 60), (33, 66, 70), (64, 49, 45),
+                                 (95, 35, 45), (300, 17, 40)])
+@pytest.mark.parametrize("positions", [False, True])
+def test_marching_cubes_cuts_of_many_cells(oracle_lib, dwg_lib, res, positions):
+    # as test_marching_cubes_cuts, on both sides of the number of cells from
+    # which rows are cut into segments (2^17)
+    test_marching_cubes_cuts(oracle_lib, dwg_lib, res, positions)
