@@ -54,7 +54,9 @@ int gauss_map(const float* P, int n, float* N, cudaStream_t s) {
 // points that find no place in kScatterProbes steps, go to global memory at
 // once).  240,000 triangles onto 10,000 points,
 // k = 15: 31 us (93 with an atomic per triangle, neighbour and component);
-// 300,000 onto 830,000: 50 (95).
+// 300,000 onto 830,000: 50 (95).  Neighbours in no spatial order at all leave
+// a table nothing to collect: 200,000 triangles, k = 15, of random points 86 us
+// (75).
 constexpr int kScatterTris = 256;
 constexpr int kScatterAdds = 2047;
 constexpr int kScatterSlots = 1024;
@@ -127,6 +129,22 @@ __global__ void __launch_bounds__(256) k_scatter(const int* __restrict__ knn, co
 }
 static_assert(kScatterSlots == 1 << 10, "10 bits of hash");
 
+// few sums: a thread per triangle and neighbour
+__global__ void k_scatter_few(const int* __restrict__ knn, const float* __restrict__ tn, long long T,
+                              const unsigned long long* __restrict__ Tdev, int k, int L,
+                              unsigned long long* __restrict__ acc) {
+    long long nt = T;
+    if (Tdev && (long long)*Tdev < nt) nt = (long long)*Tdev;
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e >= nt * k) return;
+    const int i = knn[e];
+    if (i < 0 || i >= L) return;
+    const float* n = tn + e / k * 3;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        atomicAdd(&acc[(size_t)i * 3 + d], (unsigned long long)__double2ll_rn((double)n[d] * kFix));
+}
+
 // NormalizeNormals (src/TurboDWG.cu:238-266); also clears the accumulator
 __global__ void k_finalize(long long* __restrict__ acc, int L, float* __restrict__ N,
                            unsigned char* __restrict__ is_zero, int* __restrict__ zero_count) {
@@ -153,7 +171,12 @@ __global__ void k_finalize(long long* __restrict__ acc, int L, float* __restrict
 int diffuse_scatter(const int* knn, const float* tn, long long T, const unsigned long long* Tdev, int k, int L,
                     const int* order, long long* acc, cudaStream_t s) {
     DWG_REQUIRE(knn && tn && acc && L >= 1 && k >= 1, "diffuse_normals: bad arguments");
-    if (T > 0) {
+    // (filling and emptying the tables takes longer than 2^17 sums in the open:
+    // whole calls of 10,000 triangles, k = 10, 38 and 35 us, 100 triangles 36 and 33)
+    if (T > 0 && T * k <= (1 << 17)) {
+        k_scatter_few<<<div_up(T * k, 256), 256, 0, s>>>(knn, tn, T, Tdev, k, L, (unsigned long long*)acc);
+        DWG_CHECK_LAUNCH();
+    } else if (T > 0) {
         const int each = std::min(kScatterTris, std::max(1, kScatterAdds / k));
         long long blocks = (T + each - 1) / each;
         const long long cap = (long long)num_sms() * 6;

@@ -752,3 +752,11 @@ def test_marching_cubes_cuts_of_many_cells(oracle_lib, dwg_lib, res, positions):
     # as test_marching_cubes_cuts, on both sides of the number of cells from
     # which rows are cut into segments (2^17)
     test_marching_cubes_cuts(oracle_lib, dwg_lib, res, positions)
+
+
+@pytest.mark.parametrize("T,k,L", [(13107, 10, 5000), (13108, 10, 5000), (131073, 1, 60000), (9000, 15, 400),
+                                   (9000, 15, 4000000), (200, 1000, 500), (70, 2048, 3000)])
+def test_diffusion_of_many_sums(oracle_lib, dwg_lib, T, k, L):
+    # as test_diffusion_tables, on both sides of the number of sums from which
+    # a block's are collected (2^17)
+    test_diffusion_tables(oracle_lib, dwg_lib, T, k, L)
