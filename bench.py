@@ -341,12 +341,12 @@ def run_ours(a, rank, world, local_rank):
 
 def _dominant_roofline(census, roofs):
     """The roofline of the kernel with the largest device time in one step
-    (the GWN weight read or the cell-grouped kNN, whichever leads)."""
+    (the GWN weight read or the kNN rounds, whichever leads)."""
     if not census:
         return "gwn"
     rows = census.get("all", census.get("top", []))
     top = max(rows, key=lambda r: r["ms"]) if rows else None
-    best = "knn" if top and ("k_knn" in top["kernel"] or "k_cq_" in top["kernel"]) else "gwn"
+    best = "knn" if top and "k_knn" in top["kernel"] else "gwn"
     return best if "error" not in roofs.get(best, {"error": 1}) else "gwn"
 
 

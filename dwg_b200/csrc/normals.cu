@@ -285,8 +285,8 @@ int zero_repair(const KnnIndex& ix, const float* pos, int L, float* N, const uns
     q.gate_min = min_zero;
     q.coherent = spatial_order;  // the list is in point order
     long long blocks = (long long)num_sms() * 4;
-    // seeds from the neighbours recorded by earlier calls (k <= 16: the
-    // cell-grouped search); the record starts empty
+    // seeds from the neighbours recorded by earlier calls (k <= 16: the near
+    // and far rounds start from them); the record starts empty
     int* prev = nullptr;
     if (k <= kKnnNearK) {
         if (!ws.prev.ptr || ws.prev.n < (size_t)L * k || ws.prev_k != k) {
