@@ -1429,7 +1429,9 @@ int knn_query(const KnnIndex& ix, const KnnQuery& q, int k, int* out, cudaStream
     a.far_group = nullptr;
     a.far_count = nullptr;
     a.seed = q.seed;
-    if (!q.coherent) {
+    // few queries are done sooner than ordered (the far side of a ball of 20,000
+    // points: 1 query 96 us with, 75 without; on its surface 42 and 20)
+    if (!q.coherent && q.nq > 512) {
         // bucket the queries spatially (counting sort on device counts, no host sync)
         DWG_TRY(ix.q_key.reserve(q.nq));
         DWG_TRY(ix.q_order.reserve(q.nq));

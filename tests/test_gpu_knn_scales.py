@@ -90,3 +90,14 @@ def test_knn_of_queries_at_infinity(n, k):
                       [inf, -inf, inf]], device="cuda")
     got = turbo.KnnIndex(P).query(Q, k)
     assert torch.equal(got, torch.arange(k, device="cuda", dtype=torch.int32).expand(len(Q), k))
+
+
+@pytest.mark.parametrize("m", [512, 513])
+@pytest.mark.parametrize("k", [10, 20])
+def test_knn_of_few_queries(m, k):
+    # up to 512 queries are taken as they come
+    P, g = torus(20000, seed=k)
+    Q = P[torch.randint(20000, (m,), generator=g, device="cuda")]
+    Q[::3] *= 1.7
+    P, Q = P.float().contiguous(), Q.float().contiguous()
+    assert torch.equal(turbo.KnnIndex(P).query(Q, k), brute(P, Q, k))
