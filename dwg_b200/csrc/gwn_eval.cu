@@ -9,7 +9,7 @@
 // threshold (exactly the warp kernels' test, so the same terms are taken);
 // leaves are always summed point by point.  The traversal walks the level-
 // order records with a per-level (first child, count, next) stack; point
-// queries are taken in spatial order.
+// queries beyond a few hundred are taken in spatial order.
 #include <algorithm>
 
 #include "gwn.cuh"
